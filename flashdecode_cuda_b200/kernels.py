@@ -90,6 +90,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "fd_tc_test_hook": [LL, I],
         "fd_gemv_splits": [I, I, I, I, I],
         "fd_gemv": [P, P, P, I, P, I, I, I, I, I, P, c_ulonglong, P, I, I, P],
+        "fd_gemm_f32_set_form": [I],
         "fd_gemm_simt": [P, P, P, P, I, I, I, I, I, I, P],
         "fd_attn_simt_qt": [I],
         "fd_attn_decode_group": [I, I, I],
@@ -729,6 +730,12 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
     assert w.shape[1] == K and out.shape == (M, N) and w.dtype == x.dtype
     _check(lib().fd_gemm_simt(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _dt(x.dtype),
                               _dt(bias.dtype) if bias is not None else 0, _dt(out.dtype), M, N, K, _stream()))
+
+
+def gemm_f32_set_form(form: int) -> None:
+    """The tiling of float32 products of more than 16 rows: 0 by the kernel's rule, 1..6 one of the six (tests and
+    measurements; all give the same bits)."""
+    _check(lib().fd_gemm_f32_set_form(int(form)))
 
 
 def attention_decode_heads(n_q: int, n_kv: int, head_dim: int, v_dim: int) -> int:

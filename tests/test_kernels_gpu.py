@@ -328,6 +328,33 @@ def test_gemm_simt_rows_do_not_depend_on_the_batch(N, K_):
     assert rel(big, P.linear(x.double(), w.double(), b.double())) < 2e-5
 
 
+@pytest.mark.parametrize("N,K_", [(16, 4), (333, 36), (1536, 224), (9472, 520), (9500, 132)])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 65, 130])
+def test_gemm_f32_forms_give_the_same_bits(M, N, K_):
+    """Every form of the float32 product runs one chain per output in the order of k, so all agree to the bit: with the
+    general kernel too (A off the 16-byte boundary, more than 16 rows).  Edges: one row either side of a form's rows, matrices just
+    narrow and just wide, K of one piece and beyond whole steps."""
+    g = torch.Generator().manual_seed(6)
+    buf = torch.randn(M * K_ + 1, generator=g).to(DEV)
+    x, w, b = buf[:M * K_].view(M, K_), torch.randn(N, K_, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
+    off = torch.empty(M * K_ + 1, device=DEV)[1:].view(M, K_)      # the same values, 4 bytes off
+    off.copy_(x)
+    want = torch.full((M, N), float("nan"), device=DEV)
+    K.gemm_simt(off, w, b, want)
+    # K products and K sums of size one: each rounding 2^-24 of a partial sum of at most sqrt(K) or so
+    assert rel(want, P.linear(x.double(), w.double(), b.double())) < 2e-6
+    try:
+        for form in range(7):
+            K.gemm_f32_set_form(form)
+            out = torch.full((M, N), float("nan"), device=DEV)
+            K.gemm_simt(x, w, b, out)
+            assert torch.equal(out, want), form
+            if M <= 16:                                            # the tilings are for more rows
+                break
+    finally:
+        K.gemm_f32_set_form(0)
+
+
 # ---------------------------------------------------------------------------
 # paged cache helpers for the rope and attention kernels
 # ---------------------------------------------------------------------------
