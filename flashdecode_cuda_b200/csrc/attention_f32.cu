@@ -1,0 +1,379 @@
+// Attention of the true 32-bit path over the paged cache, for head sizes 64 and 128: causal, grouped heads, with an optional
+// window or chunked visibility.  Float throughout, no tensor cores; key tiles, splits and the order of every sum are fixed in
+// absolute position, so a query's bits depend on nothing but its own sequence.  (attention_simt.cu takes every other size
+// and option.)
+//
+//  * decode: a CTA takes one (sequence, key/value head, split) and tiles of 64 keys.  Bound by the chain of lookups, one trip
+//    to memory, scores, softmax and values: all of a tile's keys and values are asked for at once, and with splits of 64 keys
+//    (attention.py) a CTA has one tile.
+//  * prompts: a CTA takes up to 64 rows (query, head of the group) and walks the keys in tiles of 64; scores and value sums
+//    are register tiles of 8 x 4 and 8 x HD/16 per thread.  Bound by the FMA pipes and what shared memory delivers.
+#include <math.h>
+
+#include "attention.cuh"
+
+namespace fd {
+
+namespace {
+
+constexpr int FT = 64;             // keys per tile
+constexpr int FTHREADS = 128;
+constexpr int GDEC = 8;            // most query heads per key/value head in the decode kernel
+
+__device__ __forceinline__ void cp16(void* dst, const void* src, bool on) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(d), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
+
+// The rows in the pools of the tile's FT tokens from t0 on (-1: outside [lo, hi) or not in the cache), by the first FT threads.
+__device__ __forceinline__ void tile_rows(const AttnParams& p, int slot, int kvh, int t0, int lo, int hi, int* row_s) {
+    const int t = t0 + (int)threadIdx.x;
+    if (threadIdx.x >= FT) return;
+    int row = -1;
+    if (t >= lo && t < hi) {
+        const int blk = p.block_table[(size_t)slot * p.max_blocks + t / p.block_size];
+        if (blk < 0 || blk >= p.num_blocks) set_status(p.status, STATUS_BAD_BLOCK);
+        else row = (blk * p.n_kv_pool + kvh) * p.block_size + t % p.block_size;
+    }
+    row_s[threadIdx.x] = row;
+}
+
+// A tile of keys (or values) to shared memory, rows LD apart; rows of -1 read as zero.
+template <int HD, int LD>
+__device__ __forceinline__ void load_tile(float* dst, const float* pool, const int* row_s) {
+    constexpr int CH = HD / 4;
+#pragma unroll 8
+    for (int c = threadIdx.x; c < FT * CH; c += FTHREADS) {
+        const int t = c / CH, e = (c % CH) * 4, row = row_s[t];
+        cp16(dst + t * LD + e, row >= 0 ? pool + (size_t)row * HD + e : pool, row >= 0);
+    }
+}
+
+template <int HD>
+constexpr int decode_smem_floats() { return FT * (HD + 4) + FT * HD + GDEC * HD + FT * GDEC + 3 * GDEC; }
+
+template <int HD>
+__global__ void __launch_bounds__(FTHREADS)
+attn_f32_decode_kernel(const AttnParams p) {
+    constexpr int LD = HD + 4, DW = HD / 4;                  // lanes that hold a row's dims, four each
+    extern __shared__ __align__(16) float sm[];
+    float* k_s = sm;                                         // [FT][LD]
+    float* v_s = k_s + FT * LD;                              // [FT][HD]
+    float* q_s = v_s + FT * HD;                              // [GDEC][HD]
+    float* p_s = q_s + GDEC * HD;                            // [FT][GDEC]: scores, then weights
+    float* m_s = p_s + FT * GDEC;                            // [GDEC] running maximum, sum, factor of the tile before
+    float* l_s = m_s + GDEC;
+    float* a_s = l_s + GDEC;
+    __shared__ int row_s[FT];
+    const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+    const int slot = p.row_slot[b];
+    if (slot < 0) return;
+    const int tok = p.row_q_start[b], pos = p.row_ctx_len[b], G = p.G;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0, hi = pos + 1;
+    if (p.chunk > 0) lo = max(lo, (pos / p.chunk) * p.chunk);
+    if (p.n_splits > 1) { lo = max(lo, split * p.split_len); hi = min(hi, (split + 1) * p.split_len); }
+    const size_t head0 = (size_t)tok * p.n_q + kvh * G;      // the group's first (token, head)
+    if (lo >= hi) {                                          // (a split without keys: only its sum is looked at)
+        if (p.n_splits > 1 && tid < G) p.part_l[(head0 + tid) * p.n_splits + split] = 0.f;
+        return;
+    }
+    const float* qg = static_cast<const float*>(p.q) + head0 * HD;
+    for (int e = tid; e < G * HD; e += FTHREADS) q_s[e] = qg[e] * p.scale;
+    if (tid < GDEC) { m_s[tid] = -INFINITY; l_s[tid] = 0.f; }
+    float acc[GDEC][4];
+#pragma unroll
+    for (int g = 0; g < GDEC; ++g) acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0.f;
+    constexpr int KS = FTHREADS / DW;                        // shares of a tile's keys in the value phase
+    const int d4 = (tid % DW) * 4, share = tid / DW;
+
+    for (int t0 = lo / FT * FT; t0 < hi; t0 += FT) {
+        __syncthreads();                                     // the tile before is consumed
+        tile_rows(p, slot, kvh, t0, lo, hi, row_s);
+        __syncthreads();
+        load_tile<HD, LD>(k_s, static_cast<const float*>(p.k_pool), row_s);
+        commit();
+        load_tile<HD, HD>(v_s, static_cast<const float*>(p.v_pool), row_s);
+        commit();
+        wait<1>();
+        __syncthreads();
+        // scores: a thread has one key and every second head
+        {
+            const int key = tid & (FT - 1), h0 = tid / FT;
+            float s[GDEC / 2];
+#pragma unroll
+            for (int i = 0; i < GDEC / 2; ++i) s[i] = 0.f;
+            const float* kr = k_s + key * LD;
+#pragma unroll 4
+            for (int e = 0; e < HD; e += 4) {
+                const float4 k4 = *reinterpret_cast<const float4*>(kr + e);
+#pragma unroll
+                for (int i = 0; i < GDEC / 2; ++i) {
+                    if (h0 + 2 * i >= G) break;
+                    const float4 q4 = *reinterpret_cast<const float4*>(q_s + (h0 + 2 * i) * HD + e);
+                    s[i] = fmaf(q4.x, k4.x, s[i]); s[i] = fmaf(q4.y, k4.y, s[i]);
+                    s[i] = fmaf(q4.z, k4.z, s[i]); s[i] = fmaf(q4.w, k4.w, s[i]);
+                }
+            }
+            const bool valid = t0 + key >= lo && t0 + key < hi;
+#pragma unroll
+            for (int i = 0; i < GDEC / 2; ++i)
+                if (h0 + 2 * i < G) p_s[key * GDEC + h0 + 2 * i] = valid ? s[i] : -INFINITY;
+        }
+        __syncthreads();
+        for (int g = warp; g < G; g += FTHREADS / 32) {      // softmax: a warp per head, two keys per lane
+            const float s0 = p_s[lane * GDEC + g], s1 = p_s[(lane + 32) * GDEC + g];
+            const float m_old = m_s[g], m_new = fmaxf(m_old, warp_max(fmaxf(s0, s1)));
+            const float e0 = s0 == -INFINITY ? 0.f : expf(s0 - m_new), e1 = s1 == -INFINITY ? 0.f : expf(s1 - m_new);
+            const float sum = warp_sum(e0 + e1);
+            p_s[lane * GDEC + g] = e0;
+            p_s[(lane + 32) * GDEC + g] = e1;
+            __syncwarp();
+            if (lane == 0) {
+                const float alpha = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
+                a_s[g] = alpha;
+                l_s[g] = l_s[g] * alpha + sum;
+                m_s[g] = m_new;
+            }
+        }
+        wait<0>();
+        __syncthreads();
+#pragma unroll
+        for (int g = 0; g < GDEC; ++g) {
+            if (g >= G) break;
+            const float al = a_s[g];
+            acc[g][0] *= al; acc[g][1] *= al; acc[g][2] *= al; acc[g][3] *= al;
+        }
+#pragma unroll 4
+        for (int t = share * (FT / KS); t < (share + 1) * (FT / KS); ++t) {
+            const float4 v4 = *reinterpret_cast<const float4*>(v_s + t * HD + d4);
+            float w[GDEC];
+            *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(p_s + t * GDEC);
+            *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(p_s + t * GDEC + 4);
+#pragma unroll
+            for (int g = 0; g < GDEC; ++g) {
+                if (g >= G) break;
+                acc[g][0] = fmaf(w[g], v4.x, acc[g][0]); acc[g][1] = fmaf(w[g], v4.y, acc[g][1]);
+                acc[g][2] = fmaf(w[g], v4.z, acc[g][2]); acc[g][3] = fmaf(w[g], v4.w, acc[g][3]);
+            }
+        }
+    }
+    // the shares' sums, added in order (through the values' place)
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < GDEC; ++g) {
+        if (g >= G) break;
+        *reinterpret_cast<float4*>(v_s + (share * GDEC + g) * HD + d4) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+    }
+    __syncthreads();
+    for (int c = tid; c < G * DW; c += FTHREADS) {
+        const int g = c / DW, e = (c % DW) * 4;
+        float4 o = *reinterpret_cast<const float4*>(v_s + g * HD + e);
+#pragma unroll
+        for (int s = 1; s < KS; ++s) {
+            const float4 x = *reinterpret_cast<const float4*>(v_s + (s * GDEC + g) * HD + e);
+            o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
+        }
+        if (p.n_splits > 1) {
+            const size_t pi = (head0 + g) * p.n_splits + split;
+            if (e == 0) { p.part_m[pi] = m_s[g]; p.part_l[pi] = l_s[g]; }
+            *reinterpret_cast<float4*>(p.part_acc + pi * HD + e) = o;
+        } else {
+            const float inv = l_s[g] > 0.f ? p.out_scale / l_s[g] : 0.f;
+            *reinterpret_cast<float4*>(static_cast<float*>(p.out) + (size_t)tok * p.out_ld + (kvh * G + g) * HD + e) =
+                make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+        }
+    }
+}
+
+constexpr int PR = 64;             // rows (query, head) per CTA of the prompt kernel
+
+template <int HD>
+constexpr int prompt_smem_floats() { return 2 * FT * (HD + 4) + FT * HD; }
+
+template <int HD>
+__global__ void __launch_bounds__(FTHREADS, 2)
+attn_f32_prompt_kernel(const AttnParams p) {
+    constexpr int LD = HD + 4, PLD = FT + 4, TM = 8, TN = 4, TV = HD / 16;     // a thread: 8 rows, 4 keys, TV dims
+    static_assert(PR * PLD <= FT * LD, "the weights take the keys' place");
+    extern __shared__ __align__(16) float sm[];
+    float* q_s = sm;                                         // [PR][LD]
+    float* k_s = q_s + PR * LD;                              // [FT][LD]; then the weights, [PR][PLD]
+    float* p_s = k_s;
+    float* v_s = k_s + FT * LD;                              // [FT][HD]
+    __shared__ int row_s[FT];
+    const int b = blockIdx.z, kvh = blockIdx.y, tile = gridDim.x - 1 - blockIdx.x;      // the longest chains first
+    const int slot = p.row_slot[b];
+    if (slot < 0) return;
+    const int q_len = p.row_q_len[b], G = p.G, QT = p.QT;
+    if (tile * QT >= q_len) return;
+    const int nq = min(QT, q_len - tile * QT), R = nq * G;
+    const int tok0 = p.row_q_start[b] + tile * QT, p_first = p.row_ctx_len[b] + tile * QT;
+    int lo = p.window > 0 ? max(0, p_first - p.window + 1) : 0;
+    if (p.chunk > 0) lo = max(lo, (p_first / p.chunk) * p.chunk);
+    const int hi = p_first + nq;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    // queries of this CTA, scaled (rows beyond R are zero)
+    for (int c = tid; c < PR * (HD / 4); c += FTHREADS) {
+        const int r = c / (HD / 4), e = (c % (HD / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < R) {
+            const int qi = r / G, g = r - qi * G;
+            v = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + ((size_t)(tok0 + qi) * p.n_q + kvh * G + g) * HD + e);
+        }
+        *reinterpret_cast<float4*>(q_s + r * LD + e) = make_float4(v.x * p.scale, v.y * p.scale, v.z * p.scale, v.w * p.scale);
+    }
+    float m_run[TM], l_run[TM], acc[TM][TV];
+    int qpos[TM], first[TM];                                 // position of a row's query, first key it sees
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        m_run[i] = -INFINITY; l_run[i] = 0.f;
+        const int r = i * (PR / TM) + ty;
+        qpos[i] = r < R ? p_first + r / G : -1;
+        first[i] = p.window > 0 ? max(0, qpos[i] - p.window + 1) : 0;
+        if (p.chunk > 0) first[i] = max(first[i], (qpos[i] / p.chunk) * p.chunk);
+#pragma unroll
+        for (int j = 0; j < TV; ++j) acc[i][j] = 0.f;
+    }
+    for (int t0 = lo / FT * FT; t0 < hi; t0 += FT) {
+        __syncthreads();                                     // the tile before is consumed (first time: nothing yet)
+        tile_rows(p, slot, kvh, t0, lo, hi, row_s);
+        __syncthreads();
+        load_tile<HD, LD>(k_s, static_cast<const float*>(p.k_pool), row_s);
+        commit();
+        load_tile<HD, HD>(v_s, static_cast<const float*>(p.v_pool), row_s);
+        commit();
+        wait<1>();
+        __syncthreads();
+        float s[TM][TN];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) s[i][j] = 0.f;
+#pragma unroll 2
+        for (int e = 0; e < HD; e += 4) {
+            float4 k4[TN];
+#pragma unroll
+            for (int j = 0; j < TN; ++j) k4[j] = *reinterpret_cast<const float4*>(k_s + (j * (FT / TN) + tx) * LD + e);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const float4 q4 = *reinterpret_cast<const float4*>(q_s + (i * (PR / TM) + ty) * LD + e);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    s[i][j] = fmaf(q4.x, k4[j].x, s[i][j]); s[i][j] = fmaf(q4.y, k4[j].y, s[i][j]);
+                    s[i][j] = fmaf(q4.z, k4[j].z, s[i][j]); s[i][j] = fmaf(q4.w, k4[j].w, s[i][j]);
+                }
+            }
+        }
+        __syncthreads();                                     // the keys are read: their place takes the weights
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            float mx = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int t = t0 + j * (FT / TN) + tx;
+                if (t < first[i] || t > qpos[i]) s[i][j] = -INFINITY;
+                mx = fmaxf(mx, s[i][j]);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float m_new = fmaxf(m_run[i], mx);
+            float alpha = 1.f, sum = 0.f;
+            if (m_new != -INFINITY) {
+                alpha = expf(m_run[i] - m_new);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) { s[i][j] = expf(s[i][j] - m_new); sum += s[i][j]; }
+            } else {
+#pragma unroll
+                for (int j = 0; j < TN; ++j) s[i][j] = 0.f;
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            l_run[i] = l_run[i] * alpha + sum;
+            m_run[i] = m_new;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) p_s[(i * (PR / TM) + ty) * PLD + j * (FT / TN) + tx] = s[i][j];
+#pragma unroll
+            for (int j = 0; j < TV; ++j) acc[i][j] *= alpha;
+        }
+        wait<0>();
+        __syncthreads();
+        for (int t = 0; t < FT; t += 4) {
+            float4 w4[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) w4[i] = *reinterpret_cast<const float4*>(p_s + (i * (PR / TM) + ty) * PLD + t);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                float v[TV];
+#pragma unroll
+                for (int j = 0; j < TV; j += 4)
+                    *reinterpret_cast<float4*>(v + j) = *reinterpret_cast<const float4*>(v_s + (t + u) * HD + (j / 4) * 64 + tx * 4);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const float w = u == 0 ? w4[i].x : (u == 1 ? w4[i].y : (u == 2 ? w4[i].z : w4[i].w));
+#pragma unroll
+                    for (int j = 0; j < TV; ++j) acc[i][j] = fmaf(w, v[j], acc[i][j]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int r = i * (PR / TM) + ty;
+        if (r >= R) continue;
+        const int qi = r / G, g = r - qi * G;
+        const float inv = l_run[i] > 0.f ? p.out_scale / l_run[i] : 0.f;
+        float* o = static_cast<float*>(p.out) + (size_t)(tok0 + qi) * p.out_ld + (kvh * G + g) * HD;
+#pragma unroll
+        for (int j = 0; j < TV; j += 4)
+            *reinterpret_cast<float4*>(o + (j / 4) * 64 + tx * 4) =
+                make_float4(acc[i][j] * inv, acc[i][j + 1] * inv, acc[i][j + 2] * inv, acc[i][j + 3] * inv);
+    }
+}
+
+template <typename KernelT>
+int configure(KernelT k, int smem, bool& done) {
+    if (done) return 0;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return fail(-3, "attention: cannot get %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    done = true;
+    return 0;
+}
+
+template <int HD>
+int launch_f32(const AttnParams& p0, int n_rows, int max_q_len, cudaStream_t stream) {
+    AttnParams p = p0;
+    if (max_q_len == 1 && p.G <= GDEC) {
+        constexpr int smem = decode_smem_floats<HD>() * (int)sizeof(float);
+        static bool done = false;
+        const int rc = configure(attn_f32_decode_kernel<HD>, smem, done);
+        if (rc != 0) return rc;
+        attn_f32_decode_kernel<HD><<<dim3(p.n_splits, p.n_kv, n_rows), FTHREADS, smem, stream>>>(p);
+        return check_launch("attention_f32_decode");
+    }
+    if (p.n_splits > 1 || p.G > PR) return 1;
+    p.QT = PR / p.G < max_q_len ? PR / p.G : max_q_len;
+    constexpr int smem = prompt_smem_floats<HD>() * (int)sizeof(float);
+    static bool done = false;
+    const int rc = configure(attn_f32_prompt_kernel<HD>, smem, done);
+    if (rc != 0) return rc;
+    attn_f32_prompt_kernel<HD><<<dim3((max_q_len + p.QT - 1) / p.QT, p.n_kv, n_rows), FTHREADS, smem, stream>>>(p);
+    return check_launch("attention_f32_prompt");
+}
+
+}  // namespace
+
+// Heads of 64 or 128 for keys and values alike, no cap, kept first keys, keyless term, repeated heads or 16-bit output; output rows
+// 16-byte aligned.  Returns 1 if it does not take the sizes.
+int launch_attn_f32(const AttnParams& p, int n_rows, int max_q_len, cudaStream_t stream) {
+    if (p.d != p.dv || p.v_ld != p.dv || p.kv_div != 1 || p.softcap > 0.f || (p.keep_first > 0 && p.window > 0) ||
+        p.sink != nullptr || p.v_rep != 1 || (uintptr_t)p.out % 16 != 0 || p.out_ld % 4 != 0)
+        return 1;
+    if (p.d == 128) return launch_f32<128>(p, n_rows, max_q_len, stream);
+    if (p.d == 64) return launch_f32<64>(p, n_rows, max_q_len, stream);
+    return 1;
+}
+
+}  // namespace fd

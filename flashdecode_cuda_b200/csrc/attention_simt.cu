@@ -22,8 +22,8 @@
 // Tile and split boundaries are fixed in absolute token index, so the order
 // of the floating-point sums of a query does not depend on what else is in
 // the batch.  Scores, softmax and the value sum are float; bfloat16 is only a
-// storage format here.  This is the attention of the true 32-bit path and the
-// fallback for head sizes the tensor-core kernels do not take.
+// storage format here.  This is the fallback for the head sizes and options that
+// the tensor-core kernels and, in float32, attention_f32.cu do not take.
 #include <math.h>
 
 #include "attention.cuh"
@@ -589,6 +589,7 @@ static int attention_impl(const void* q, const void* k_pool, const void* v_pool,
         if (tc_options && dv == d) rc = launch_attn_prefill_tcgen05(p, n_rows, T, max_q_len, stream);
         if (rc == 1) rc = launch_attn_prefill_mma_ext(p, n_rows, max_q_len, stream);
     }
+    if (dtype == 0 && use_mma != 0) rc = launch_attn_f32(p, n_rows, max_q_len, stream);
     if (rc == 1)
         rc = dtype == 0 ? launch_attn<float>(p, n_rows, max_q_len, stream)
                         : launch_attn<bf16>(p, n_rows, max_q_len, stream);

@@ -18,6 +18,10 @@ MAX_SPLITS = 32
 PREFETCH_BYTES = 16 << 20   # an output projection up to this size is asked for ahead by the decode q/k/v kernel (whole; a 16 MB
                             # beginning of a larger one made the step slower: + 1.4 % at the sizes of Qwen2.5-7B, batch 8)
 FP32_SPLIT_LEN = 256      # keys per split of a decode step in float32
+# The same for attention without options: one tile of the kernel for heads of 64 and 128, so that a CTA is one chain of lookups,
+# loads, scores and values (csrc/attention_f32.cu) - where no sequence of the cache is so long that the merge would have
+# more than 512 splits to add.
+FP32_TILE_LEN, FP32_MAX_SPLITS = 64, 512
 
 
 def plan_splits(n_rows: int, n_kv: int, kv_len_bound: int, sm_count: int):
@@ -38,6 +42,13 @@ def plan_splits(n_rows: int, n_kv: int, kv_len_bound: int, sm_count: int):
     split_len = max(128, -(-split_len // 32) * 32)
     n_splits = max(1, -(-kv_len_bound // split_len))
     return n_splits, split_len
+
+
+def fp32_splits(ctx):
+    """(n_splits, split_len) of a decode step in float32.  The splits have a fixed length (one per cache), so that where
+    a sequence's partial sums are cut - and with it every bit of its result - depends on nothing but its own length."""
+    split_len = FP32_TILE_LEN if ctx.cache.max_len <= FP32_TILE_LEN * FP32_MAX_SPLITS else FP32_SPLIT_LEN
+    return max(1, -(-ctx.kv_len_bound // split_len)), split_len
 
 
 @register_part("mixer", "gqa_attention")
@@ -156,10 +167,7 @@ class GQAAttention(Mixer):
         attn = ws.get("attn", (T, self.n_q * d), x.dtype)
         n_splits, split_len, scratch = 1, 0, None
         if ctx.max_q_len == 1 and x.dtype == torch.float32:
-            # the 32-bit path: splits of a fixed length, so that where a sequence's partial sums are cut - and with
-            # it every bit of its result - depends on nothing but its own length
-            split_len = FP32_SPLIT_LEN
-            n_splits = max(1, -(-ctx.kv_len_bound // split_len))
+            n_splits, split_len = fp32_splits(ctx)
             if n_splits > 1:
                 scratch = ws.get("attn_scratch", (K.attention_scratch_floats(T, self.n_q, d, n_splits),),
                                  torch.float32)

@@ -854,6 +854,25 @@ def test_attention_decode_tensor_cores_window_and_far_key(window, decode_form):
         assert rel(got, want) < TOL["bfloat16"], key_pos
 
 
+@pytest.mark.parametrize("n_q,n_kv,d,bs,window", [(12, 2, 128, 16, 0), (8, 1, 64, 64, 0), (3, 3, 128, 7, 0), (16, 2, 64, 16, 70),
+                                                  (9, 1, 128, 32, 0), (64, 1, 64, 16, 100)])
+def test_attention_f32_decode_and_prompts(n_q, n_kv, d, bs, window):
+    """The 32-bit kernels for heads of 64 and 128: one query head per group up to one more than the decode kernel takes (and the
+    most the prompt kernel takes); contexts at the edges of its 64-key tiles and of splits, splits of one tile, of more and off
+    the tiles; prompts whose rows fill a CTA's 64, leave a remainder, and go on after cached keys."""
+    ctx = [0, 1, 62, 63, 64, 65, 127, 128, 300]
+    for n_splits, split_len in ((1, 0), (5, 64), (3, 128), (4, 96)):
+        got, want, pad = run_attention("float32", n_q, n_kv, d, bs, ctx=ctx, new=[1] * len(ctx), window=window,
+                                       n_splits=n_splits, split_len=split_len, pad_rows=1, fn=K.attention)
+        assert rel(got, want) < TOL["float32"], (n_splits, split_len)
+        if n_splits > 1:
+            assert float(pad.float().abs().max()) == 0.0
+    per = 64 // (n_q // n_kv)
+    for c, new in (([0, 0, 0], [1, per + 1, 2 * per]), ([63, 64, 130], [70, 3, 65]), ([0], [200])):
+        got, want, _ = run_attention("float32", n_q, n_kv, d, bs, ctx=c, new=new, window=window, fn=K.attention)
+        assert rel(got, want) < TOL["float32"], (c, new)
+
+
 def test_attention_refuses_what_it_cannot_do():
     with pytest.raises(K.KernelError, match="head size"):
         run_attention("float32", 4, 2, 20, 4, ctx=[0], new=[3])
