@@ -667,8 +667,23 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 }
 
 // ---- host side ------------------------------------------------------------
-int g_tc_wide = 1;      // 2: the two-SM kernel where N >= 256; 1: the persistent one-SM kernel (128 x 256 tiles, or 128 x 128
-                        // where those number no more than the SMs); 3: the same with 128 x 256 tiles always; 0: 128 x 128 tiles, one per CTA
+int g_tc_wide = 1;      // where N >= 256: 1: the persistent one-SM kernel (128 x 256 tiles, or 128 x 128 where those number no more
+                        // than the SMs), or the two-SM kernel where pair_pays; 2: the two-SM kernel; 3: one SM and 128 x 256 tiles
+                        // always; 0: 128 x 128 tiles, one per CTA
+
+// Whether two SMs per 256 x 256 tile beat one SM per 128 x 256: a pair's round takes 0.87 of the time where the products of a tile
+// are long (measured us, pair / one SM: gate/up of 5,120 columns at 1,200 and 2,048 rows 250 / 280 and 378 / 442, of 3,584 columns
+// at 2,048 rows 376 / 444, q/k/v of the same 142 / 162 and 67 / 78) and 0.94 at 1,536 columns (gate/up at 2,048 and 9,208 rows
+// 83 / 89 and 336 / 365), where the q/k/v epilogue is the longer part and the pair slower (78 / 68) - but its rounds
+// are coarser (gate/up of 3,584 columns at 384 rows: four instead of three, 103 / 91).
+static bool pair_pays(const TcParams& p, int sms) {
+    const long long tn = (p.N + TW_BN - 1) / TW_BN, tiles = (long long)((p.M + TC_BM - 1) / TC_BM) * tn;
+    const long long pairs = (long long)((p.M + 2 * TC_BM - 1) / (2 * TC_BM)) * tn;
+    const long long rounds = (tiles + sms - 1) / sms, pair_rounds = (pairs + sms / 2 - 1) / (sms / 2);
+    if (rounds < 2) return false;
+    if (p.K < 2048) return p.mode != 4 && p.M >= 1024 && pair_rounds * 19 < rounds * 20;
+    return pair_rounds * 9 < rounds * 10;
+}
 
 // w_stack: matrices in the stack w [w_stack][N, K] (the grouped form; 1: the plain product).
 static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRope& ra, cudaStream_t stream,
@@ -689,10 +704,10 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
     }
     const int tiles_m = (p.M + TC_BM - 1) / TC_BM;
     const bool wide = g_tc_wide && p.N >= TW_BN;
-    const bool pair = wide && g_tc_wide == 2;
     // 128 x 128 tiles where even those give no CTA a second tile: twice the CTAs at work.  (Where CTAs would take two
     // of them in a row, the wider tile is faster: q/k/v of 2,048 tokens 22.5 against 25.3 us.)
-    const bool narrow = wide && !pair && g_tc_wide != 3 && (long long)tiles_m * ((p.N + TN_BN - 1) / TN_BN) <= sms;
+    const bool narrow = wide && g_tc_wide == 1 && (long long)tiles_m * ((p.N + TN_BN - 1) / TN_BN) <= sms;
+    const bool pair = wide && (g_tc_wide == 2 || (g_tc_wide == 1 && !narrow && p.tile_expert == nullptr && pair_pays(p, sms)));
     CUtensorMap mx, mw;
     if (pair) {
         const int tiles_m2 = (p.M + 2 * TC_BM - 1) / (2 * TC_BM), tiles_n = (p.N + TW_BN - 1) / TW_BN;
@@ -734,8 +749,8 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
 
 using namespace fd;
 
-// Which tiling the products use from now on where N >= 256 (1, the default: persistent CTAs with 128 x 256 tiles, or
-// with 128 x 128 tiles where those number no more than the SMs; 3: persistent CTAs with 128 x 256 tiles always; 2: two
+// Which tiling the products use from now on where N >= 256 (1, the default: persistent CTAs with 128 x 256 tiles,
+// with 128 x 128 tiles where those number no more than the SMs, or two SMs per tile where that is faster; 3: persistent CTAs with 128 x 256 tiles always; 2: two
 // SMs per 256 x 256 tile; 0: 128 x 128 tiles, one per CTA, everywhere).  For tests and measurements.
 extern "C" int fd_gemm_tc_set_wide(int on) {
     g_tc_wide = on < 0 ? 0 : (on > 3 ? 3 : on);

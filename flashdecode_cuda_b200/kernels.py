@@ -147,6 +147,9 @@ def _declare(L: ctypes.CDLL) -> None:
         "fd_moe_combine": [P, P, P, P, P, P, P, I, I, I, I, I, P],
         "fd_moe_gather": [P, P, P, P, I, I, I, I, P],
         "fd_gemm_tc_grouped": [P, P, P, I, I, I, I, I, P, P, F, P, P],
+        "fd_dense_mixer": [P, P, P],
+        "fd_dense_gate_up": [P, P],
+        "fd_dense_layers": [P, P, I],
         "fd_sample": [P, I, I, P, P, P, c_ulonglong, P, P, P, P],
         "fd_copy_h2d_async": [P, P, LL, P],
         "fd_copy_d2h_sync": [P, P, LL, P],
