@@ -25,6 +25,7 @@ from ..parts.base import KVRequest, LayerCache, Runtime
 from ..registry import architecture, part_class
 from ..weights import loader as W
 from .blueprint import ModelBlueprint, PartSpec
+from .native import DensePrompts
 
 Want = Union[str, None, Sequence[Sequence[int]]]
 
@@ -156,6 +157,8 @@ class Model:
         self.trace: Optional[Dict[str, torch.Tensor]] = None    # set to {} to record per-layer activations
         self.last_meta_host: Optional[np.ndarray] = None        # the index array of the last prepared step
         self.bound = False
+        # prompt steps of dense models are launched from native code; None: every step goes through the parts
+        self.native: Optional[DensePrompts] = None
 
     # ------------------------------------------------------------------ build
     @classmethod
@@ -220,6 +223,7 @@ class Model:
         on_dev = {n: W.cast(by_name[n], t, self.dtype, self.device) for n, t in tensors.items()}
         for p in self.all_parts():
             p.bind(on_dev, self.rt)
+        self.native = DensePrompts.of(self) if self.device.type == "cuda" else None
         self.bound = True
         return self
 
@@ -402,9 +406,12 @@ class Model:
             # stream operations may read the embedding output again later in the step
             embedded = ctx.ws.get("embedded", (ctx.T, self.hidden_size), torch.float32)
             embedded.copy_(resid)
-        caches = self._layer_caches(ctx.cache)
         delta = None
-        for i, run in enumerate(self.schedule):
+        entries = self.schedule
+        if self.native is not None and self.trace is None and self.native.takes(ctx):
+            delta, entries = self.native.run(ctx, resid), []
+        caches = self._layer_caches(ctx.cache) if entries else []
+        for i, run in enumerate(entries):
             if run.before is not None:
                 # the operation adds the pending delta itself and leaves the new stream in resid
                 if run.before_index is None:

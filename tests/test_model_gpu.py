@@ -115,6 +115,48 @@ def test_long_decoding(engines, folders, name, dtype):
     eng.model.check_status()
 
 
+@pytest.mark.parametrize("block_size", [7, 64])
+@pytest.mark.parametrize("name", CONFIGS)
+def test_native_prompt_steps_change_no_bit(engines, name, block_size):
+    """Prompt steps launched from native code give the bits that the parts give, and leave the same keys and values: at the edges
+    of the streaming products (16 | 17 and 128 | 129 tokens), whole, in portions after cached keys, and with a sequence that
+    brings a single token."""
+    m = engines[(name, "bfloat16")].model
+    assert m.native is not None
+    native = m.native
+    taken = []
+
+    def steps(on):
+        m.native = native if on else None
+        cache = m.new_cache(max_tokens=2048, block_size=block_size, max_slots=6)
+        out = []
+        limit = min(cache.max_len, 120 if name == "A" else 250)      # the configurations' longest sequences
+        for lens in ([9, 8], [limit // 2, 1], [16, 1], [limit, limit - 1, 3], [17], [limit] * 4):
+            slots = [cache.admit() for _ in lens]
+            for at in (0, 60, 190):
+                live = [i for i, n in enumerate(lens) if n > at]
+                if not live:
+                    break
+                end = {0: 60, 60: 190, 190: 1 << 30}[at]
+                reqs = [prompts_for(m.vocab_size, [n], seed=60 + n)[0][at:end] for n in lens]
+                if on:
+                    before = native.run
+                    native.run = lambda *a, f=before: (taken.append(1), f(*a))[1]
+                out.append(m.step(cache, [slots[i] for i in live], [reqs[i] for i in live], "all").clone())
+                if on:
+                    del native.run
+            for s in slots:
+                out += list(cache.gather(s, 0, 0))
+                cache.release(s)
+        return out
+    try:
+        a, b = steps(True), steps(False)
+    finally:
+        m.native = native
+    m.check_status()
+    assert len(taken) >= 6 and len(a) == len(b) and all(torch.equal(x, y) for x, y in zip(a, b))
+
+
 @pytest.mark.parametrize("name", ["D", "E"])
 def test_asking_l2_for_what_comes_next_changes_no_bit(engines, folders, name, monkeypatch):
     """Decode steps hand ``ctx.upcoming`` (the weights the step streams next) to their kernels, which ask L2
