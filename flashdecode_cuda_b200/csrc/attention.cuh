@@ -60,11 +60,14 @@ int launch_attn_prefill_mma(const AttnParams& p, int n_rows, int max_q_len, cuda
 // decode steps and later portions of prompts over one cached row per position that is every head's key and, its first dv
 // dimensions, every head's value (n_kv 1, bfloat16)
 int launch_attn_latent_mma(const AttnParams& p, const int* tok_row, int T, cudaStream_t stream);
-// the true 32-bit path for heads of 64 and 128 (attention_f32.cu); same return convention
+// the true 32-bit path for heads of 64 and 128 (attention_rows.cu); same return convention
 int launch_attn_f32(const AttnParams& p, int n_rows, int max_q_len, cudaStream_t stream);
+// decode steps in bfloat16 with kept first keys or mixed heads, heads of 64 and 128 (attention_rows.cu); same return convention
+int launch_attn_rows_ext(const AttnParams& p, int n_rows, cudaStream_t stream);
 // prompt steps with capped scores, kept first keys, a keyless softmax term or repeated value heads (head sizes 64 and 128)
 int launch_attn_prefill_mma_ext(const AttnParams& p, int n_rows, int max_q_len, cudaStream_t stream);
 // the same on the tcgen05 tensor cores (head size 128, block sizes 8..128 that divide 128)
-int launch_attn_prefill_tcgen05(const AttnParams& p, int n_rows, int T, int max_q_len, cudaStream_t stream);
+int launch_attn_prefill_tcgen05(const AttnParams& p, int n_rows, int T, int max_q_len, cudaStream_t stream,
+                                float* scratch = nullptr, int kv_len = 0, const int* tok_row = nullptr);
 
 }  // namespace fd

@@ -37,6 +37,10 @@
 // heads, so no long tile starts in a late wave.  A prompt so short that this
 // grid leaves SMs empty runs a second form of the kernel (SPLIT below): 128
 // queries per CTA, their key tiles dealt to the two groups of softmax warps.
+// Where even these CTAs fill less than half of the GPU and walk many keys (a
+// prompt's later portions), the keys are cut into parts, a CTA each, whose
+// unnormalised outputs a second kernel adds up (384 new tokens behind 2,600
+// cached ones, 12 heads: 36 CTAs, 28 us without parts).
 //
 // DENSE: the keys and values of whole prompts as plain rows, one per token of the step, before anything is paged: kv
 // [T, heads * (64 KN + 64 VS)] holds every head's own key dimensions and its value (a latent attention's expanded keys and
@@ -202,7 +206,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // The head is the fastest grid index and the query tiles run from the last to the first: CTAs start in the
     // order of their work (a causal tile's key range grows with its position), the longest of every head
     // first, and the heads of a group walk the same keys at the same time.
-    const int tile = gridDim.y - 1 - blockIdx.y, h = blockIdx.x, b = blockIdx.z;
+    const int tile = gridDim.y - 1 - blockIdx.y, h = blockIdx.x;
+    const int parts = SPLIT && !DENSE ? p.n_splits : 1, b = blockIdx.z / parts, part = blockIdx.z - b * parts;
     const int slot = p.row_slot[b];
     const int q_len = slot >= 0 ? p.row_q_len[b] : 0;
     constexpr int CTA_ROWS = SPLIT ? TA_BM : TA_ROWS;        // query tokens of a CTA
@@ -227,6 +232,17 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         q_hi[qt] = p_first[qt] + nq[qt];
         q_lo[qt] = p.window > 0 ? max(0, p_first[qt] - p.window + 1) : 0;
         if (p.chunk > 0) q_lo[qt] = max(q_lo[qt], (p_first[qt] / p.chunk) * p.chunk);    // chunked visibility
+    }
+    if (parts > 1) {
+        // this CTA's share of the key tiles, in whole tiles; without any it leaves sums of zero
+        const int first = q_lo[0] / TA_BN, all = (q_hi[0] + TA_BN - 1) / TA_BN - first, per = (all + parts - 1) / parts;
+        const int from = (first + part * per) * TA_BN, to = (first + min(all, (part + 1) * per)) * TA_BN;
+        if (part * per >= all) {
+            for (int i = threadIdx.x; i < nq[0]; i += TA_THREADS) p.part_l[((size_t)(tok0 + i) * p.n_q + h) * parts + part] = 0.f;
+            return;                                          // uniform for the CTA; nothing allocated yet
+        }
+#pragma unroll
+        for (int qt = 0; qt < TA_NQ; ++qt) { q_lo[qt] = max(q_lo[qt], from); q_hi[qt] = min(q_hi[qt], to); }
     }
     const int lo = q_lo[0];
     const int hi = !SPLIT && nq[1] > 0 ? q_hi[1] : q_hi[0];
@@ -559,10 +575,18 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const float a0 = m0 == -INFINITY ? 0.f : ta_ex2(m0 - m);
                 const float a1 = m1 == -INFINITY ? 0.f : ta_ex2(m1 - m);
                 float l = l_run * a0 + l1 * a1;
+                if (parts > 1) {
+                    // left to the merge: the sum and the output over this part's keys, relative to its maximum (natural)
+                    const size_t row = ((size_t)(tok0 + r) * p.n_q + h) * parts + part;
+                    if (r < nq[qt]) { p.part_m[row] = m * 0.6931471805599453f; p.part_l[row] = l; }
+                    w_own = a0;
+                    w_other = a1;
+                } else {
                 if (p.sink != nullptr && l > 0.f) l += ta_ex2(sink_log2 - m);
                 const float inv = l > 0.f ? p.out_scale / l : 0.f;
                 w_own = a0 * inv;
                 w_other = a1 * inv;
+                }
                 if (has_other) o_other = o_x + r;
             }
         }
@@ -583,7 +607,13 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
                     for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * w_own);
                 }
-                if (r < nq[qt]) {
+                if (parts > 1) {
+                    if (r < nq[qt]) {
+                        float* dst = p.part_acc + (((size_t)(tok0 + r) * p.n_q + h) * parts + part) * DV + c0;
+#pragma unroll
+                        for (int c = 0; c < 32; c += 4) *reinterpret_cast<uint4*>(dst + c) = make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+                    }
+                } else if (r < nq[qt]) {
                     if (DENSE && grow != nullptr) {            // the heads' output gate
 #pragma unroll
                         for (int c = 0; c < 32; c += 8) {
@@ -617,6 +647,42 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
+}
+
+// Adds up the parts of every (token, head), a warp each, four dimensions a lane: m = max m_s, out = sum acc_s e^(m_s - m) / sum
+// l_s e^(m_s - m).  A part without visible keys (l_s = 0) is left out; tokens of padding rows are left alone, as above.
+constexpr int TA_MAX_PARTS = 8;
+
+__global__ void __launch_bounds__(256)
+attn_prompt_merge_kernel(const AttnParams p, const int* __restrict__ tok_row, int n) {
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;      // row = token * n_q + head
+    if (row >= n) return;
+    const int tok = row / p.n_q, h = row - tok * p.n_q;
+    if (p.row_slot[tok_row[tok]] < 0) return;
+    float l_s[TA_MAX_PARTS], m_s[TA_MAX_PARTS];
+    float4 a[TA_MAX_PARTS];
+#pragma unroll
+    for (int s = 0; s < TA_MAX_PARTS; ++s) {
+        l_s[s] = s < p.n_splits ? p.part_l[(size_t)row * p.n_splits + s] : 0.f;
+        m_s[s] = s < p.n_splits ? p.part_m[(size_t)row * p.n_splits + s] : 0.f;
+        a[s] = s < p.n_splits ? *reinterpret_cast<const float4*>(p.part_acc + ((size_t)row * p.n_splits + s) * TA_D + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float m = p.sink != nullptr ? p.sink[h] : -INFINITY;
+#pragma unroll
+    for (int s = 0; s < TA_MAX_PARTS; ++s) if (l_s[s] > 0.f) m = fmaxf(m, m_s[s]);
+    float l = p.sink != nullptr ? expf(p.sink[h] - m) : 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int s = 0; s < TA_MAX_PARTS; ++s) {
+        if (!(l_s[s] > 0.f)) continue;
+        const float w = expf(m_s[s] - m);
+        l = fmaf(l_s[s], w, l);
+        o.x = fmaf(a[s].x, w, o.x); o.y = fmaf(a[s].y, w, o.y); o.z = fmaf(a[s].z, w, o.z); o.w = fmaf(a[s].w, w, o.w);
+    }
+    const float inv = l > 0.f ? p.out_scale / l : 0.f;
+    const __nv_bfloat162 lo2 = __floats2bfloat162_rn(o.x * inv, o.y * inv), hi2 = __floats2bfloat162_rn(o.z * inv, o.w * inv);
+    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.out) + (size_t)tok * p.out_ld + h * TA_D + lane * 4) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo2), *reinterpret_cast<const uint32_t*>(&hi2));
 }
 
 // ---- host side ------------------------------------------------------------
@@ -690,9 +756,9 @@ static int ta_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
     // Two query tiles per CTA share every key tile; while that leaves SMs without a CTA, one query tile per
     // CTA with its key tiles dealt to the two softmax groups finishes sooner.
     const int shared_ctas = ((max_q_len + TA_ROWS - 1) / TA_ROWS) * p.n_q * n_rows;
-    const bool split = g_ta_form == 2 || (g_ta_form == 0 && shared_ctas < ta_sm_count());
+    const bool split = p.n_splits > 1 || g_ta_form == 2 || (g_ta_form == 0 && shared_ctas < ta_sm_count());
     if (split) {
-        dim3 grid(p.n_q, (max_q_len + TA_BM - 1) / TA_BM, n_rows);
+        dim3 grid(p.n_q, (max_q_len + TA_BM - 1) / TA_BM, n_rows * (DENSE ? 1 : p.n_splits));
         attn_prefill_tcgen05_kernel<KS, VS, true, DENSE><<<grid, TA_THREADS, smem_split, stream>>>(mq, mk, mv, mr, p, g_tc_wait_ns, g_tc_skip_last);
     } else {
         dim3 grid(p.n_q, (max_q_len + TA_ROWS - 1) / TA_ROWS, n_rows);
@@ -701,10 +767,24 @@ static int ta_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
     return check_launch("attention_prefill_tcgen05");
 }
 
+// Into how many parts a prompt step's keys are cut: as many as keep one CTA per SM, with four key tiles each (two for
+// each of a CTA's groups) or more; 1 where the CTAs fill more than half of the GPU.
+static int ta_parts(int n_q, int n_rows, int max_q_len, int kv_len) {
+    if (g_ta_form != 0) return 1;
+    const long long ctas = (long long)n_q * ((max_q_len + TA_BM - 1) / TA_BM) * n_rows;
+    const long long fit = ta_sm_count() / ctas, most = (kv_len + TA_BN - 1) / TA_BN / 4;
+    const long long parts = fit < most ? fit : most;
+    return parts < 2 ? 1 : (parts > TA_MAX_PARTS ? TA_MAX_PARTS : (int)parts);
+}
+
 // Returns 1 when it does not take the sizes (the caller falls back to the mma.sync kernel):
-// head size 128, block size a multiple of 8 that divides 128, no split of the keys.
-int launch_attn_prefill_tcgen05(const AttnParams& p, int n_rows, int T, int max_q_len, cudaStream_t stream) {
+// head size 128, block size a multiple of 8 that divides 128, no split of the keys.  With `scratch` (p.part_acc; fd_attn_prompt_scratch_floats
+// of it, for sequences of up to kv_len tokens) the kernel may cut the keys into parts of its own.
+int launch_attn_prefill_tcgen05(const AttnParams& p0, int n_rows, int T, int max_q_len, cudaStream_t stream, float* scratch,
+                                int kv_len, const int* tok_row) {
+    AttnParams p = p0;
     if (p.d != TA_D || p.n_splits != 1) return 1;
+    const int parts = scratch != nullptr ? ta_parts(p.n_q, n_rows, max_q_len, kv_len) : 1;
     const int bs = p.block_size;
     if (bs < 8 || bs > 128 || bs % 8 != 0 || 128 % bs != 0) return 1;
     if ((max_q_len + TA_BM - 1) / TA_BM > 65535 || n_rows > 65535) return 1;
@@ -714,7 +794,15 @@ int launch_attn_prefill_tcgen05(const AttnParams& p, int n_rows, int T, int max_
     const int box = bs < TA_BN ? bs : TA_BN;
     if (ta_map(p.k_pool, pool_rows, TA_D, box, &mk) != 0) return 1;
     if (ta_map(p.v_pool, pool_rows, TA_D, box, &mv) != 0) return 1;
-    return ta_launch<2, 2, false>(mq, mk, mv, mk, p, n_rows, max_q_len, stream);
+    if (parts > 1 && (long long)n_rows * parts <= 65535) {
+        const size_t n = (size_t)T * p.n_q * parts;
+        p.n_splits = parts;
+        p.part_acc = scratch; p.part_m = scratch + n * TA_D; p.part_l = p.part_m + n;
+    }
+    const int rc = ta_launch<2, 2, false>(mq, mk, mv, mk, p, n_rows, max_q_len, stream);
+    if (rc != 0 || p.n_splits == 1) return rc;
+    attn_prompt_merge_kernel<<<(T * p.n_q + 7) / 8, 256, 0, stream>>>(p, tok_row, T * p.n_q);
+    return check_launch("attention_prompt_merge");
 }
 
 // Whole prompts with keys and values as plain rows (DENSE above).  kv [T, n_q * (64 kn + dv)], rot [T, d - 64 kn] (null when
@@ -758,6 +846,13 @@ extern "C" int fd_attention_dense(const void* q, const void* kv, const void* rot
     const int rc = fd::launch_attn_prefill_dense(p, kv, rot, n_rows, T, max_q_len, stream);
     FD_REQUIRE(rc != 1, -2, "attention_dense: key parts of %d x 64 and %d, values of %d are not taken", kn, dr, dv);
     return rc;
+}
+
+// Floats of scratch with which a prompt step of T tokens may be cut into parts (0: it would not be).
+extern "C" long long fd_attn_prompt_scratch_floats(int T, int n_q, int d, int n_rows, int max_q_len, int kv_len) {
+    if (d != fd::TA_D || T < 1 || n_rows < 1 || max_q_len < 2) return 0;
+    const int parts = fd::ta_parts(n_q, n_rows, max_q_len, kv_len);
+    return parts > 1 ? (long long)T * n_q * parts * (fd::TA_D + 2) : 0;
 }
 
 // 0: the launcher chooses; 1: two query tiles per CTA; 2: one query tile, its key tiles dealt to the two groups

@@ -23,7 +23,7 @@
 // of the floating-point sums of a query does not depend on what else is in
 // the batch.  Scores, softmax and the value sum are float; bfloat16 is only a
 // storage format here.  This is the fallback for the head sizes and options that
-// the tensor-core kernels and, in float32, attention_f32.cu do not take.
+// the tensor-core kernels and, in float32, attention_rows.cu do not take.
 #include <math.h>
 
 #include "attention.cuh"
@@ -512,7 +512,8 @@ static int attention_impl(const void* q, const void* k_pool, const void* v_pool,
                           int n_splits, int split_len, float* scratch, int* counters, int* status, int use_mma,
                           cudaStream_t stream, const void* prefetch = nullptr, unsigned long long prefetch_bytes = 0,
                           float softcap = 0.f, int keep_first = 0, const float* sink = nullptr, int v_rep = 1,
-                          int out_f32 = 0, int ext_mma = 0, int v_ld = 0, int out_ld = 0, float out_scale = 1.f) {
+                          int out_f32 = 0, int ext_mma = 0, int v_ld = 0, int out_ld = 0, float out_scale = 1.f,
+                          float* prompt_scratch = nullptr, int kv_len = 0) {
     if (n_rows == 0 || T == 0) return 0;
     FD_REQUIRE(softcap >= 0.f && keep_first >= 0 && v_rep >= 1 && (v_rep == 1 || v_rep == n_kv), -2,
                "attention: soft cap %g, %d kept first keys, weights applied to %d value heads of %d", softcap, keep_first,
@@ -581,7 +582,7 @@ static int attention_impl(const void* q, const void* k_pool, const void* v_pool,
         if (rc == 0 && pd.counters != nullptr) return 0;
     }
     else if (use_mma && dtype == 1) {
-        rc = use_mma == 2 ? 1 : launch_attn_prefill_tcgen05(p, n_rows, T, max_q_len, stream);
+        rc = use_mma == 2 ? 1 : launch_attn_prefill_tcgen05(p, n_rows, T, max_q_len, stream, prompt_scratch, kv_len, tok_row);
         if (rc == 1) rc = launch_attn_prefill_mma(p, n_rows, max_q_len, stream);
     }
     if (latent) rc = launch_attn_latent_mma(p, tok_row, T, stream);
@@ -589,6 +590,7 @@ static int attention_impl(const void* q, const void* k_pool, const void* v_pool,
         if (tc_options && dv == d) rc = launch_attn_prefill_tcgen05(p, n_rows, T, max_q_len, stream);
         if (rc == 1) rc = launch_attn_prefill_mma_ext(p, n_rows, max_q_len, stream);
     }
+    if (rc == 1 && ext && ext_mma && !latent && dtype == 1 && max_q_len == 1) rc = launch_attn_rows_ext(p, n_rows, stream);
     if (dtype == 0 && use_mma != 0) rc = launch_attn_f32(p, n_rows, max_q_len, stream);
     if (rc == 1)
         rc = dtype == 0 ? launch_attn<float>(p, n_rows, max_q_len, stream)
@@ -664,7 +666,8 @@ extern "C" int fd_attention_simt(const void* q, const void* k_pool, const void* 
 // a (sequence, KV head) merge the splits itself (it leaves them zero again); without them the
 // separate merge kernel runs.  prefetch / prefetch_bytes (optional, 16-byte aligned): memory that a
 // later kernel streams, which the tensor-core decode kernel asks L2 for when its own reads are
-// through (the other kernels ignore it).
+// through (the other kernels ignore it).  prompt_scratch (optional, fd_attn_prompt_scratch_floats, 16-byte aligned) with kv_len, the
+// longest sequence after the step: a prompt step of few CTAs may cut its keys into parts.
 extern "C" int fd_attention(const void* q, const void* k_pool, const void* v_pool, void* out, int dtype,
                             const int* block_table, int max_blocks, int num_blocks, int block_size,
                             const int* tok_row, const int* row_slot, const int* row_q_start,
@@ -672,12 +675,13 @@ extern "C" int fd_attention(const void* q, const void* k_pool, const void* v_poo
                             int max_q_len, int n_q, int n_kv, int d, float scale, int window, int dv, int chunk,
                             int n_splits, int split_len, float* scratch, int* counters, int* status,
                             const void* prefetch, unsigned long long prefetch_bytes, int out_ld, float out_scale,
-                            cudaStream_t stream) {
-    FD_REQUIRE((uintptr_t)prefetch % 16 == 0, -2, "attention: the memory to prefetch must be 16-byte aligned");
+                            float* prompt_scratch, int kv_len, cudaStream_t stream) {
+    FD_REQUIRE((uintptr_t)prefetch % 16 == 0 && (uintptr_t)prompt_scratch % 16 == 0, -2,
+               "attention: the memory to prefetch and the scratch memory must be 16-byte aligned");
     return attention_impl(q, k_pool, v_pool, out, dtype, block_table, max_blocks, num_blocks, block_size, tok_row,
                           row_slot, row_q_start, row_q_len, row_ctx_len, n_rows, T, max_q_len, n_q, n_kv, d, scale,
                           window, dv, chunk, n_splits, split_len, scratch, counters, status, 1, stream, prefetch, prefetch_bytes,
-                          0.f, 0, nullptr, 1, 0, 0, 0, out_ld, out_scale);
+                          0.f, 0, nullptr, 1, 0, 0, 0, out_ld, out_scale, prompt_scratch, kv_len);
 }
 
 // The same without the tcgen05 kernel: prompts go to the mma.sync kernel (head sizes other than 128 always

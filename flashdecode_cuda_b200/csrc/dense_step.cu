@@ -28,7 +28,7 @@ int fd_attention(const void* q, const void* k_pool, const void* v_pool, void* ou
                  const int* row_q_start, const int* row_q_len, const int* row_ctx_len, int n_rows, int T, int max_q_len,
                  int n_q, int n_kv, int d, float scale, int window, int dv, int chunk, int n_splits, int split_len,
                  float* scratch, int* counters, int* status, const void* prefetch, unsigned long long prefetch_bytes,
-                 int out_ld, float out_scale, cudaStream_t stream);
+                 int out_ld, float out_scale, float* prompt_scratch, int kv_len, cudaStream_t stream);
 }
 
 // One schedule entry; weights and sizes, fixed when the model is bound (engine/native.py has the same order).
@@ -48,7 +48,8 @@ struct FdDenseStep {
     const int *tok_row, *tok_pos, *row_slot, *row_q_start, *row_q_len, *row_ctx_len;
     int* status;
     cudaStream_t stream;
-    long long T, n_rows, max_q_len, num_blocks, block_size;
+    float* attn_scratch;                           // null: the attention's keys are not cut into parts
+    long long T, n_rows, max_q_len, kv_len, num_blocks, block_size;
     long long streams;                             // the products are the weight-streaming kernel's (up to 128 tokens)
     char *k_base[8], *v_base[8];
     const int* table[8];
@@ -79,7 +80,8 @@ extern "C" int fd_dense_mixer(const FdDenseStep* s, const FdDenseLayer* L, const
     return fd_attention(s->q, kp, vp, s->attn, 1, s->table[g], (int)s->max_blocks[g], (int)s->num_blocks, (int)s->block_size,
                         s->tok_row, s->row_slot, s->row_q_start, s->row_q_len, s->row_ctx_len, (int)s->n_rows, T,
                         (int)s->max_q_len, (int)L->n_q, (int)L->n_kv, (int)L->d, (float)L->scale, (int)L->window, (int)L->d,
-                        (int)L->chunk, 1, 0, nullptr, nullptr, s->status, nullptr, 0, 0, 1.f, s->stream);
+                        (int)L->chunk, 1, 0, nullptr, nullptr, s->status, nullptr, 0, 0, 1.f, s->attn_scratch,
+                        (int)s->kv_len, s->stream);
 }
 
 // norm of the stream with the mixer's output added, gate/up with the activation.

@@ -25,7 +25,7 @@ import torch
 
 from .. import kernels as K
 from ..parts import linear
-from ..parts.attention import GQAAttention
+from ..parts.attention import GQAAttention, prompt_scratch
 from ..parts.block import PreNormBlock
 from ..parts.mlp import SwiGLU
 from ..parts.norm import RMSNorm
@@ -42,8 +42,9 @@ class _Layer(ctypes.Structure):
 
 class _Step(ctypes.Structure):
     _fields_ = ([(n, c_void_p) for n in ("resid", "normed", "q", "attn", "mixer_out", "act", "ffn_out", "tok_row", "tok_pos",
-                                         "row_slot", "row_q_start", "row_q_len", "row_ctx_len", "status", "stream")]
-                + [(n, c_longlong) for n in ("T", "n_rows", "max_q_len", "num_blocks", "block_size", "streams")]
+                                         "row_slot", "row_q_start", "row_q_len", "row_ctx_len", "status", "stream",
+                                         "attn_scratch")]
+                + [(n, c_longlong) for n in ("T", "n_rows", "max_q_len", "kv_len", "num_blocks", "block_size", "streams")]
                 + [(n, c_void_p * MAX_GROUPS) for n in ("k_base", "v_base", "table")]
                 + [(n, c_longlong * MAX_GROUPS) for n in ("k_stride", "v_stride", "max_blocks")]
                 + [(n, c_void_p * MAX_POSITIONS) for n in ("cos", "sin")] + [("table_len", c_longlong * MAX_POSITIONS)])
@@ -120,7 +121,9 @@ class DensePrompts:
         s.tok_row, s.tok_pos, s.row_slot = ctx.tok_row.data_ptr(), ctx.tok_pos.data_ptr(), ctx.row_slot.data_ptr()
         s.row_q_start, s.row_q_len = ctx.row_q_start.data_ptr(), ctx.row_q_len.data_ptr()
         s.row_ctx_len, s.status, s.stream = ctx.row_ctx_len.data_ptr(), ctx.rt.status.data_ptr(), K._stream()
-        s.T, s.n_rows, s.max_q_len = T, ctx.n_rows, ctx.max_q_len
+        s.T, s.n_rows, s.max_q_len, s.kv_len = T, ctx.n_rows, ctx.max_q_len, ctx.kv_len_bound
+        scratch = prompt_scratch(ctx, self.n_q, self.d)
+        s.attn_scratch = None if scratch is None else scratch.data_ptr()
         s.num_blocks, s.block_size, s.streams = cache.num_blocks, cache.block_size, T <= linear.STREAM_MAX_ROWS
         for i, g in enumerate(cache.groups):
             s.k_base[i], s.v_base[i], s.table[i] = g.keys.data_ptr(), g.values.data_ptr(), g.table.data_ptr()

@@ -95,7 +95,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "fd_attn_simt_qt": [I],
         "fd_attn_decode_group": [I, I, I],
         "fd_attention_simt": [P, P, P, P, I, P, I, I, I, P, P, P, P, P, I, I, I, I, I, I, F, I, I, I, I, I, P, P, P],
-        "fd_attention": [P, P, P, P, I, P, I, I, I, P, P, P, P, P, I, I, I, I, I, I, F, I, I, I, I, I, P, P, P, P, c_ulonglong, I, F, P],
+        "fd_attention": [P, P, P, P, I, P, I, I, I, P, P, P, P, P, I, I, I, I, I, I, F, I, I, I, I, I, P, P, P, P, c_ulonglong, I, F, P, I, P],
         "fd_attention_mma_sync": [P, P, P, P, I, P, I, I, I, P, P, P, P, P, I, I, I, I, I, I, F, I, I, I, I, I, P, P, P, P],
         "fd_attention_dense": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, P, P, I, P, P],
         "fd_conv_rope_append": [P, I, I, P, P, P, P, P, I, I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, I, P, P, F, I, I, P],
@@ -159,6 +159,8 @@ def _declare(L: ctypes.CDLL) -> None:
         fn.argtypes = args
         fn.restype = I
     L.fd_attn_scratch_floats.argtypes = [I, I, I, I]
+    L.fd_attn_prompt_scratch_floats.argtypes = [I] * 6
+    L.fd_attn_prompt_scratch_floats.restype = LL
     L.fd_launch_count.restype = c_ulonglong
     L.fd_launch_count.argtypes = []
     L.fd_attn_scratch_floats.restype = LL
@@ -752,6 +754,11 @@ def attention_scratch_floats(n_tokens: int, n_q: int, head_dim: int, n_splits: i
     return int(lib().fd_attn_scratch_floats(n_tokens, n_q, head_dim, n_splits))
 
 
+def attention_prompt_scratch_floats(n_tokens: int, n_q: int, head_dim: int, n_rows: int, max_q_len: int, kv_len: int) -> int:
+    """Floats of scratch with which ``attention`` may cut a bfloat16 prompt step's keys into parts; 0: it would not."""
+    return int(lib().fd_attn_prompt_scratch_floats(n_tokens, n_q, head_dim, n_rows, max_q_len, kv_len))
+
+
 _attn_counters = {}      # per device: zeroed ints the decode kernel counts arriving splits in (kept alive for good)
 
 
@@ -764,7 +771,8 @@ def _counters(device, n: int) -> torch.Tensor:
 
 def _attention(fn_name, q, k_pool, v_pool, out, block_table, tok_row, row_slot, row_q_start, row_q_len,
                row_ctx_len, n_rows, max_q_len, n_q, n_kv, head_dim, scale, window, n_splits, split_len,
-               scratch, status, prefetch=None, prefetch_bytes=0, chunk=0, out_col=None, out_scale=1.0) -> None:
+               scratch, status, prefetch=None, prefetch_bytes=0, chunk=0, out_col=None, out_scale=1.0, prompt_scratch=None,
+               kv_len=0) -> None:
     T = q.shape[0]
     num_blocks, _, block_size, _ = k_pool.shape
     v_dim = v_pool.shape[-1]
@@ -784,7 +792,10 @@ def _attention(fn_name, q, k_pool, v_pool, out, block_table, tok_row, row_slot, 
         args.append(_ptr(_counters(q.device, n_rows * n_q)) if fused else None)
     args.append(_ptr(status))
     if fn_name == "fd_attention":
-        args += list(_prefetch_args(prefetch, prefetch_bytes)) + [0 if out_col is None else out.shape[-1], float(out_scale)]
+        assert prompt_scratch is None or (prompt_scratch.dtype == torch.float32 and prompt_scratch.numel() >=
+                                          attention_prompt_scratch_floats(T, n_q, head_dim, n_rows, max_q_len, kv_len))
+        args += list(_prefetch_args(prefetch, prefetch_bytes)) + [0 if out_col is None else out.shape[-1], float(out_scale),
+                                                                  _ptr(prompt_scratch), int(kv_len)]
     args.append(_stream())
     _check(getattr(lib(), fn_name)(*args))
 
@@ -796,7 +807,8 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: 
               window: int = 0, n_splits: int = 1, split_len: int = 0,
               scratch: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None,
               prefetch: Optional[torch.Tensor] = None, prefetch_bytes: int = 0, chunk: int = 0,
-              out_col: Optional[int] = None, out_scale: float = 1.0) -> None:
+              out_col: Optional[int] = None, out_scale: float = 1.0, prompt_scratch: Optional[torch.Tensor] = None,
+              kv_len: int = 0) -> None:
     """Causal GQA attention of the step's tokens over the paged cache, by the
     fastest kernel that takes the sizes (tensor cores for bfloat16 decode steps
     with head size 64 or 128; the CUDA-core kernel otherwise).  ``window`` > 0: a query
@@ -805,10 +817,13 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: 
     is that of ``v_pool`` (the tensor-core kernels take it equal to the key's).  ``prefetch``: a
     tensor that a later kernel streams; the tensor-core decode kernel asks L2 for its
     first ``prefetch_bytes`` when its own reads are through (the other kernels do not).  ``out_col``: the heads go to the
-    columns from there on of a wider ``out`` (columns and rows at multiples of 8); ``out_scale`` multiplies them."""
+    columns from there on of a wider ``out`` (columns and rows at multiples of 8); ``out_scale`` multiplies them.
+    ``prompt_scratch`` (float32, ``attention_prompt_scratch_floats`` of it) with ``kv_len``, a bound on the longest sequence
+    after the step: a prompt step whose CTAs leave most SMs idle may cut the keys into parts and add their outputs up."""
     _attention("fd_attention", q, k_pool, v_pool, out, block_table, tok_row, row_slot, row_q_start, row_q_len,
                row_ctx_len, n_rows, max_q_len, n_q, n_kv, head_dim, scale, window, n_splits, split_len,
-               scratch, status, prefetch, prefetch_bytes, chunk=chunk, out_col=out_col, out_scale=out_scale)
+               scratch, status, prefetch, prefetch_bytes, chunk=chunk, out_col=out_col, out_scale=out_scale,
+               prompt_scratch=prompt_scratch, kv_len=kv_len)
 
 
 def attention_mma_sync(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor,

@@ -19,7 +19,7 @@ PREFETCH_BYTES = 16 << 20   # an output projection up to this size is asked for 
                             # beginning of a larger one made the step slower: + 1.4 % at the sizes of Qwen2.5-7B, batch 8)
 FP32_SPLIT_LEN = 256      # keys per split of a decode step in float32
 # The same for attention without options: one tile of the kernel for heads of 64 and 128, so that a CTA is one chain of lookups,
-# loads, scores and values (csrc/attention_f32.cu) - where no sequence of the cache is so long that the merge would have
+# loads, scores and values (csrc/attention_rows.cu) - where no sequence of the cache is so long that the merge would have
 # more than 512 splits to add.
 FP32_TILE_LEN, FP32_MAX_SPLITS = 64, 512
 
@@ -49,6 +49,12 @@ def fp32_splits(ctx):
     a sequence's partial sums are cut - and with it every bit of its result - depends on nothing but its own length."""
     split_len = FP32_TILE_LEN if ctx.cache.max_len <= FP32_TILE_LEN * FP32_MAX_SPLITS else FP32_SPLIT_LEN
     return max(1, -(-ctx.kv_len_bound // split_len)), split_len
+
+
+def prompt_scratch(ctx, n_q: int, head_dim: int) -> Optional[torch.Tensor]:
+    """Workspace memory with which the attention of a prompt step may cut the keys into parts; None where it would not."""
+    n = K.attention_prompt_scratch_floats(ctx.T, n_q, head_dim, ctx.n_rows, ctx.max_q_len, ctx.kv_len_bound)
+    return ctx.ws.get("attn_prompt_parts", (n,), torch.float32) if n else None
 
 
 @register_part("mixer", "gqa_attention")
@@ -176,12 +182,14 @@ class GQAAttention(Mixer):
             if n_splits > 1:
                 scratch = ws.get("attn_scratch", (K.attention_scratch_floats(T, self.n_q, d, n_splits),),
                                  torch.float32)
+        parts = prompt_scratch(ctx, self.n_q, d) if ctx.max_q_len > 1 and x.dtype == torch.bfloat16 else None
         # a small decode step: when its keys and values are through, the attention kernel asks L2 for the beginning of
         # what the step streams after this part (the output projection's weights are in L2 already, see above)
         ahead = ctx.upcoming if ctx.max_q_len == 1 and T <= GEMV_MAX_ROWS and x.dtype == torch.bfloat16 else None
         K.attention(q, lc.k_pool, lc.v_pool, attn, lc.group.table, ctx.tok_row, ctx.row_slot,
                          ctx.row_q_start, ctx.row_q_len, ctx.row_ctx_len, ctx.n_rows, ctx.max_q_len,
                          self.n_q, self.n_kv, d, self.scale, self.window or 0, n_splits, split_len, scratch,
-                         self.rt.status, prefetch=ahead, prefetch_bytes=UPCOMING_BYTES, chunk=self.chunk or 0)
+                         self.rt.status, prefetch=ahead, prefetch_bytes=UPCOMING_BYTES, chunk=self.chunk or 0,
+                         prompt_scratch=parts, kv_len=ctx.kv_len_bound)
         out = ws.get("mixer_out", (T, self.hidden_size), x.dtype)
         return matmul(attn, self.w_o, None, out, target_ctas=4 * self.rt.sm_count, status=self.rt.status)

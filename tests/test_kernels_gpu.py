@@ -854,6 +854,25 @@ def test_attention_decode_tensor_cores_window_and_far_key(window, decode_form):
         assert rel(got, want) < TOL["bfloat16"], key_pos
 
 
+@pytest.mark.parametrize("n_q,n_kv,bs,window", [(12, 2, 16, 0), (12, 2, 64, 0), (4, 4, 128, 0), (2, 1, 32, 700), (7, 1, 16, 130)])
+def test_attention_prompts_in_parts(n_q, n_kv, bs, window):
+    """Later portions of long prompts, whose few CTAs cut the keys into parts: two to eight of them, parts that some or all
+    rows of a CTA see nothing of (short sequences beside long ones, the diagonal, windows), queries that fill a CTA and not."""
+    used = []
+
+    def fn(q, kp, vp, out, table, tok_row, slots, starts, lens, ctx, rows, most, nq, nkv, d, scale, win, splits, split_len, scr, st):
+        kv_len = int((lens + ctx).max())
+        n = K.attention_prompt_scratch_floats(q.shape[0], nq, d, rows, most, kv_len)
+        used.append(n // (q.shape[0] * nq * (d + 2)))
+        K.attention(q, kp, vp, out, table, tok_row, slots, starts, lens, ctx, rows, most, nq, nkv, d, scale, win, splits, split_len,
+                    scr, st, prompt_scratch=torch.full((max(n, 1),), float("nan"), device=DEV) if n else None, kv_len=kv_len)
+    for ctx, new in (([1000], [129]), ([700, 0], [40, 40]), ([3000], [2]), ([511], [1]), ([0], [128]), ([2048, 64, 1500], [1, 130, 17])):
+        got, want, _ = run_attention("bfloat16", n_q, n_kv, 128, bs, ctx=ctx, new=new, window=window, pad_rows=1, fn=fn,
+                                     spike=(0, ctx[0] + new[0] - 1))
+        assert rel(got, want) < TOL["bfloat16"], (ctx, new)
+    assert max(used) >= 4 and min(used) == 0 and any(1 < u < 4 for u in used)
+
+
 @pytest.mark.parametrize("n_q,n_kv,d,bs,window", [(12, 2, 128, 16, 0), (8, 1, 64, 64, 0), (3, 3, 128, 7, 0), (16, 2, 64, 16, 70),
                                                   (9, 1, 128, 32, 0), (64, 1, 64, 16, 100)])
 def test_attention_f32_decode_and_prompts(n_q, n_kv, d, bs, window):
