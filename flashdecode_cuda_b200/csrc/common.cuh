@@ -130,11 +130,11 @@ namespace fd {
 extern int g_pdl;      // 1: launches carry the programmatic-serialization attribute (runtime.cu)
 extern unsigned long long g_launches;      // kernels of this library launched so far (runtime.cu)
 
-// Launch with the attributes this library uses: programmatic dependent launch (when enabled)
-// and an optional thread-block cluster shape.
+// Launch with the attributes this library uses: programmatic dependent launch (`pdl`; the kernel calls pdl_wait
+// before anything else that touches memory an earlier kernel uses) and an optional thread-block cluster shape.
 template <typename... KArgs, typename... Args>
-inline int launch(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                  dim3 cluster, Args... args) {
+inline int launch_with(bool pdl, const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                       cudaStream_t stream, dim3 cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -142,7 +142,7 @@ inline int launch(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 bl
     cfg.stream = stream;
     cudaLaunchAttribute attrs[2];
     int n = 0;
-    if (g_pdl) {
+    if (pdl) {
         attrs[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attrs[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;
@@ -161,6 +161,18 @@ inline int launch(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 bl
     ++g_launches;
     return 0;
 }
+
+// The same, programmatic only while that is switched on for every kernel (fd_set_pdl; off by default).
+template <typename... KArgs, typename... Args>
+inline int launch(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                  dim3 cluster, Args... args) {
+    return launch_with(g_pdl != 0, what, kernel, grid, block, smem, stream, cluster, args...);
+}
+
+// Steps of more rows than this launch their norms, products and prompt attention programmatically: a kernel is set up, and
+// its barriers and tensor memory are ready, while the one before it drains.  Smaller steps are replayed from graphs,
+// where every programmatic edge cost more than it gave.
+constexpr int PDL_MIN_ROWS = 129;
 }  // namespace fd
 
 #define FD_REQUIRE(cond, code, ...) \

@@ -388,7 +388,7 @@ extern "C" int fd_add_rmsnorm(const void* delta, int delta_dtype, int n_parts, l
         (uintptr_t)delta % 16 == 0) {
         const int threads = ((H / 8 + 31) / 32) * 32;
 #define FD_NORM_ROW(T_, TW_)                                                                                             \
-    return launch("add_rmsnorm", add_rmsnorm_row_kernel<T_, TW_>, dim3(n_out), dim3(threads), 0, stream, dim3(1, 1, 1), \
+    return launch_with(g_pdl != 0 || n_out >= PDL_MIN_ROWS, "add_rmsnorm", add_rmsnorm_row_kernel<T_, TW_>, dim3(n_out), dim3(threads), 0, stream, dim3(1, 1, 1), \
                   (const T_*)delta, resid, write_resid, (const TW_*)weight, eps, (T_*)out, rows, H, dscale)
         if (out_dtype == 1) {
             if (w_dtype == 0) FD_NORM_ROW(bf16, float);

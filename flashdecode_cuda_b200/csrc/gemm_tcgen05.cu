@@ -373,9 +373,6 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k_iters = (p.K + TC_BK - 1) / TC_BK;
-    // the grouped form: only the row tiles that the device-side grouping filled
-    const int tm = p.n_row_tiles != nullptr ? min(tiles_m, *p.n_row_tiles) : tiles_m;
-    const int n_tiles = tm * tiles_n;
 
     if (threadIdx.x == 0) {
         abort_flag[0] = 0;
@@ -398,6 +395,10 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();                                  // everything above may run while the kernel before this one drains
+    // the grouped form: only the row tiles that the device-side grouping filled
+    const int tm = p.n_row_tiles != nullptr ? min(tiles_m, *p.n_row_tiles) : tiles_m;
+    const int n_tiles = tm * tiles_n;
 
     if (warp == 0 && lane == 0) {
         // ---- producer ----
@@ -570,6 +571,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     cluster_sync_all();              // the peer's barriers exist before anything of this CTA signals them
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();                      // everything above may run while the kernel before this one drains
 
     if (warp == 0 && lane == 0) {
         // ---- producer (in both CTAs): this CTA's 128 rows of x and its half of the W tile ----
@@ -708,6 +710,7 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
     // of them in a row, the wider tile is faster: q/k/v of 2,048 tokens 22.5 against 25.3 us.)
     const bool narrow = wide && g_tc_wide == 1 && (long long)tiles_m * ((p.N + TN_BN - 1) / TN_BN) <= sms;
     const bool pair = wide && (g_tc_wide == 2 || (g_tc_wide == 1 && !narrow && p.tile_expert == nullptr && pair_pays(p, sms)));
+    const bool pdl = g_pdl != 0 || p.M >= PDL_MIN_ROWS;
     CUtensorMap mx, mw;
     if (pair) {
         const int tiles_m2 = (p.M + 2 * TC_BM - 1) / (2 * TC_BM), tiles_n = (p.N + TW_BN - 1) / TW_BN;
@@ -717,12 +720,12 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
         // two k-blocks per copy where the three-dimensional view of the operands exists
         if (p.K % 64 == 0 && p.K >= 128 && tensor_map_blocks(x, p.M, p.K, &mx, TC_BM, 2) == 0 &&
             tensor_map_blocks(w, p.N, p.K, &mw, TC_BM, 2) == 0)
-            return launch(what, gemm_tcgen05_pair_kernel<2>, dim3(2 * pairs), dim3(TW_THREADS), TP_SMEM, stream, dim3(2, 1, 1), mx, mw,
+            return launch_with(pdl, what, gemm_tcgen05_pair_kernel<2>, dim3(2 * pairs), dim3(TW_THREADS), TP_SMEM, stream, dim3(2, 1, 1), mx, mw,
                           p, ra, tiles_m2, tiles_n);
         int rc = tensor_map(x, p.M, p.K, &mx, TC_BM);
         if (rc == 0) rc = tensor_map(w, p.N, p.K, &mw, TC_BM);
         if (rc != 0) return rc;
-        return launch(what, gemm_tcgen05_pair_kernel<1>, dim3(2 * pairs), dim3(TW_THREADS), TP_SMEM, stream, dim3(2, 1, 1), mx, mw, p, ra,
+        return launch_with(pdl, what, gemm_tcgen05_pair_kernel<1>, dim3(2 * pairs), dim3(TW_THREADS), TP_SMEM, stream, dim3(2, 1, 1), mx, mw, p, ra,
                       tiles_m2, tiles_n);
     }
     int rc = tensor_map(x, p.M, p.K, &mx, TC_BM);
@@ -735,9 +738,11 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
         const long long n_tiles = (long long)tiles_m * tiles_n;
         FD_REQUIRE(n_tiles < (1ll << 30), -2, "gemm_tcgen05: %lld tiles", n_tiles);
         const int grid = (int)(n_tiles < sms ? n_tiles : sms);
-        if (narrow) gemm_tcgen05_wide_kernel<TN_BN, TN_STAGES><<<grid, TW_THREADS, TN_SMEM, stream>>>(mx, mw, p, ra, tiles_m, tiles_n);
-        else gemm_tcgen05_wide_kernel<TW_BN, TW_STAGES><<<grid, TW_THREADS, TW_SMEM, stream>>>(mx, mw, p, ra, tiles_m, tiles_n);
-        return check_launch(what);
+        if (narrow)
+            return launch_with(pdl, what, gemm_tcgen05_wide_kernel<TN_BN, TN_STAGES>, dim3(grid), dim3(TW_THREADS), TN_SMEM, stream,
+                               dim3(1, 1, 1), mx, mw, p, ra, tiles_m, tiles_n);
+        return launch_with(pdl, what, gemm_tcgen05_wide_kernel<TW_BN, TW_STAGES>, dim3(grid), dim3(TW_THREADS), TW_SMEM, stream,
+                           dim3(1, 1, 1), mx, mw, p, ra, tiles_m, tiles_n);
     }
     dim3 grid((p.N + TC_BN - 1) / TC_BN, tiles_m);
     FD_REQUIRE(grid.y <= 65535, -2, "gemm_tcgen05: M=%d too large for one launch", p.M);
