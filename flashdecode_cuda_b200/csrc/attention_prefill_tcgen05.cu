@@ -745,7 +745,7 @@ static int ta_sm_count() {
 
 template <int KS, int VS, bool DENSE>
 static int ta_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, const AttnParams& p,
-                     int n_rows, int T, int max_q_len, cudaStream_t stream) {
+                     int n_rows, int max_q_len, cudaStream_t stream) {
     constexpr int smem_two = ta_smem(KS, VS, false), smem_split = ta_smem(KS, VS, true);
     static bool configured = false;
     if (!configured) {
@@ -758,15 +758,14 @@ static int ta_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
     // Two query tiles per CTA share every key tile; while that leaves SMs without a CTA, one query tile per
     // CTA with its key tiles dealt to the two softmax groups finishes sooner.
     const int shared_ctas = ((max_q_len + TA_ROWS - 1) / TA_ROWS) * p.n_q * n_rows;
-    const bool pdl = g_pdl != 0 || T >= PDL_MIN_ROWS;
     const bool split = p.n_splits > 1 || g_ta_form == 2 || (g_ta_form == 0 && shared_ctas < ta_sm_count());
     if (split) {
         dim3 grid(p.n_q, (max_q_len + TA_BM - 1) / TA_BM, n_rows * (DENSE ? 1 : p.n_splits));
-        return launch_with(pdl, "attention_prefill_tcgen05", attn_prefill_tcgen05_kernel<KS, VS, true, DENSE>, grid, dim3(TA_THREADS),
+        return launch_with(true, "attention_prefill_tcgen05", attn_prefill_tcgen05_kernel<KS, VS, true, DENSE>, grid, dim3(TA_THREADS),
                            smem_split, stream, dim3(1, 1, 1), mq, mk, mv, mr, p, g_tc_wait_ns, g_tc_skip_last);
     } else {
         dim3 grid(p.n_q, (max_q_len + TA_ROWS - 1) / TA_ROWS, n_rows);
-        return launch_with(pdl, "attention_prefill_tcgen05", attn_prefill_tcgen05_kernel<KS, VS, false, DENSE>, grid, dim3(TA_THREADS),
+        return launch_with(true, "attention_prefill_tcgen05", attn_prefill_tcgen05_kernel<KS, VS, false, DENSE>, grid, dim3(TA_THREADS),
                            smem_two, stream, dim3(1, 1, 1), mq, mk, mv, mr, p, g_tc_wait_ns, g_tc_skip_last);
     }
 }
@@ -803,9 +802,9 @@ int launch_attn_prefill_tcgen05(const AttnParams& p0, int n_rows, int T, int max
         p.n_splits = parts;
         p.part_acc = scratch; p.part_m = scratch + n * TA_D; p.part_l = p.part_m + n;
     }
-    const int rc = ta_launch<2, 2, false>(mq, mk, mv, mk, p, n_rows, T, max_q_len, stream);
+    const int rc = ta_launch<2, 2, false>(mq, mk, mv, mk, p, n_rows, max_q_len, stream);
     if (rc != 0 || p.n_splits == 1) return rc;
-    return launch_with(g_pdl != 0 || T >= PDL_MIN_ROWS, "attention_prompt_merge", attn_prompt_merge_kernel, dim3((T * p.n_q + 7) / 8), dim3(256),
+    return launch_with(true, "attention_prompt_merge", attn_prompt_merge_kernel, dim3((T * p.n_q + 7) / 8), dim3(256),
                        0, stream, dim3(1, 1, 1), p, tok_row, T * p.n_q);
 }
 
@@ -821,11 +820,11 @@ int launch_attn_prefill_dense(const AttnParams& p, const void* kv, const void* r
     if (ta_map(kv, T, p.n_q * (64 * kn + p.dv), TA_BN, &mk) != 0) return 1;
     mr = mk;
     if (kn < ks && ta_map(rot, T, p.d - 64 * kn, TA_BN, &mr) != 0) return 1;
-    if (ks == 1) return ta_launch<1, 1, true>(mq, mk, mk, mr, p, n_rows, T, max_q_len, stream);
-    if (ks == 2) return vs == 1 ? ta_launch<2, 1, true>(mq, mk, mk, mr, p, n_rows, T, max_q_len, stream)
-                                : ta_launch<2, 2, true>(mq, mk, mk, mr, p, n_rows, T, max_q_len, stream);
-    return vs == 1 ? ta_launch<3, 1, true>(mq, mk, mk, mr, p, n_rows, T, max_q_len, stream)
-                   : ta_launch<3, 2, true>(mq, mk, mk, mr, p, n_rows, T, max_q_len, stream);
+    if (ks == 1) return ta_launch<1, 1, true>(mq, mk, mk, mr, p, n_rows, max_q_len, stream);
+    if (ks == 2) return vs == 1 ? ta_launch<2, 1, true>(mq, mk, mk, mr, p, n_rows, max_q_len, stream)
+                                : ta_launch<2, 2, true>(mq, mk, mk, mr, p, n_rows, max_q_len, stream);
+    return vs == 1 ? ta_launch<3, 1, true>(mq, mk, mk, mr, p, n_rows, max_q_len, stream)
+                   : ta_launch<3, 2, true>(mq, mk, mk, mr, p, n_rows, max_q_len, stream);
 }
 
 }  // namespace fd

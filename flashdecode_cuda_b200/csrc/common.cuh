@@ -169,10 +169,15 @@ inline int launch(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 bl
     return launch_with(g_pdl != 0, what, kernel, grid, block, smem, stream, cluster, args...);
 }
 
-// Steps of more rows than this launch their norms, products and prompt attention programmatically: a kernel is set up, and
-// its barriers and tensor memory are ready, while the one before it drains.  Smaller steps are replayed from graphs,
-// where every programmatic edge cost more than it gave.
+// Prompt steps launch their norms, products and attention programmatically: a kernel is set up, and its barriers and tensor
+// memory are ready, while the one before it drains.  Decode steps are replayed from graphs, where every programmatic edge
+// cost more than it gave: a norm or product that does not know its step's kind goes by the number of rows.
 constexpr int PDL_MIN_ROWS = 129;
+
+// fd_add_rmsnorm with the choice of a programmatic launch (elementwise.cu)
+int add_rmsnorm(const void* delta, int delta_dtype, int n_parts, long long part_stride, float* resid, int write_resid,
+                const void* weight, int w_dtype, float eps, void* out, int out_dtype, const int* rows, int n_out, int H,
+                float dscale, bool pdl, cudaStream_t stream);
 }  // namespace fd
 
 #define FD_REQUIRE(cond, code, ...) \

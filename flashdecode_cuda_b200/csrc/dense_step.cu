@@ -7,9 +7,6 @@
 #include "common.cuh"
 
 extern "C" {
-int fd_add_rmsnorm(const void* delta, int delta_dtype, int n_parts, long long part_stride, float* resid, int write_resid,
-                   const void* weight, int w_dtype, float eps, void* out, int out_dtype, const int* rows, int n_out, int H,
-                   float dscale, cudaStream_t stream);
 int fd_gemm_stream(const void* x, const void* w, const void* bias, int bias_f32, void* out, int mode, int M, int N, int K,
                    int splits, int* status, void* tail_out, int tail_from, int tail_ld, cudaStream_t stream);
 int fd_gemm_stream_qkv_rope(const void* x, const void* w, const void* bias, int bias_f32, void* q_out, int M, int K, int splits,
@@ -63,8 +60,8 @@ extern "C" int fd_dense_mixer(const FdDenseStep* s, const FdDenseLayer* L, const
     const int T = (int)s->T, H = (int)L->hidden, g = (int)L->group, r = (int)L->position;
     char* kp = s->k_base[g] + L->index * s->k_stride[g];
     char* vp = s->v_base[g] + L->index * s->v_stride[g];
-    int rc = fd_add_rmsnorm(delta, 1, 1, 0, s->resid, 1, L->norm1, L->norm1_f32 ? 0 : 1, (float)L->eps1, s->normed, 1, nullptr, T, H,
-                            1.f, s->stream);
+    int rc = fd::add_rmsnorm(delta, 1, 1, 0, s->resid, 1, L->norm1, L->norm1_f32 ? 0 : 1, (float)L->eps1, s->normed, 1, nullptr, T, H,
+                             1.f, true, s->stream);
     if (rc != 0) return rc;
     if (s->streams)
         rc = fd_gemm_stream_qkv_rope(s->normed, L->w_qkv, L->b_qkv, (int)L->bias_f32, s->q, T, H, 0, s->cos_t[r], s->sin_t[r],
@@ -87,8 +84,8 @@ extern "C" int fd_dense_mixer(const FdDenseStep* s, const FdDenseLayer* L, const
 // norm of the stream with the mixer's output added, gate/up with the activation.
 extern "C" int fd_dense_gate_up(const FdDenseStep* s, const FdDenseLayer* L) {
     const int T = (int)s->T, H = (int)L->hidden, I = (int)L->inter;
-    const int rc = fd_add_rmsnorm(s->mixer_out, 1, 1, 0, s->resid, 1, L->norm2, L->norm2_f32 ? 0 : 1, (float)L->eps2, s->normed, 1,
-                                  nullptr, T, H, 1.f, s->stream);
+    const int rc = fd::add_rmsnorm(s->mixer_out, 1, 1, 0, s->resid, 1, L->norm2, L->norm2_f32 ? 0 : 1, (float)L->eps2, s->normed, 1,
+                                  nullptr, T, H, 1.f, true, s->stream);
     if (rc != 0) return rc;
     if (s->streams) return fd_gemm_stream(s->normed, L->w_gate_up, nullptr, 0, s->act, 3, T, 2 * I, H, 0, s->status, nullptr, 0, 0, s->stream);
     return fd_gemm_tc(s->normed, L->w_gate_up, nullptr, 0, s->act, 3, T, 2 * I, H, s->status, s->stream);

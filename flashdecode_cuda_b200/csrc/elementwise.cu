@@ -375,10 +375,10 @@ static int launch_norm(const void* delta, int n_parts, size_t part_stride, float
 }
 
 // delta_dtype / w_dtype / out_dtype: 0 = float32, 1 = bfloat16.  dscale: what delta is multiplied by as it is added.
-extern "C" int fd_add_rmsnorm(const void* delta, int delta_dtype, int n_parts, long long part_stride,
-                              float* resid, int write_resid, const void* weight, int w_dtype, float eps,
-                              void* out, int out_dtype, const int* rows, int n_out, int H, float dscale,
-                              cudaStream_t stream) {
+// pdl: the launch is programmatic (the row form of one delta only).
+int fd::add_rmsnorm(const void* delta, int delta_dtype, int n_parts, long long part_stride, float* resid, int write_resid,
+                    const void* weight, int w_dtype, float eps, void* out, int out_dtype, const int* rows, int n_out, int H,
+                    float dscale, bool pdl, cudaStream_t stream) {
     if (n_out == 0) return 0;
     FD_REQUIRE(H > 0, -2, "add_rmsnorm: bad width %d", H);
     FD_REQUIRE(delta == nullptr || n_parts >= 1, -2, "add_rmsnorm: n_parts=%d", n_parts);
@@ -388,7 +388,7 @@ extern "C" int fd_add_rmsnorm(const void* delta, int delta_dtype, int n_parts, l
         (uintptr_t)delta % 16 == 0) {
         const int threads = ((H / 8 + 31) / 32) * 32;
 #define FD_NORM_ROW(T_, TW_)                                                                                             \
-    return launch_with(g_pdl != 0 || n_out >= PDL_MIN_ROWS, "add_rmsnorm", add_rmsnorm_row_kernel<T_, TW_>, dim3(n_out), dim3(threads), 0, stream, dim3(1, 1, 1), \
+    return launch_with(pdl || g_pdl != 0, "add_rmsnorm", add_rmsnorm_row_kernel<T_, TW_>, dim3(n_out), dim3(threads), 0, stream, dim3(1, 1, 1), \
                   (const T_*)delta, resid, write_resid, (const TW_*)weight, eps, (T_*)out, rows, H, dscale)
         if (out_dtype == 1) {
             if (w_dtype == 0) FD_NORM_ROW(bf16, float);
@@ -422,6 +422,14 @@ extern "C" int fd_add_rmsnorm(const void* delta, int delta_dtype, int n_parts, l
     if (delta_dtype == 0 && out_dtype == 1)
         return launch_norm<float, bf16>(delta, n_parts, ps, resid, write_resid, weight, w_dtype, eps, out, rows, n_out, H, dscale, stream);
     return fail(-2, "add_rmsnorm: unsupported dtypes delta=%d out=%d", delta_dtype, out_dtype);
+}
+
+extern "C" int fd_add_rmsnorm(const void* delta, int delta_dtype, int n_parts, long long part_stride,
+                              float* resid, int write_resid, const void* weight, int w_dtype, float eps,
+                              void* out, int out_dtype, const int* rows, int n_out, int H, float dscale,
+                              cudaStream_t stream) {
+    return fd::add_rmsnorm(delta, delta_dtype, n_parts, part_stride, resid, write_resid, weight, w_dtype, eps, out, out_dtype,
+                           rows, n_out, H, dscale, n_out >= PDL_MIN_ROWS, stream);
 }
 
 // tiled == 0: gu = [gate (I columns) | up (I columns)]; tiled != 0: tiles of 8 gate + 8 up columns.

@@ -353,6 +353,9 @@ constexpr int TW_SMEM = TW_STAGES * TW_STAGE_BYTES + 1024 /* alignment slack */ 
 // chain of copies and MMAs (q/k/v with its epilogue at 512 and 1,024 tokens: 16 against 22 us).
 constexpr int TN_BN = 128, TN_STAGES = 6;
 constexpr int TN_SMEM = TN_STAGES * (TC_A_BYTES + TN_BN * TC_BK * 2) + 1024 + 256;
+// And with 128 x 192 tiles and five stages of 40 KB (choose_tiling).
+constexpr int TM_BN = 192, TM_STAGES = 5;
+constexpr int TM_SMEM = TM_STAGES * (TC_A_BYTES + TM_BN * TC_BK * 2) + 1024 + 256;
 constexpr int TW_EPI_WARPS = 8;               // two per quarter of the tensor-memory lanes, half of the columns each
 constexpr int TW_THREADS = (2 + TW_EPI_WARPS) * 32;
 
@@ -360,6 +363,7 @@ template <int BN, int STAGES>
 __global__ void __launch_bounds__(TW_THREADS, 1)
 gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                          const TcParams p, const TcRope ra, const int tiles_m, const int tiles_n) {
+    constexpr int TMEM_COLS = BN <= 128 ? 256 : 512;             // two accumulators, in a power of two of columns
     constexpr int STAGE_BYTES = TC_A_BYTES + BN * TC_BK * 2;
     extern __shared__ unsigned char tc_smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -388,7 +392,7 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_addr(tmem_slot)), "r"(2 * BN) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_addr(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -481,7 +485,7 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
     }
 }
 
@@ -670,21 +674,28 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 
 // ---- host side ------------------------------------------------------------
 int g_tc_wide = 1;      // where N >= 256: 1: the persistent one-SM kernel (128 x 256 tiles, or 128 x 128 where those number no more
-                        // than the SMs), or the two-SM kernel where pair_pays; 2: the two-SM kernel; 3: one SM and 128 x 256 tiles
-                        // always; 0: 128 x 128 tiles, one per CTA
+                        // than the SMs), 128 x 192 or the two-SM kernel by choose_tiling; 2: the two-SM kernel; 3, 4: one SM and
+                        // 128 x 256 or 128 x 192 tiles always; 0: 128 x 128 tiles, one per CTA
 
-// Whether two SMs per 256 x 256 tile beat one SM per 128 x 256: a pair's round takes 0.87 of the time where the products of a tile
-// are long (measured us, pair / one SM: gate/up of 5,120 columns at 1,200 and 2,048 rows 250 / 280 and 378 / 442, of 3,584 columns
-// at 2,048 rows 376 / 444, q/k/v of the same 142 / 162 and 67 / 78) and 0.94 at 1,536 columns (gate/up at 2,048 and 9,208 rows
-// 83 / 89 and 336 / 365), where the q/k/v epilogue is the longer part and the pair slower (78 / 68) - but its rounds
-// are coarser (gate/up of 3,584 columns at 384 rows: four instead of three, 103 / 91).
-static bool pair_pays(const TcParams& p, int sms) {
-    const long long tn = (p.N + TW_BN - 1) / TW_BN, tiles = (long long)((p.M + TC_BM - 1) / TC_BM) * tn;
-    const long long pairs = (long long)((p.M + 2 * TC_BM - 1) / (2 * TC_BM)) * tn;
-    const long long rounds = (tiles + sms - 1) / sms, pair_rounds = (pairs + sms / 2 - 1) / (sms / 2);
-    if (rounds < 2) return false;
-    if (p.K < 2048) return p.mode != 4 && p.M >= 1024 && pair_rounds * 19 < rounds * 20;
-    return pair_rounds * 9 < rounds * 10;
+// The tiling of a product of several rounds over the SMs: 0 one SM per 128 x 256 tile, 1 one SM per 128 x 192, 2 two SMs per 256 x 256.  A
+// round's time goes with the bytes it brings in (rows of x + rows of W), and a pair's takes 0.87 of the wide tile's where the
+// products of a tile are long: gate/up of 5,120 columns at 1,200 and 2,048 rows 250 / 280 and 378 / 442 us (pair / one SM), of 3,584
+// columns at 2,048 rows 376 / 444, q/k/v of the same 142 / 162 and 67 / 78; 0.94 at 1,536 columns (gate/up at 2,048 and 9,208
+// rows 83 / 89 and 336 / 365), where the q/k/v epilogue is the longer part and the pair slower (78 / 68).  Coarser rounds can lose
+// that again (gate/up of 3,584 columns at 384 rows: four instead of three, 103 / 91), and the narrower tile wins where it
+// fills a last round that the wide one leaves half empty (gate/up of 1,536 columns at 384 rows: 210 tiles on 148 SMs).
+static int choose_tiling(const TcParams& p, int sms) {
+    const long long tm = (p.M + TC_BM - 1) / TC_BM, tn = (p.N + TW_BN - 1) / TW_BN;
+    auto rounds = [](long long tiles, long long at_once) { return (tiles + at_once - 1) / at_once; };
+    const long long wide = rounds(tm * tn, sms);
+    if (wide < 2) return 0;
+    double best = (double)wide * (TC_BM + TW_BN);
+    int form = 0;
+    const double mid = (double)rounds(tm * ((p.N + TM_BN - 1) / TM_BN), sms) * (TC_BM + TM_BN);
+    if (mid < best) { best = mid; form = 1; }
+    const double pair = (double)rounds((long long)((p.M + 2 * TC_BM - 1) / (2 * TC_BM)) * tn, sms / 2) * (TC_BM + TW_BN) * (p.K < 2048 ? 0.95 : 0.9);
+    if (pair < best && (p.K >= 2048 || (p.mode != 4 && p.M >= 1024))) form = 2;
+    return form;
 }
 
 // w_stack: matrices in the stack w [w_stack][N, K] (the grouped form; 1: the plain product).
@@ -696,6 +707,7 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
         cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_wide_kernel<TW_BN, TW_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, TW_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_wide_kernel<TN_BN, TN_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, TN_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_wide_kernel<TM_BN, TM_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, TM_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM);
         if (e != cudaSuccess) return fail(-3, "gemm_tcgen05: cannot get %d bytes of shared memory: %s", TW_SMEM, cudaGetErrorString(e));
@@ -709,7 +721,8 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
     // 128 x 128 tiles where even those give no CTA a second tile: twice the CTAs at work.  (Where CTAs would take two
     // of them in a row, the wider tile is faster: q/k/v of 2,048 tokens 22.5 against 25.3 us.)
     const bool narrow = wide && g_tc_wide == 1 && (long long)tiles_m * ((p.N + TN_BN - 1) / TN_BN) <= sms;
-    const bool pair = wide && (g_tc_wide == 2 || (g_tc_wide == 1 && !narrow && p.tile_expert == nullptr && pair_pays(p, sms)));
+    const int tiling = wide && !narrow && g_tc_wide == 1 && p.tile_expert == nullptr ? choose_tiling(p, sms) : 0;
+    const bool pair = wide && (g_tc_wide == 2 || tiling == 2), mid = wide && (g_tc_wide == 4 || tiling == 1);
     const bool pdl = g_pdl != 0 || p.M >= PDL_MIN_ROWS;
     CUtensorMap mx, mw;
     if (pair) {
@@ -730,16 +743,19 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
     }
     int rc = tensor_map(x, p.M, p.K, &mx, TC_BM);
     if (rc != 0) return rc;
-    rc = tensor_map(w, w_stack * p.N, p.K, &mw, (wide && !narrow) ? TW_BN : TC_BM);
+    rc = tensor_map(w, w_stack * p.N, p.K, &mw, mid ? TM_BN : ((wide && !narrow) ? TW_BN : TC_BM));
     if (rc != 0) return rc;
     if (wide) {
-        const int bn = narrow ? TN_BN : TW_BN;
+        const int bn = mid ? TM_BN : (narrow ? TN_BN : TW_BN);
         const int tiles_n = (p.N + bn - 1) / bn;
         const long long n_tiles = (long long)tiles_m * tiles_n;
         FD_REQUIRE(n_tiles < (1ll << 30), -2, "gemm_tcgen05: %lld tiles", n_tiles);
         const int grid = (int)(n_tiles < sms ? n_tiles : sms);
         if (narrow)
             return launch_with(pdl, what, gemm_tcgen05_wide_kernel<TN_BN, TN_STAGES>, dim3(grid), dim3(TW_THREADS), TN_SMEM, stream,
+                               dim3(1, 1, 1), mx, mw, p, ra, tiles_m, tiles_n);
+        if (mid)
+            return launch_with(pdl, what, gemm_tcgen05_wide_kernel<TM_BN, TM_STAGES>, dim3(grid), dim3(TW_THREADS), TM_SMEM, stream,
                                dim3(1, 1, 1), mx, mw, p, ra, tiles_m, tiles_n);
         return launch_with(pdl, what, gemm_tcgen05_wide_kernel<TW_BN, TW_STAGES>, dim3(grid), dim3(TW_THREADS), TW_SMEM, stream,
                            dim3(1, 1, 1), mx, mw, p, ra, tiles_m, tiles_n);
@@ -755,10 +771,11 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
 using namespace fd;
 
 // Which tiling the products use from now on where N >= 256 (1, the default: persistent CTAs with 128 x 256 tiles,
-// with 128 x 128 tiles where those number no more than the SMs, or two SMs per tile where that is faster; 3: persistent CTAs with 128 x 256 tiles always; 2: two
+// with 128 x 128 tiles where those number no more than the SMs, with 128 x 192 or two SMs per tile where that is faster; 4: 128 x 192
+// always; 3: persistent CTAs with 128 x 256 tiles always; 2: two
 // SMs per 256 x 256 tile; 0: 128 x 128 tiles, one per CTA, everywhere).  For tests and measurements.
 extern "C" int fd_gemm_tc_set_wide(int on) {
-    g_tc_wide = on < 0 ? 0 : (on > 3 ? 3 : on);
+    g_tc_wide = on < 0 ? 0 : (on > 4 ? 4 : on);
     return 0;
 }
 

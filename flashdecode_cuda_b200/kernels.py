@@ -545,7 +545,8 @@ GEMV_GATED_GELU = 6      # gated with the tanh form of GELU instead of SiLU; bot
 def gemm_tc_set_wide(on) -> None:
     """Which tiling ``gemm_tc`` and ``gemm_tc_qkv_rope`` use from now on where N >= 256: 2 = two SMs per
     256 x 256 tile (``tcgen05.mma.cta_group::2``), 1 / True = one persistent CTA per SM with 128 x 256
-    tiles, with 128 x 128 tiles where those number no more than the SMs, or two SMs where that is faster, 3 = 128 x 256 tiles
+    tiles, with 128 x 128 tiles where those number no more than the SMs, or as in 4 or 2 where that is faster, 4 = 128 x 192
+    tiles always, 3 = 128 x 256 tiles
     always, 0 / False = 128 x 128 tiles, one per CTA, everywhere.  For tests and measurements."""
     lib().fd_gemm_tc_set_wide(int(on))
 

@@ -269,9 +269,9 @@ def test_gemm_stream_refuses_what_it_cannot_do():
 TC_DEFAULT_TILING = 1
 
 
-@pytest.fixture(params=[2, 3, 1, 0], ids=["pair", "wide", "auto", "square"])
+@pytest.fixture(params=[2, 3, 4, 1, 0], ids=["pair", "wide", "mid", "auto", "square"])
 def tc_tiling(request):
-    """The tilings of the tcgen05 product: two SMs per 256 x 256 tile, persistent CTAs with 128 x 256 tiles, the
+    """The tilings of the tcgen05 product: two SMs per 256 x 256 tile, persistent CTAs with 128 x 256 and with 128 x 192 tiles, the
     default (persistent CTAs with 128 x 128 tiles where those number no more than the SMs: most shapes of these
     tests), and 128 x 128 tiles with one CTA each."""
     K.gemm_tc_set_wide(request.param)
