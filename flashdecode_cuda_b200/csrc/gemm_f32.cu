@@ -360,7 +360,7 @@ int launch_gemm_f32(const float* A, const float* W, const float* bias, float* C,
             if (form < 0 || t < best) { form = i; best = t; }
         }
     }
-    FD_REQUIRE((M + 31) / 32 <= 65535, -2, "gemm_f32: M=%d too large for one launch", M);
+    FD_REQUIRE((M + bm[form] - 1) / bm[form] <= 65535, -2, "gemm_f32: M=%d too large for one launch", M);
     switch (form) {
         case 0: return launch_tile<128, 128, 8, 16, 16, 3>(A, W, bias, C, M, N, K, stream);
         case 1: return launch_tile<64, 128, 8, 8, 32, 3>(A, W, bias, C, M, N, K, stream);
