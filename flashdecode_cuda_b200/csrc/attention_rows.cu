@@ -1,10 +1,12 @@
 // Attention on the CUDA cores over the paged cache for head sizes 64 and 128, in tiles of 64 keys: the true 32-bit path (causal,
 // grouped heads, with an optional window or chunked visibility), and the decode steps in bfloat16 whose options no tensor-core kernel
 // has (kept first keys, heads whose weights are mixed).  Scores, softmax and sums are float; key tiles, splits and the
-// order of every sum are fixed in absolute position, so in float32 a query's bits depend on nothing but its own sequence.
+// order of every sum are fixed in absolute position, so in float32 a query's bits depend on nothing but its own sequence (and on
+// whether that brings one token to the step or more).
 // (attention_simt.cu takes every other size and option.)
 //
-//  * decode: a CTA takes one (sequence, key/value head, split) and tiles of 64 keys.  Bound by the chain of lookups, one trip
+//  * decode: a CTA takes one (sequence, key/value head, split), up to eight heads of the group, and tiles of 64 keys.  Bound by the
+//    chain of lookups, one trip
 //    to memory, scores, softmax and values: all of a tile's keys and values are asked for at once, and with splits of 64 keys
 //    (attention.py) a CTA has one tile.
 //  * prompts: a CTA takes up to 64 rows (query, head of the group) and walks the keys in tiles of 64; scores and value sums
@@ -19,7 +21,7 @@ namespace {
 
 constexpr int FT = 64;             // keys per tile
 constexpr int FTHREADS = 128;
-constexpr int GDEC = 8;            // most query heads per key/value head in the decode kernel
+constexpr int GDEC = 8;            // most query heads of a CTA of the decode kernel; larger groups are cut (p.kv_div pieces)
 
 __device__ __forceinline__ void cp16(void* dst, const void* src, bool on) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -93,10 +95,12 @@ attn_rows_decode_kernel(const AttnParams p) {
     float* l_s = m_s + GDEC;
     float* a_s = l_s + GDEC;
     __shared__ int row_s[FT], vrow_s[FT];
-    const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+    // pieces of a group of more than GDEC heads are as equal as whole heads allow: the last one may have fewer
+    const int split = blockIdx.x, kvh = blockIdx.y / p.kv_div, per = (p.G + p.kv_div - 1) / p.kv_div, b = blockIdx.z;
+    const int g0 = (blockIdx.y - kvh * p.kv_div) * per, G = min(per, p.G - g0), head = kvh * p.G + g0;
     const int slot = p.row_slot[b];
     if (slot < 0) return;
-    const int tok = p.row_q_start[b], pos = p.row_ctx_len[b], G = p.G;
+    const int tok = p.row_q_start[b], pos = p.row_ctx_len[b];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0, hi = pos + 1;
     if (p.chunk > 0) lo = max(lo, (pos / p.chunk) * p.chunk);
@@ -108,7 +112,7 @@ attn_rows_decode_kernel(const AttnParams p) {
         kf = min(kf, hi);
     }
     if (kf <= s_lo) kf = 0;
-    const size_t head0 = (size_t)tok * p.n_q + kvh * G;      // the group's first (token, head)
+    const size_t head0 = (size_t)tok * p.n_q + head;         // the CTA's first (token, head)
     if (lo >= hi && kf == 0) {                               // (a split without keys: only its sums are looked at)
         if (p.n_splits > 1 && tid < G * VR) p.part_l[(head0 * VR + tid) * p.n_splits + split] = 0.f;
         return;
@@ -237,12 +241,12 @@ attn_rows_decode_kernel(const AttnParams p) {
             }
             float l = l_s[g], f = 1.f;
             if (p.sink != nullptr) {                         // one more term in the denominator: exp(sink), no key, no value
-                const float sk = p.sink[kvh * G + g], m2 = fmaxf(m_s[g], sk);
+                const float sk = p.sink[head + g], m2 = fmaxf(m_s[g], sk);
                 f = expf(m_s[g] - m2);
                 l = l * f + expf(sk - m2);
             }
             const float inv = l > 0.f ? f * p.out_scale / l : 0.f;
-            const size_t at = (size_t)tok * p.out_ld + ((kvh * G + g) * VR + j) * HD + e;
+            const size_t at = (size_t)tok * p.out_ld + ((head + g) * VR + j) * HD + e;
             if (sizeof(T) == 4 || p.out_f32)
                 *reinterpret_cast<float4*>(static_cast<float*>(p.out) + at) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
             else {
@@ -414,15 +418,21 @@ int launch_decode(const AttnParams& p, int n_rows, cudaStream_t stream) {
     static bool done = false;
     const int rc = configure(attn_rows_decode_kernel<T, HD, VR, GM>, smem, done);
     if (rc != 0) return rc;
-    attn_rows_decode_kernel<T, HD, VR, GM><<<dim3(p.n_splits, p.n_kv, n_rows), FTHREADS, smem, stream>>>(p);
+    attn_rows_decode_kernel<T, HD, VR, GM><<<dim3(p.n_splits, p.n_kv * p.kv_div, n_rows), FTHREADS, smem, stream>>>(p);
     return check_launch("attention_rows_decode");
 }
 
 template <int HD>
 int launch_f32(const AttnParams& p0, int n_rows, int max_q_len, cudaStream_t stream) {
     AttnParams p = p0;
-    if (max_q_len == 1 && p.G <= GDEC) return launch_decode<float, HD, 1, GDEC>(p, n_rows, stream);
-    if (p.n_splits > 1 || p.G > PR) return 1;
+    // Which kernel takes a row depends on its group and on how many tokens it brings, never on the splits: those follow from the
+    // batch's longest sequence, and a row's bits must not.
+    if (p.G > PR) return 1;
+    if (max_q_len == 1) {
+        p.kv_div = (p.G + GDEC - 1) / GDEC;
+        return p.n_kv * p.kv_div <= 65535 ? launch_decode<float, HD, 1, GDEC>(p, n_rows, stream) : 1;
+    }
+    if (p.n_splits > 1) return 1;
     p.QT = PR / p.G < max_q_len ? PR / p.G : max_q_len;
     constexpr int smem = prompt_smem_floats<HD>() * (int)sizeof(float);
     static bool done = false;

@@ -892,6 +892,18 @@ def test_attention_f32_decode_and_prompts(n_q, n_kv, d, bs, window):
         assert rel(got, want) < TOL["float32"], (c, new)
 
 
+@pytest.mark.parametrize("n_q,n_kv,d", [(1, 1, 128), (16, 2, 64), (9, 1, 128), (34, 2, 64), (64, 1, 64), (12, 2, 96)])
+def test_attention_f32_decode_bits_do_not_depend_on_the_batch(n_q, n_kv, d):
+    """How many splits a decode step has follows from its longest sequence.  A shorter sequence's result is the same bits with as
+    many splits as it needs itself and with more: groups up to eight query heads, more (in equal pieces and unequal ones), and a
+    head size that the general kernel takes."""
+    for ctx in (0, 39, 63, 64, 150):
+        own = ctx // 64 + 1
+        outs = [run_attention("float32", n_q, n_kv, d, 16, ctx=[ctx], new=[1], n_splits=n, split_len=64, fn=K.attention)[0]
+                for n in (own, 8, 37)]
+        assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]), ctx
+
+
 def test_attention_refuses_what_it_cannot_do():
     with pytest.raises(K.KernelError, match="head size"):
         run_attention("float32", 4, 2, 20, 4, ctx=[0], new=[3])
