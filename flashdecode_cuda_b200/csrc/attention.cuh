@@ -5,6 +5,8 @@
 
 namespace fd {
 
+enum { ROWS_ALL = 0, ROWS_SINGLE = 1, ROWS_LONGER = 2 };
+
 struct AttnParams {
     const void* q;             // [T, n_q * d]
     const void* k_pool;        // [num_blocks, n_kv, block_size, d]
@@ -41,6 +43,9 @@ struct AttnParams {
                                // n_kv heads); out is then [T, n_q, v_rep, dv]
     int v_all;                 // set by the CUDA-core launcher: a CTA takes a key head and all v_rep value heads, not one
     int out_f32;               // out is float whatever the type of q and the pools
+    // float32 steps in which some rows bring one token and others more: ROWS_SINGLE takes only the former (their partial sums lie by
+    // row, not by token), ROWS_LONGER the others
+    int row_kind;
     // whole prompts over plain rows only (attention_prefill_tcgen05.cu): slabs of 64 key dimensions that are a head's own, and
     // the heads' output gate, [T, gate_ld], or null
     int dense_kn;

@@ -99,7 +99,7 @@ attn_rows_decode_kernel(const AttnParams p) {
     const int split = blockIdx.x, kvh = blockIdx.y / p.kv_div, per = (p.G + p.kv_div - 1) / p.kv_div, b = blockIdx.z;
     const int g0 = (blockIdx.y - kvh * p.kv_div) * per, G = min(per, p.G - g0), head = kvh * p.G + g0;
     const int slot = p.row_slot[b];
-    if (slot < 0) return;
+    if (slot < 0 || p.row_q_len[b] != 1) return;
     const int tok = p.row_q_start[b], pos = p.row_ctx_len[b];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0, hi = pos + 1;
@@ -112,9 +112,10 @@ attn_rows_decode_kernel(const AttnParams p) {
         kf = min(kf, hi);
     }
     if (kf <= s_lo) kf = 0;
-    const size_t head0 = (size_t)tok * p.n_q + head;         // the CTA's first (token, head)
+    const size_t head0 = (size_t)tok * p.n_q + head;         // the CTA's first (token, head), and that of its partial sums
+    const size_t part0 = p.row_kind == ROWS_SINGLE ? (size_t)b * p.n_q + head : head0;
     if (lo >= hi && kf == 0) {                               // (a split without keys: only its sums are looked at)
-        if (p.n_splits > 1 && tid < G * VR) p.part_l[(head0 * VR + tid) * p.n_splits + split] = 0.f;
+        if (p.n_splits > 1 && tid < G * VR) p.part_l[(part0 * VR + tid) * p.n_splits + split] = 0.f;
         return;
     }
     const T* qg = static_cast<const T*>(p.q) + head0 * HD;
@@ -234,7 +235,7 @@ attn_rows_decode_kernel(const AttnParams p) {
                 o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
             }
             if (p.n_splits > 1) {
-                const size_t pi = ((head0 + g) * VR + j) * p.n_splits + split;
+                const size_t pi = ((part0 + g) * VR + j) * p.n_splits + split;
                 if (e == 0) { p.part_m[pi] = m_s[g]; p.part_l[pi] = l_s[g]; }
                 *reinterpret_cast<float4*>(p.part_acc + pi * HD + e) = o;
                 continue;
@@ -278,7 +279,7 @@ attn_f32_prompt_kernel(const AttnParams p) {
     const int slot = p.row_slot[b];
     if (slot < 0) return;
     const int q_len = p.row_q_len[b], G = p.G, QT = p.QT;
-    if (tile * QT >= q_len) return;
+    if (tile * QT >= q_len || (p.row_kind == ROWS_LONGER && q_len == 1)) return;
     const int nq = min(QT, q_len - tile * QT), R = nq * G;
     const int tok0 = p.row_q_start[b] + tile * QT, p_first = p.row_ctx_len[b] + tile * QT;
     int lo = p.window > 0 ? max(0, p_first - p.window + 1) : 0;

@@ -77,7 +77,7 @@ attn_tile_kernel(const AttnParams p) {
     const int slot = p.row_slot[b];
     if (slot < 0) return;
     const int q_len = p.row_q_len[b];
-    if (tile * p.QT >= q_len) return;
+    if (tile * p.QT >= q_len || (p.row_kind == ROWS_SINGLE && q_len != 1) || (p.row_kind == ROWS_LONGER && q_len == 1)) return;
     const int ctx = p.row_ctx_len[b];
     const int tok0 = p.row_q_start[b] + tile * p.QT;       // first query token of this CTA
     const int nq = min(p.QT, q_len - tile * p.QT);
@@ -325,7 +325,7 @@ attn_tile_kernel(const AttnParams p) {
         size_t row = (size_t)(tok0 + qi) * p.n_q + head;
         if (p.v_rep > 1) row = row * p.v_rep + vh + jv;
         if (p.n_splits > 1) {
-            const size_t pi = row * p.n_splits + split;
+            const size_t pi = (p.row_kind == ROWS_SINGLE ? (size_t)b * p.n_q + head : row) * p.n_splits + split;
             if (dc == 0) { p.part_m[pi] = alpha_s[r]; p.part_l[pi] = l_s[r]; }
             *reinterpret_cast<float4*>(p.part_acc + pi * dv + dc * 4) =
                 make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
@@ -363,13 +363,16 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_m, const floa
                                     const float* __restrict__ part_acc, T* __restrict__ out,
                                     const int* __restrict__ tok_row, const int* __restrict__ row_slot,
                                     int n_q, int d, int n_splits, const float* __restrict__ sink, int v_rep,
-                                    int out_f32, int out_ld, float out_scale) {
+                                    int out_f32, int out_ld, float out_scale, const int* __restrict__ row_q_start,
+                                    const int* __restrict__ row_q_len) {
     __shared__ float w_s[COMBINE_MAX_SPLITS];
     __shared__ float red[33];
     pdl_launch_dependents();
     pdl_wait();
-    const int tok = blockIdx.y, h = blockIdx.x;
-    const size_t row = (size_t)tok * n_q + h;
+    // row_q_len given: the partial sums of rows (ROWS_SINGLE), of which those that bring one token have any
+    const int h = blockIdx.x, tok = row_q_len != nullptr ? row_q_start[blockIdx.y] : blockIdx.y;
+    const size_t row = (size_t)blockIdx.y * n_q + h;
+    if (row_q_len != nullptr && (row_slot[blockIdx.y] < 0 || row_q_len[blockIdx.y] != 1)) return;
     T* o = out + (size_t)tok * out_ld + (size_t)h * d;
     float* of = reinterpret_cast<float*>(out) + (size_t)tok * out_ld + (size_t)h * d;       // the same row when the output is float whatever T is
     if (row_slot[tok_row[tok]] < 0) {
@@ -557,6 +560,7 @@ static int attention_impl(const void* q, const void* k_pool, const void* v_pool,
     p.n_q = n_q; p.n_kv = n_kv; p.G = G; p.d = d; p.dv = dv; p.v_ld = v_ld; p.chunk = chunk;
     p.n_kv_pool = n_kv; p.kv_div = 1;
     p.softcap = softcap; p.keep_first = keep_first; p.sink = sink; p.v_rep = v_rep; p.out_f32 = out_f32; p.v_all = 0;
+    p.row_kind = ROWS_ALL;
     if (dv != d) use_mma = 0;          // the tensor-core kernels keep keys and values of one size
     int qt = G <= RMAX ? fd_attn_simt_qt(G) : 1;
     if ((d > 256 || dv > 256) && qt > RWIDE / G) qt = RWIDE / G > 0 ? RWIDE / G : 1;
@@ -564,6 +568,27 @@ static int attention_impl(const void* q, const void* k_pool, const void* v_pool,
     p.QT = qt; p.n_splits = n_splits; p.split_len = split_len; p.window = window; p.scale = scale;
 
     int rc = 1;
+    if (dtype == 0 && max_q_len > 1 && n_splits == 1 && split_len > 0 && kv_len > 0) {
+        // float32: rows that bring one token run as in a step of such rows alone (same kernel, same splits), so that their bits
+        // do not depend on what the other rows bring
+        AttnParams one = p;
+        one.row_kind = ROWS_SINGLE; one.QT = 1; one.split_len = split_len; one.n_splits = (kv_len + split_len - 1) / split_len;
+        FD_REQUIRE(split_len % KT == 0 && one.n_splits <= COMBINE_MAX_SPLITS && (one.n_splits == 1 || prompt_scratch != nullptr), -2,
+                   "attention: rows of single tokens: splits of %d keys of up to %d, or their scratch memory is missing", split_len, kv_len);
+        const size_t n = (size_t)n_rows * n_q * one.n_splits;
+        one.part_acc = prompt_scratch;
+        one.part_m = prompt_scratch ? prompt_scratch + n * dv : nullptr;
+        one.part_l = prompt_scratch ? one.part_m + n : nullptr;
+        if (use_mma != 0) rc = launch_attn_f32(one, n_rows, 1, stream);
+        if (rc == 1) rc = launch_attn<float>(one, n_rows, 1, stream);
+        if (rc == 0 && one.n_splits > 1)
+            rc = launch("attention_combine", attn_combine_kernel<float>, dim3(n_q, n_rows), dim3(128), 0, stream, dim3(1, 1, 1),
+                        (const float*)one.part_m, (const float*)one.part_l, (const float*)one.part_acc, (float*)out, tok_row,
+                        row_slot, n_q, dv, one.n_splits, (const float*)nullptr, 1, 0, p.out_ld, out_scale, row_q_start, row_q_len);
+        if (rc != 0) return rc;
+        p.row_kind = ROWS_LONGER;
+        rc = 1;
+    }
     if (decode_mma) {
         AttnParams pd = p;
         const int cut = fd_attn_decode_group(G, d, dv);     // a large group as several smaller ones on the same pool head
@@ -591,10 +616,12 @@ static int attention_impl(const void* q, const void* k_pool, const void* v_pool,
     if (dtype == 0)
         return launch("attention_combine", attn_combine_kernel<float>, grid, dim3(128), 0, stream, dim3(1, 1, 1),
                       (const float*)p.part_m, (const float*)p.part_l, (const float*)p.part_acc, (float*)out, tok_row,
-                      row_slot, n_q * v_rep, dv, n_splits, sink, v_rep, out_f32, p.out_ld, out_scale);
+                      row_slot, n_q * v_rep, dv, n_splits, sink, v_rep, out_f32, p.out_ld, out_scale, (const int*)nullptr,
+                      (const int*)nullptr);
     return launch("attention_combine", attn_combine_kernel<bf16>, grid, dim3(128), 0, stream, dim3(1, 1, 1),
                   (const float*)p.part_m, (const float*)p.part_l, (const float*)p.part_acc, (bf16*)out, tok_row,
-                  row_slot, n_q * v_rep, dv, n_splits, sink, v_rep, out_f32, p.out_ld, out_scale);
+                  row_slot, n_q * v_rep, dv, n_splits, sink, v_rep, out_f32, p.out_ld, out_scale, (const int*)nullptr,
+                  (const int*)nullptr);
 }
 
 // out[t, h, :] = scale * sum_g mix[h, g] * o[t, g, vh(h), :] with vh(h) = h / (n_q / n_kv): every head takes the other
@@ -658,7 +685,9 @@ extern "C" int fd_attention_simt(const void* q, const void* k_pool, const void* 
 // separate merge kernel runs.  prefetch / prefetch_bytes (optional, 16-byte aligned): memory that a
 // later kernel streams, which the tensor-core decode kernel asks L2 for when its own reads are
 // through (the other kernels ignore it).  prompt_scratch (optional, fd_attn_prompt_scratch_floats, 16-byte aligned) with kv_len, the
-// longest sequence after the step: a prompt step of few CTAs may cut its keys into parts.
+// longest sequence after the step: a prompt step of few CTAs may cut its keys into parts.  In float32, with kv_len and split_len > 0
+// and n_splits 1 (fd_attn_scratch_floats(n_rows, n_q, dv, ceil(kv_len / split_len)) of prompt_scratch where that is more than one
+// split): rows that bring one token are computed as a step of single tokens with splits of split_len would.
 extern "C" int fd_attention(const void* q, const void* k_pool, const void* v_pool, void* out, int dtype,
                             const int* block_table, int max_blocks, int num_blocks, int block_size,
                             const int* tok_row, const int* row_slot, const int* row_q_start,

@@ -773,7 +773,7 @@ def _counters(device, n: int) -> torch.Tensor:
 def _attention(fn_name, q, k_pool, v_pool, out, block_table, tok_row, row_slot, row_q_start, row_q_len,
                row_ctx_len, n_rows, max_q_len, n_q, n_kv, head_dim, scale, window, n_splits, split_len,
                scratch, status, prefetch=None, prefetch_bytes=0, chunk=0, out_col=None, out_scale=1.0, prompt_scratch=None,
-               kv_len=0) -> None:
+               kv_len=0, single_split_len=0) -> None:
     T = q.shape[0]
     num_blocks, _, block_size, _ = k_pool.shape
     v_dim = v_pool.shape[-1]
@@ -787,14 +787,21 @@ def _attention(fn_name, q, k_pool, v_pool, out, block_table, tok_row, row_slot, 
             num_blocks, block_size, _ptr(tok_row), _ptr(row_slot), _ptr(row_q_start), _ptr(row_q_len),
             _ptr(row_ctx_len), n_rows, T, max_q_len, n_q, n_kv, head_dim, float(scale), int(window), int(v_dim),
             int(chunk), n_splits, split_len, _ptr(scratch)]
+    if fn_name == "fd_attention":
+        if q.dtype == torch.float32:
+            singles = single_split_len > 0 and max_q_len > 1 and n_splits == 1
+            need = attention_scratch_floats(n_rows, n_q, v_dim, -(-kv_len // single_split_len)) if singles else 0
+            args[-2] = single_split_len if singles else split_len
+            kv_len = kv_len if singles else 0
+        else:
+            need = attention_prompt_scratch_floats(T, n_q, head_dim, n_rows, max_q_len, kv_len)
+        assert prompt_scratch is None or (prompt_scratch.dtype == torch.float32 and prompt_scratch.numel() >= need)
     if fn_name != "fd_attention_simt":
         fused = n_splits > 1 and max_q_len == 1 and q.dtype == torch.bfloat16
         # (a large group of query heads may be cut into several: at most one counter per query head)
         args.append(_ptr(_counters(q.device, n_rows * n_q)) if fused else None)
     args.append(_ptr(status))
     if fn_name == "fd_attention":
-        assert prompt_scratch is None or (prompt_scratch.dtype == torch.float32 and prompt_scratch.numel() >=
-                                          attention_prompt_scratch_floats(T, n_q, head_dim, n_rows, max_q_len, kv_len))
         args += list(_prefetch_args(prefetch, prefetch_bytes)) + [0 if out_col is None else out.shape[-1], float(out_scale),
                                                                   _ptr(prompt_scratch), int(kv_len)]
     args.append(_stream())
@@ -809,7 +816,7 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: 
               scratch: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None,
               prefetch: Optional[torch.Tensor] = None, prefetch_bytes: int = 0, chunk: int = 0,
               out_col: Optional[int] = None, out_scale: float = 1.0, prompt_scratch: Optional[torch.Tensor] = None,
-              kv_len: int = 0) -> None:
+              kv_len: int = 0, single_split_len: int = 0) -> None:
     """Causal GQA attention of the step's tokens over the paged cache, by the
     fastest kernel that takes the sizes (tensor cores for bfloat16 decode steps
     with head size 64 or 128; the CUDA-core kernel otherwise).  ``window`` > 0: a query
@@ -820,11 +827,14 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: 
     first ``prefetch_bytes`` when its own reads are through (the other kernels do not).  ``out_col``: the heads go to the
     columns from there on of a wider ``out`` (columns and rows at multiples of 8); ``out_scale`` multiplies them.
     ``prompt_scratch`` (float32, ``attention_prompt_scratch_floats`` of it) with ``kv_len``, a bound on the longest sequence
-    after the step: a prompt step whose CTAs leave most SMs idle may cut the keys into parts and add their outputs up."""
+    after the step: a prompt step whose CTAs leave most SMs idle may cut the keys into parts and add their outputs up.
+    ``single_split_len`` > 0 with ``kv_len``, in a float32 step whose longest row brings several tokens: rows that bring one token
+    are computed, to the bit, as a step of single tokens with splits of that length computes them
+    (``attention_scratch_floats(n_rows, ...)`` of ``prompt_scratch`` where the keys are more than one split)."""
     _attention("fd_attention", q, k_pool, v_pool, out, block_table, tok_row, row_slot, row_q_start, row_q_len,
                row_ctx_len, n_rows, max_q_len, n_q, n_kv, head_dim, scale, window, n_splits, split_len,
                scratch, status, prefetch, prefetch_bytes, chunk=chunk, out_col=out_col, out_scale=out_scale,
-               prompt_scratch=prompt_scratch, kv_len=kv_len)
+               prompt_scratch=prompt_scratch, kv_len=kv_len, single_split_len=single_split_len)
 
 
 def attention_mma_sync(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor,

@@ -51,6 +51,21 @@ def fp32_splits(ctx):
     return max(1, -(-ctx.kv_len_bound // split_len)), split_len
 
 
+def single_rows(ctx, n_q: int, v_dim: int, dtype: torch.dtype, split_len: int) -> dict:
+    """What ``K.attention`` needs, in float32, for a step in which some sequences bring one token and others more: the former are
+    then computed as in a step of their own, with splits of ``split_len`` keys, so that a decoded token's bits do not
+    depend on whether a prompt is taken in the same step.  Nothing for any other step."""
+    if dtype != torch.float32 or ctx.max_q_len == 1 or 1 not in ctx.h_q_len:
+        return {}
+    n = -(-ctx.kv_len_bound // split_len)
+    if n > FP32_MAX_SPLITS:                  # (a step of single tokens would be refused)
+        return {}
+    scratch = None
+    if n > 1:
+        scratch = ctx.ws.get("attn_scratch", (K.attention_scratch_floats(ctx.n_rows, n_q, v_dim, n),), torch.float32)
+    return dict(prompt_scratch=scratch, kv_len=ctx.kv_len_bound, single_split_len=split_len)
+
+
 def prompt_scratch(ctx, n_q: int, head_dim: int) -> Optional[torch.Tensor]:
     """Workspace memory with which the attention of a prompt step may cut the keys into parts; None where it would not."""
     n = K.attention_prompt_scratch_floats(ctx.T, n_q, head_dim, ctx.n_rows, ctx.max_q_len, ctx.kv_len_bound)
@@ -182,7 +197,10 @@ class GQAAttention(Mixer):
             if n_splits > 1:
                 scratch = ws.get("attn_scratch", (K.attention_scratch_floats(T, self.n_q, d, n_splits),),
                                  torch.float32)
-        parts = prompt_scratch(ctx, self.n_q, d) if ctx.max_q_len > 1 and x.dtype == torch.bfloat16 else None
+        if x.dtype == torch.float32:
+            cut = single_rows(ctx, self.n_q, d, x.dtype, fp32_splits(ctx)[1])
+        else:
+            cut = dict(prompt_scratch=prompt_scratch(ctx, self.n_q, d) if ctx.max_q_len > 1 else None, kv_len=ctx.kv_len_bound)
         # a small decode step: when its keys and values are through, the attention kernel asks L2 for the beginning of
         # what the step streams after this part (the output projection's weights are in L2 already, see above)
         ahead = ctx.upcoming if ctx.max_q_len == 1 and T <= GEMV_MAX_ROWS and x.dtype == torch.bfloat16 else None
@@ -190,6 +208,6 @@ class GQAAttention(Mixer):
                          ctx.row_q_start, ctx.row_q_len, ctx.row_ctx_len, ctx.n_rows, ctx.max_q_len,
                          self.n_q, self.n_kv, d, self.scale, self.window or 0, n_splits, split_len, scratch,
                          self.rt.status, prefetch=ahead, prefetch_bytes=UPCOMING_BYTES, chunk=self.chunk or 0,
-                         prompt_scratch=parts, kv_len=ctx.kv_len_bound)
+                         **cut)
         out = ws.get("mixer_out", (T, self.hidden_size), x.dtype)
         return matmul(attn, self.w_o, None, out, target_ctas=4 * self.rt.sm_count, status=self.rt.status)

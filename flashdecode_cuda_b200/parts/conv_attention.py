@@ -13,7 +13,7 @@ from .. import kernels as K
 from ..cache.paged import StateSpec
 from ..registry import register_part
 from ..weights.spec import TensorSpec
-from .attention import FP32_SPLIT_LEN, plan_splits
+from .attention import FP32_SPLIT_LEN, plan_splits, single_rows
 from .base import KVRequest, LayerCache, Mixer, Runtime
 from .linear import matmul
 from .normed_attention import _pad_heads, _up8
@@ -229,7 +229,8 @@ class ConvGatedAttention(Mixer):
             attn = ws.get("cga_attn", (T, self.n_q * self.dv), dt)
             K.attention(q, lc.k_pool, lc.v_pool, attn, lc.group.table, ctx.tok_row, ctx.row_slot, ctx.row_q_start,
                         ctx.row_q_len, ctx.row_ctx_len, ctx.n_rows, ctx.max_q_len, self.n_q, self.n_kv, self.d, self.scale,
-                        self.window or 0, n_splits, split_len, scratch, rt.status, chunk=self.chunk or 0)
+                        self.window or 0, n_splits, split_len, scratch, rt.status, chunk=self.chunk or 0,
+                        **single_rows(ctx, self.n_q, self.dv, dt, FP32_SPLIT_LEN))
         else:
             attn = ws.get("cga_attn_f" if self.talk else "cga_attn", (T, heads_out * self.dv),
                           torch.float32 if self.talk else dt)

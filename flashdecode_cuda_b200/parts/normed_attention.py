@@ -11,7 +11,7 @@ import torch
 from .. import kernels as K
 from ..registry import register_part
 from ..weights.spec import TensorSpec
-from .attention import FP32_SPLIT_LEN, plan_splits
+from .attention import FP32_SPLIT_LEN, plan_splits, single_rows
 from .base import KVRequest, LayerCache, Mixer, Runtime
 from .linear import matmul
 
@@ -226,7 +226,7 @@ class QKNormedAttention(Mixer):
         if self.extended:
             K.attention_ext(*args, softcap=self.softcap or 0.0, sink=self.sink_w, out_col=act_col, out_scale=scale)
         else:
-            K.attention(*args, out_col=act_col, out_scale=scale)
+            K.attention(*args, out_col=act_col, out_scale=scale, **single_rows(ctx, self.n_q, self.dvp, proj.dtype, FP32_SPLIT_LEN))
         return act
 
     def forward(self, ctx, x: torch.Tensor, lc: LayerCache) -> torch.Tensor:
@@ -416,7 +416,7 @@ class LatentAttention(Mixer):
         if tensor_rows or not plain:
             K.attention_ext(*args, sink=self.sink, value_dim=self.r if self.rot else 0)
         else:
-            K.attention(*args)
+            K.attention(*args, **single_rows(ctx, n, self.r, x.dtype, FP32_SPLIT_LEN))
         v = ws.get("lat_v", (T, n * self.vx), x.dtype)
         gated = self.has_gate and (T < K.HEAD_GEMM_LIBRARY_ROWS or x.dtype != torch.bfloat16)
         K.head_gemm(ac, self.w_cv, v, gate=proj if gated else None, gate_col=self.gate_col)

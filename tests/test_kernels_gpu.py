@@ -904,6 +904,34 @@ def test_attention_f32_decode_bits_do_not_depend_on_the_batch(n_q, n_kv, d):
         assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]), ctx
 
 
+@pytest.mark.parametrize("n_q,n_kv,d,window", [(12, 2, 128, 0), (9, 1, 64, 0), (5, 5, 128, 100), (12, 2, 96, 0), (66, 1, 128, 0)])
+@pytest.mark.parametrize("split_len", [64, 256])
+def test_attention_f32_single_tokens_beside_prompts(n_q, n_kv, d, window, split_len):
+    """Rows of one token beside rows of more give the bits that they give in a step of their own: within one split and over several,
+    first tokens of a sequence, a padding row, and (d 96, 66 heads) where the general kernel computes both."""
+    checked = []
+
+    def fn(q, kp, vp, out, table, tok_row, slots, starts, lens, ctx, rows, most, nq, nkv, d, scale, win, splits, s_len, scr, st):
+        kv_len = int((lens + ctx).max())
+        parts = torch.full((K.attention_scratch_floats(rows, nq, d, -(-kv_len // split_len)),), float("nan"), device=DEV)
+        K.attention(q, kp, vp, out, table, tok_row, slots, starts, lens, ctx, rows, most, nq, nkv, d, scale, win, splits, s_len, scr, st,
+                    prompt_scratch=parts, kv_len=kv_len, single_split_len=split_len)
+        for b in range(rows):
+            if int(lens[b]) != 1 or int(slots[b]) < 0:
+                continue
+            n = -(-(int(ctx[b]) + 1) // split_len)
+            alone = torch.empty(1, nq * d, device=DEV)
+            at = int(starts[b])
+            K.attention(q[at:at + 1].clone(), kp, vp, alone, table, tok_row[:1] * 0, slots[b:b + 1].clone(), starts[:1] * 0,
+                        lens[b:b + 1].clone(), ctx[b:b + 1].clone(), 1, 1, nq, nkv, d, scale, win, n, split_len,
+                        torch.empty(K.attention_scratch_floats(1, nq, d, n), device=DEV), st)
+            checked.append(torch.equal(out[at], alone[0]))
+    got, want, _ = run_attention("float32", n_q, n_kv, d, 16, ctx=[39, 0, 300, 700, 0, 50], new=[1, 70, 1, 1, 1, 9], window=window,
+                                 pad_rows=1, fn=fn)
+    assert rel(got, want) < TOL["float32"]
+    assert len(checked) == 4 and all(checked)
+
+
 def test_attention_refuses_what_it_cannot_do():
     with pytest.raises(K.KernelError, match="head size"):
         run_attention("float32", 4, 2, 20, 4, ctx=[0], new=[3])

@@ -310,6 +310,27 @@ def test_float32_decode_does_not_depend_on_the_batch(engines, folders):
     eng.model.check_status()
 
 
+@pytest.mark.parametrize("name", CONFIGS)
+def test_float32_decode_beside_a_prompt_keeps_its_bits(engines, name):
+    """In float32 a decoded token's logits are the same bits in a step of its own and in one in which another sequence brings its
+    prompt: within the first split of the keys and over several."""
+    eng = engines[(name, "float32")]
+    V = TINY[name]["vocab_size"]
+    cache = eng.model.new_cache(max_tokens=64 * 24, block_size=16, max_slots=4)
+    limit = min(cache.max_len, 125 if name == "A" else 600)
+    a, b, other = prompts_for(V, [40, limit, 90], seed=45)
+    sa, sb = cache.admit(), cache.admit()
+    eng.model.step(cache, [sa, sb], [a[:-1], b[:-1]], None)
+    alone = eng.model.step(cache, [sa, sb], [a[-1:], b[-1:]], "last").clone()
+    cache.release(sa)
+    cache.release(sb)
+    sb, sc, sa = cache.admit(), cache.admit(), cache.admit()
+    eng.model.step(cache, [sb, sa], [b[:-1], a[:-1]], None)
+    got = eng.model.step(cache, [sb, sc, sa], [b[-1:], other, a[-1:]], "last")
+    assert torch.equal(got[2], alone[0]) and torch.equal(got[0], alone[1])
+    eng.model.check_status()
+
+
 REAL_WIDTHS = {
     # the layer sizes of the three presets (two layers each, the whole vocabulary): groups of 6, 7 and 5 query heads
     "qwen2.5-1.5b": [40, 33, 140],
