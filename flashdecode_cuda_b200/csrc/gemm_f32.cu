@@ -355,12 +355,13 @@ int launch_gemm_f32(const float* A, const float* W, const float* bias, float* C,
     if (form < 0) {
         float best = 0.f;
         for (int i = 0; i < 6; ++i) {
+            if ((M + bm[i] - 1) / bm[i] > 65535) continue;           // more rows of tiles than a grid has
             const long long tiles = (long long)((M + bm[i] - 1) / bm[i]) * ((N + bn[i] - 1) / bn[i]);
             const float per_sm = (float)((tiles + 147) / 148) * shared[i], t = per_sm > alone[i] ? per_sm : alone[i];
             if (form < 0 || t < best) { form = i; best = t; }
         }
     }
-    FD_REQUIRE((M + bm[form] - 1) / bm[form] <= 65535, -2, "gemm_f32: M=%d too large for one launch", M);
+    FD_REQUIRE(form >= 0 && (M + bm[form] - 1) / bm[form] <= 65535, -2, "gemm_f32: M=%d too large for one launch", M);
     switch (form) {
         case 0: return launch_tile<128, 128, 8, 16, 16, 3>(A, W, bias, C, M, N, K, stream);
         case 1: return launch_tile<64, 128, 8, 8, 32, 3>(A, W, bias, C, M, N, K, stream);

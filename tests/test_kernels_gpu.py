@@ -359,6 +359,19 @@ def test_gemm_f32_forms_give_the_same_bits(M, N, K_):
 # paged cache helpers for the rope and attention kernels
 # ---------------------------------------------------------------------------
 
+@pytest.mark.parametrize("M,N", [(65535 * 32 + 1, 5), (65535 * 64, 17)])
+def test_gemm_f32_takes_millions_of_rows(M, N):
+    """Narrow products of more rows than 65,535 of the tiles of 32 rows that would be chosen for them, up to the largest number that
+    the entry point takes."""
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x, w = torch.randn(M, 4, device=DEV, generator=g), torch.randn(N, 4, device=DEV, generator=g)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    K.gemm_simt(x, w, None, out)
+    assert rel(out, x.double() @ w.double().T) < TOL["float32"]
+    with pytest.raises(K.KernelError, match="too large"):
+        K.gemm_simt(torch.empty(65535 * 64 + 1, 4, device=DEV), w, None, torch.empty(65535 * 64 + 1, N, device=DEV))
+
+
 def scrambled_table(lens, block_size, n_slots, gen, spare=3):
     """Block table [n_slots, max_blocks] whose blocks are handed out in a
     random order, so a kernel that ignores the table cannot pass."""
