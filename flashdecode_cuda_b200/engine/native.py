@@ -10,9 +10,14 @@ nothing between the layers - the same launches are made by ``fd_dense_layers``
 output and down projections.  Everything else, and every step that this module
 does not take, goes through the parts' ``forward``.
 
-Kept from step to step: the weights' addresses, which do not change while a
-model is bound.  The cache's, the step's and the workspace's addresses are taken
-anew for every step.
+A part whose ``forward`` was wrapped or replaced, on the object or on its class,
+is called: such a model's steps go through the parts.
+
+Kept from step to step: the weights, and their addresses.  Every step looks
+whether a part has changed since (``Part.changes``) and whether the weights lie
+where they lay, and derives everything anew if not (some 10 us at 28 layers).
+The cache's, the step's and the workspace's addresses are taken anew for every
+step.
 """
 
 from __future__ import annotations
@@ -26,11 +31,15 @@ import torch
 from .. import kernels as K
 from ..parts import linear
 from ..parts.attention import GQAAttention, prompt_scratch
+from ..parts.base import Part
 from ..parts.block import PreNormBlock
 from ..parts.mlp import SwiGLU
 from ..parts.norm import RMSNorm
 
 MAX_GROUPS, MAX_POSITIONS = 8, 4
+KINDS = (PreNormBlock, RMSNorm, GQAAttention, SwiGLU)
+FORWARDS = [kind.forward for kind in KINDS]                         # what the native calls stand for
+_address = torch.Tensor.data_ptr
 
 
 class _Layer(ctypes.Structure):
@@ -56,9 +65,25 @@ class DensePrompts:
 
     @staticmethod
     def of(model) -> Optional["DensePrompts"]:
+        native = DensePrompts(model)
+        return native if native.layers is not None else None
+
+    def __init__(self, model):
+        self.model = model
+        self._derive()
+
+    def _derive(self) -> None:
+        """The launches' constants from the model's parts as they are now; ``layers`` None: not a model of this kind."""
+        self.derived_at = Part.changes                              # before anything is read
+        self.blocks = list(self.model.blocks)
+        self.tensors, self.where = [], []
+        self.layers = self._layers()
+
+    def _layers(self):
+        model = self.model
         if model.dtype != torch.bfloat16 or model.blueprint.lanes != 1 or model.stream_ops:
             return None
-        blocks = [model.blocks[run.layer] for run in model.schedule]
+        blocks = [self.blocks[run.layer] for run in model.schedule]
         for run, b in zip(model.schedule, blocks):
             if run.before is not None or type(b) is not PreNormBlock or b.side is not None:
                 return None
@@ -66,6 +91,8 @@ class DensePrompts:
                     type(b.feed_forward) is not SwiGLU or not (b.mixer.paired and b.feed_forward.tiled):
                 return None
             if b.norm1.delta_scale != 1.0 or b.norm2.delta_scale != 1.0 or b.norm1.weight is None or b.norm2.weight is None:
+                return None
+            if any("forward" in vars(p) for p in (b, b.norm1, b.norm2, b.mixer, b.feed_forward)):
                 return None
         sizes = {(b.mixer.n_q, b.mixer.n_kv, b.mixer.d, b.feed_forward.inter) for b in blocks}
         positions = list({id(b.mixer.position): b.mixer.position for b in blocks}.values())
@@ -75,18 +102,25 @@ class DensePrompts:
                                                b.feed_forward.w_gate_up, b.feed_forward.w_down) if t is not None]
         if not blocks or not all(t.is_cuda and t.is_contiguous() for t in tensors):
             return None
-        return DensePrompts(model, blocks, positions)
-
-    def __init__(self, model, blocks: list, positions: list):
-        self.model, self.positions, self.n = model, positions, len(blocks)
-        self.hidden = model.hidden_size
+        H = model.hidden_size
+        for b in blocks:                                            # (replaced weights may be anything)
+            m, f = b.mixer, b.feed_forward
+            shapes = ((m.w_qkv, ((m.n_q + 2 * m.n_kv) * m.d, H)), (m.w_o, (H, m.n_q * m.d)), (f.w_gate_up, (2 * f.inter, H)),
+                      (f.w_down, (H, f.inter)))
+            vectors = [(b.norm1.weight, H), (b.norm2.weight, H)] + ([] if m.b_qkv is None else [(m.b_qkv, m.w_qkv.shape[0])])
+            if any(w.dtype != torch.bfloat16 or w.shape != shape for w, shape in shapes) or \
+                    any(v.dtype not in (torch.bfloat16, torch.float32) or v.shape != (n,) for v, n in vectors):
+                return None
+        self.tensors, self.where = tensors, list(map(_address, tensors))
+        self.positions, self.n = positions, len(blocks)
+        self.hidden = H
         m, f = blocks[0].mixer, blocks[0].feed_forward
         self.n_q, self.n_kv, self.d, self.inter = m.n_q, m.n_kv, m.d, f.inter
         self.qkv = (m.n_q + 2 * m.n_kv) * m.d
-        self.layers = (_Layer * self.n)()
+        layers = (_Layer * self.n)()
         self.products = []                                          # (w_o^T, w_down^T): the library products' operands
         for i, (b, (gi, li, writes, _)) in enumerate(zip(blocks, model._layout[2])):
-            m, f, L = b.mixer, b.feed_forward, self.layers[i]
+            m, f, L = b.mixer, b.feed_forward, layers[i]
             L.norm1, L.norm2 = b.norm1.weight.data_ptr(), b.norm2.weight.data_ptr()
             L.w_qkv, L.b_qkv = m.w_qkv.data_ptr(), None if m.b_qkv is None else m.b_qkv.data_ptr()
             L.w_o, L.w_gate_up, L.w_down = m.w_o.data_ptr(), f.w_gate_up.data_ptr(), f.w_down.data_ptr()
@@ -97,13 +131,19 @@ class DensePrompts:
             L.group, L.index, L.position = gi, li, [p is m.position for p in positions].index(True)
             L.eps1, L.eps2, L.scale = b.norm1.eps, b.norm2.eps, m.scale
             self.products.append((m.w_o.t(), f.w_down.t()))
-        self.addresses = [ctypes.addressof(self.layers[i]) for i in range(self.n)]
+        self.addresses = [ctypes.addressof(layers[i]) for i in range(self.n)]
+        return layers
 
     def takes(self, ctx) -> bool:
         """Whether the parts would run this step on the kernels that the native calls launch."""
-        T, H = ctx.T, self.hidden
+        T = ctx.T
         if linear.PROMPT_GEMM != "auto" or ctx.max_q_len < 2 or T <= linear.GEMV_MAX_ROWS:
             return False
+        if self.derived_at != Part.changes or self.blocks != self.model.blocks or list(map(_address, self.tensors)) != self.where:
+            self._derive()
+        if self.layers is None or [kind.forward for kind in KINDS] != FORWARDS:
+            return False
+        H = self.hidden
         if T <= linear.STREAM_MAX_ROWS:
             return all(linear.stream_gemm(T, n, k) for n, k in ((self.qkv, H), (H, self.n_q * self.d), (2 * self.inter, H), (H, self.inter)))
         return linear.fused_prompt_gemm(T, self.qkv, H) and linear.fused_prompt_gemm(T, 2 * self.inter, H)

@@ -65,7 +65,6 @@ class PartTimer:
         self._wrap_launcher(torch, "mm", "library_mm")
         self._wrap_launcher(torch, "addmm", "library_mm")
         m = self.model
-        self._native, m.native = m.native, None         # steps go through the parts, launch by launch
         self._wrap_part(m.embedding, "embedding")
         self._wrap_part(m.final_norm, "norm")
         self._wrap_part(m.head, "head")
@@ -86,7 +85,6 @@ class PartTimer:
         return self
 
     def __exit__(self, *exc) -> None:
-        self.model.native = self._native
         for owner, name, fn in reversed(self._saved):
             if fn is None:
                 del owner.forward              # the instance attribute; the class's method shows again

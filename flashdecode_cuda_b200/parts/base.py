@@ -35,6 +35,7 @@ A norm, block or mixer that knows nothing of this gets plain [T, H] tensors.
 
 from __future__ import annotations
 
+import itertools
 from dataclasses import dataclass
 from typing import Dict, List, Optional
 
@@ -91,8 +92,23 @@ class LayerCache:
         return self.group.v_pool(self.layer)
 
 
+_change_numbers = itertools.count(1)
+
+
 class Part:
     kind = ""
+    # A new number whenever an attribute of any part is set or deleted - its weights bound or replaced, its ``forward``
+    # wrapped: what was derived from parts (engine/native.py) is current while this is the number it was derived at.
+    changes = 0
+
+    def __setattr__(self, name, value) -> None:
+        object.__setattr__(self, name, value)
+        Part.changes = next(_change_numbers)
+
+    def __delattr__(self, name) -> None:
+        object.__delattr__(self, name)
+        Part.changes = next(_change_numbers)
+
     # False for a part whose forward reads the step's host mirrors (``ctx.h_*``) or
     # otherwise decides on the host: its steps cannot be replayed from a CUDA graph.
     graph_safe = True

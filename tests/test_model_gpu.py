@@ -157,6 +157,62 @@ def test_native_prompt_steps_change_no_bit(engines, name, block_size):
     assert len(taken) >= 6 and len(a) == len(b) and all(torch.equal(x, y) for x, y in zip(a, b))
 
 
+def test_native_prompt_steps_see_what_became_of_the_parts(engines, monkeypatch):
+    """A forward wrapped on a part or on its class is called, and replaced weights are used, by prompt steps of every length (18
+    tokens: one native call; 140: two per layer) as by the parts; steps that change nothing derive nothing anew."""
+    from flashdecode_cuda_b200.parts.mlp import SwiGLU
+    m = engines[("D", "bfloat16")].model
+    native, block = m.native, m.blocks[0]
+    reqs = prompts_for(m.vocab_size, [18, 140], seed=77)
+
+    def logits():
+        out = []
+        for r in reqs:
+            cache = m.new_cache(max_tokens=256, block_size=16)
+            out.append(m.step(cache, [cache.admit()], [r], "last").clone())
+        return out
+
+    def through_parts():
+        m.native = None
+        try:
+            return logits()
+        finally:
+            m.native = native
+    first = logits()
+    derived = []
+    monkeypatch.setattr(native, "_derive", lambda f=native._derive: (derived.append(1), f())[1])
+    assert all(torch.equal(a, b) for a, b in zip(logits(), first)) and not derived
+    called = []
+    for part in (block, block.norm1, block.norm2, block.mixer, block.feed_forward):
+        part.forward = lambda *a, f=part.forward, **kw: (called.append(1), f(*a, **kw))[1]
+        try:
+            got = logits()
+            assert len(called) == 2 and all(torch.equal(a, b) for a, b in zip(got, first))
+        finally:
+            del part.forward
+        called.clear()
+    with monkeypatch.context() as mp:
+        mp.setattr(SwiGLU, "forward", lambda self, *a, f=SwiGLU.forward, **kw: (called.append(1), f(self, *a, **kw))[1])
+        assert all(torch.equal(a, b) for a, b in zip(logits(), first)) and len(called) == 2 * len(m.blocks)
+    for part, attr in ((block.norm1, "weight"), (block.norm2, "weight"), (block.mixer, "w_qkv"), (block.mixer, "w_o"),
+                       (block.feed_forward, "w_gate_up"), (block.feed_forward, "w_down")):
+        old = getattr(part, attr)
+        setattr(part, attr, old.flip(-1).contiguous())
+        try:
+            got, want = logits(), through_parts()
+        finally:
+            setattr(part, attr, old)
+        assert all(torch.equal(a, b) and not torch.equal(a, c) for a, b, c in zip(got, want, first)), attr
+        kept, old.data = old.data, old.flip(-1).contiguous()         # the same tensor object, other memory
+        try:
+            assert all(torch.equal(a, b) for a, b in zip(logits(), want)), attr
+        finally:
+            old.data = kept
+    before = len(derived)
+    assert all(torch.equal(a, b) for a, b in zip(logits(), first)) and len(derived) <= before + 1
+    m.check_status()
+
+
 @pytest.mark.parametrize("name", ["D", "E"])
 def test_asking_l2_for_what_comes_next_changes_no_bit(engines, folders, name, monkeypatch):
     """Decode steps hand ``ctx.upcoming`` (the weights the step streams next) to their kernels, which ask L2
