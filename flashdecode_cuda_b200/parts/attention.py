@@ -18,10 +18,13 @@ MAX_SPLITS = 32
 PREFETCH_BYTES = 16 << 20   # an output projection up to this size is asked for ahead by the decode q/k/v kernel (whole; a 16 MB
                             # beginning of a larger one made the step slower: + 1.4 % at the sizes of Qwen2.5-7B, batch 8)
 FP32_SPLIT_LEN = 256      # keys per split of a decode step in float32
-# The same for attention without options: one tile of the kernel for heads of 64 and 128, so that a CTA is one chain of lookups,
-# loads, scores and values (csrc/attention_rows.cu) - where no sequence of the cache is so long that the merge would have
-# more than 512 splits to add.
-FP32_TILE_LEN, FP32_MAX_SPLITS = 64, 512
+# The same for attention without options and heads of 64 and more: 64 keys - one tile of the kernel for heads of 64 and 128, so that
+# a CTA is one chain of lookups, loads, scores and values (csrc/attention_rows.cu) - while that is at most 128 splits of the cache's
+# longest sequence, then 128 keys, then 256.  No scratch memory is then larger than splits of 256 make it at 32,768 tokens (64 rows of 40 heads
+# of 128: 170 MB; splits of 64 would take 680).  Measured, 64 against 256 keys, us: 1 row of 1,300 keys, 12 heads of 128
+# 15 / 35; 8 heads of 96 (the general kernel) 25 / 73, of 256 42 / 132; 16 rows of 3,000 keys, heads of 96 216 / 211, of 256 410 / 414, but of 32
+# 145 / 138: smaller heads, whose merge weighs more, stay at 256.
+FP32_TILE_LEN, FP32_TILE_SPLITS, FP32_MAX_SPLITS = 64, 128, 512
 
 
 def plan_splits(n_rows: int, n_kv: int, kv_len_bound: int, sm_count: int):
@@ -44,10 +47,12 @@ def plan_splits(n_rows: int, n_kv: int, kv_len_bound: int, sm_count: int):
     return n_splits, split_len
 
 
-def fp32_splits(ctx):
-    """(n_splits, split_len) of a decode step in float32.  The splits have a fixed length (one per cache), so that where
+def fp32_splits(ctx, head_dim: int):
+    """(n_splits, split_len) of a decode step in float32.  The splits have a fixed length (one per head size and cache), so that where
     a sequence's partial sums are cut - and with it every bit of its result - depends on nothing but its own length."""
-    split_len = FP32_TILE_LEN if ctx.cache.max_len <= FP32_TILE_LEN * FP32_MAX_SPLITS else FP32_SPLIT_LEN
+    split_len = FP32_TILE_LEN if head_dim >= 64 else FP32_SPLIT_LEN
+    while split_len < FP32_SPLIT_LEN and ctx.cache.max_len > split_len * FP32_TILE_SPLITS:
+        split_len *= 2
     return max(1, -(-ctx.kv_len_bound // split_len)), split_len
 
 
@@ -188,7 +193,7 @@ class GQAAttention(Mixer):
         attn = ws.get("attn", (T, self.n_q * d), x.dtype)
         n_splits, split_len, scratch = 1, 0, None
         if ctx.max_q_len == 1 and x.dtype == torch.float32:
-            n_splits, split_len = fp32_splits(ctx)
+            n_splits, split_len = fp32_splits(ctx, d)
             if n_splits > 1:
                 scratch = ws.get("attn_scratch", (K.attention_scratch_floats(T, self.n_q, d, n_splits),),
                                  torch.float32)
@@ -198,7 +203,7 @@ class GQAAttention(Mixer):
                 scratch = ws.get("attn_scratch", (K.attention_scratch_floats(T, self.n_q, d, n_splits),),
                                  torch.float32)
         if x.dtype == torch.float32:
-            cut = single_rows(ctx, self.n_q, d, x.dtype, fp32_splits(ctx)[1])
+            cut = single_rows(ctx, self.n_q, d, x.dtype, fp32_splits(ctx, d)[1])
         else:
             cut = dict(prompt_scratch=prompt_scratch(ctx, self.n_q, d) if ctx.max_q_len > 1 else None, kv_len=ctx.kv_len_bound)
         # a small decode step: when its keys and values are through, the attention kernel asks L2 for the beginning of

@@ -206,3 +206,18 @@ def test_fragmentation_counts_the_unused_tails():
     cache.release(a)
     assert cache.fragmentation() == 0.0
     assert "fragmentation" in repr(cache)
+
+
+@pytest.mark.parametrize("max_len", [64, 1000, 8192, 8193, 16384, 16385, 32768, 32769, 131072])
+def test_float32_decode_splits_stay_bounded(max_len):
+    """The scratch memory of a float32 decode step never exceeds what splits of 256 keys take at 32,768 tokens (128 splits), or
+    at the cache's longest sequence if that is longer; the length of a split does not depend on the step; heads below 64 keep 256."""
+    from types import SimpleNamespace
+    from flashdecode_cuda_b200.parts.attention import FP32_SPLIT_LEN, fp32_splits
+    for d in (16, 32, 48, 64, 96, 128, 256):
+        lengths = set()
+        for bound in {1, 40, min(max_len, 5000), max_len}:
+            n, length = fp32_splits(SimpleNamespace(cache=SimpleNamespace(max_len=max_len), kv_len_bound=bound), d)
+            assert n == -(-bound // length) and n <= max(128, -(-max_len // FP32_SPLIT_LEN)) and length % 64 == 0
+            lengths.add(length)
+        assert len(lengths) == 1 and (d >= 64 or lengths == {FP32_SPLIT_LEN})
