@@ -771,13 +771,23 @@ static int ta_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
 }
 
 // Into how many parts a prompt step's keys are cut: as many as keep one CTA per SM, with four key tiles each (two for
-// each of a CTA's groups) or more; 1 where the CTAs fill more than half of the GPU.
-static int ta_parts(int n_q, int n_rows, int max_q_len, int kv_len) {
+// each of a CTA's groups) or more; 1 where the CTAs fill more than half of the GPU.  What counts is the keys that a CTA's 128
+// queries see: with a window or chunks no more than those and 127.  (Counted from the whole sequence, 128 tokens behind 3,000 with a
+// window of 64, 40 heads, took 17.4 us in three parts and 13.1 in one.)  And only where the tiles that a CTA is spared, 0.8 us
+// each, are more than the parts' stores and the merge take, 3.5 us and half a microsecond per thousand rows (query, head): with a window
+// of 512 two parts took 16.6 us against 17.4 for 4 heads and 128 tokens, but 19.8 against 18.1 for 12 heads and 384.
+static int ta_parts(int n_q, int n_rows, int max_q_len, int kv_len, int window, int chunk) {
     if (g_ta_form != 0) return 1;
+    long long seen = kv_len;
+    if (window > 0 && window + TA_BM - 1ll < seen) seen = window + TA_BM - 1;
+    if (chunk > 0 && chunk + TA_BM - 1ll < seen) seen = chunk + TA_BM - 1;
     const long long ctas = (long long)n_q * ((max_q_len + TA_BM - 1) / TA_BM) * n_rows;
-    const long long fit = ta_sm_count() / ctas, most = (kv_len + TA_BN - 1) / TA_BN / 4;
-    const long long parts = fit < most ? fit : most;
-    return parts < 2 ? 1 : (parts > TA_MAX_PARTS ? TA_MAX_PARTS : (int)parts);
+    const long long fit = ta_sm_count() / ctas, most = (seen + TA_BN - 1) / TA_BN / 4;
+    long long parts = fit < most ? fit : most;
+    if (parts > TA_MAX_PARTS) parts = TA_MAX_PARTS;
+    if (parts < 2) return 1;
+    const double spared = 0.8 * (double)((seen + TA_BN - 1) / TA_BN) * (double)(parts - 1) / (double)parts;
+    return spared > 3.5 + 0.0005 * (double)n_q * n_rows * max_q_len ? (int)parts : 1;
 }
 
 // Returns 1 when it does not take the sizes (the caller falls back to the mma.sync kernel):
@@ -787,7 +797,7 @@ int launch_attn_prefill_tcgen05(const AttnParams& p0, int n_rows, int T, int max
                                 int kv_len, const int* tok_row) {
     AttnParams p = p0;
     if (p.d != TA_D || p.n_splits != 1) return 1;
-    const int parts = scratch != nullptr ? ta_parts(p.n_q, n_rows, max_q_len, kv_len) : 1;
+    const int parts = scratch != nullptr ? ta_parts(p.n_q, n_rows, max_q_len, kv_len, p.window, p.chunk) : 1;
     const int bs = p.block_size;
     if (bs < 8 || bs > 128 || bs % 8 != 0 || 128 % bs != 0) return 1;
     if ((max_q_len + TA_BM - 1) / TA_BM > 65535 || n_rows > 65535) return 1;
@@ -851,10 +861,11 @@ extern "C" int fd_attention_dense(const void* q, const void* kv, const void* rot
     return rc;
 }
 
-// Floats of scratch with which a prompt step of T tokens may be cut into parts (0: it would not be).
-extern "C" long long fd_attn_prompt_scratch_floats(int T, int n_q, int d, int n_rows, int max_q_len, int kv_len) {
+// Floats of scratch with which a prompt step of T tokens may be cut into parts (0: it would not be); without window and
+// chunk enough for any.
+extern "C" long long fd_attn_prompt_scratch_floats(int T, int n_q, int d, int n_rows, int max_q_len, int kv_len, int window, int chunk) {
     if (d != fd::TA_D || T < 1 || n_rows < 1 || max_q_len < 2) return 0;
-    const int parts = fd::ta_parts(n_q, n_rows, max_q_len, kv_len);
+    const int parts = fd::ta_parts(n_q, n_rows, max_q_len, kv_len, window, chunk);
     return parts > 1 ? (long long)T * n_q * parts * (fd::TA_D + 2) : 0;
 }
 

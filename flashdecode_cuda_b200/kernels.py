@@ -159,7 +159,7 @@ def _declare(L: ctypes.CDLL) -> None:
         fn.argtypes = args
         fn.restype = I
     L.fd_attn_scratch_floats.argtypes = [I, I, I, I]
-    L.fd_attn_prompt_scratch_floats.argtypes = [I] * 6
+    L.fd_attn_prompt_scratch_floats.argtypes = [I] * 8
     L.fd_attn_prompt_scratch_floats.restype = LL
     L.fd_launch_count.restype = c_ulonglong
     L.fd_launch_count.argtypes = []
@@ -755,9 +755,11 @@ def attention_scratch_floats(n_tokens: int, n_q: int, head_dim: int, n_splits: i
     return int(lib().fd_attn_scratch_floats(n_tokens, n_q, head_dim, n_splits))
 
 
-def attention_prompt_scratch_floats(n_tokens: int, n_q: int, head_dim: int, n_rows: int, max_q_len: int, kv_len: int) -> int:
-    """Floats of scratch with which ``attention`` may cut a bfloat16 prompt step's keys into parts; 0: it would not."""
-    return int(lib().fd_attn_prompt_scratch_floats(n_tokens, n_q, head_dim, n_rows, max_q_len, kv_len))
+def attention_prompt_scratch_floats(n_tokens: int, n_q: int, head_dim: int, n_rows: int, max_q_len: int, kv_len: int,
+                                    window: int = 0, chunk: int = 0) -> int:
+    """Floats of scratch with which ``attention`` may cut a bfloat16 prompt step's keys into parts; 0: it would not.  Without
+    ``window`` and ``chunk``: enough for any."""
+    return int(lib().fd_attn_prompt_scratch_floats(n_tokens, n_q, head_dim, n_rows, max_q_len, kv_len, window, chunk))
 
 
 _attn_counters = {}      # per device: zeroed ints the decode kernel counts arriving splits in (kept alive for good)
@@ -794,7 +796,7 @@ def _attention(fn_name, q, k_pool, v_pool, out, block_table, tok_row, row_slot, 
             args[-2] = single_split_len if singles else split_len
             kv_len = kv_len if singles else 0
         else:
-            need = attention_prompt_scratch_floats(T, n_q, head_dim, n_rows, max_q_len, kv_len)
+            need = attention_prompt_scratch_floats(T, n_q, head_dim, n_rows, max_q_len, kv_len, int(window), int(chunk))
         assert prompt_scratch is None or (prompt_scratch.dtype == torch.float32 and prompt_scratch.numel() >= need)
     if fn_name != "fd_attention_simt":
         fused = n_splits > 1 and max_q_len == 1 and q.dtype == torch.bfloat16

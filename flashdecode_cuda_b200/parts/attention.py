@@ -71,9 +71,10 @@ def single_rows(ctx, n_q: int, v_dim: int, dtype: torch.dtype, split_len: int) -
     return dict(prompt_scratch=scratch, kv_len=ctx.kv_len_bound, single_split_len=split_len)
 
 
-def prompt_scratch(ctx, n_q: int, head_dim: int) -> Optional[torch.Tensor]:
-    """Workspace memory with which the attention of a prompt step may cut the keys into parts; None where it would not."""
-    n = K.attention_prompt_scratch_floats(ctx.T, n_q, head_dim, ctx.n_rows, ctx.max_q_len, ctx.kv_len_bound)
+def prompt_scratch(ctx, n_q: int, head_dim: int, window: int = 0, chunk: int = 0) -> Optional[torch.Tensor]:
+    """Workspace memory with which the attention of a prompt step may cut the keys into parts; None where it would not.  Without
+    ``window`` and ``chunk``: enough for any."""
+    n = K.attention_prompt_scratch_floats(ctx.T, n_q, head_dim, ctx.n_rows, ctx.max_q_len, ctx.kv_len_bound, window, chunk)
     return ctx.ws.get("attn_prompt_parts", (n,), torch.float32) if n else None
 
 
@@ -205,7 +206,8 @@ class GQAAttention(Mixer):
         if x.dtype == torch.float32:
             cut = single_rows(ctx, self.n_q, d, x.dtype, fp32_splits(ctx, d)[1])
         else:
-            cut = dict(prompt_scratch=prompt_scratch(ctx, self.n_q, d) if ctx.max_q_len > 1 else None, kv_len=ctx.kv_len_bound)
+            parts = prompt_scratch(ctx, self.n_q, d, self.window or 0, self.chunk or 0) if ctx.max_q_len > 1 else None
+            cut = dict(prompt_scratch=parts, kv_len=ctx.kv_len_bound)
         # a small decode step: when its keys and values are through, the attention kernel asks L2 for the beginning of
         # what the step streams after this part (the output projection's weights are in L2 already, see above)
         ahead = ctx.upcoming if ctx.max_q_len == 1 and T <= GEMV_MAX_ROWS and x.dtype == torch.bfloat16 else None

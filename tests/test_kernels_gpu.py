@@ -886,6 +886,20 @@ def test_attention_prompts_in_parts(n_q, n_kv, bs, window):
     assert max(used) >= 4 and min(used) == 0 and any(1 < u < 4 for u in used)
 
 
+@pytest.mark.parametrize("window,most", [(1, 1), (64, 1), (128, 1), (300, 1), (600, 3), (1100, 5), (5000, 8)])
+def test_attention_prompts_in_parts_by_what_a_window_shows(window, most):
+    """The keys are cut by how many of them a CTA's queries see, not by the sequence: no parts (and no merge) for short windows,
+    four key tiles of 64 each at least (window + 127 keys), and right results with the scratch memory that a window asks for."""
+    def fn(q, kp, vp, out, table, tok_row, slots, starts, lens, ctx, rows, m, nq, nkv, d, scale, win, splits, split_len, scr, st):
+        n = K.attention_prompt_scratch_floats(q.shape[0], nq, d, rows, m, 3030, window=win)
+        assert n == (q.shape[0] * nq * most * (d + 2) if most > 1 else 0)
+        assert n == K.attention_prompt_scratch_floats(q.shape[0], nq, d, rows, m, 3030, chunk=win)
+        K.attention(q, kp, vp, out, table, tok_row, slots, starts, lens, ctx, rows, m, nq, nkv, d, scale, win, splits, split_len, scr,
+                    st, prompt_scratch=torch.full((n,), float("nan"), device=DEV) if n else None, kv_len=3030)
+    got, want, _ = run_attention("bfloat16", 4, 1, 128, 64, ctx=[3000], new=[30], window=window, fn=fn, spike=(0, 3029))
+    assert rel(got, want) < TOL["bfloat16"]
+
+
 @pytest.mark.parametrize("n_q,n_kv,d,bs,window", [(12, 2, 128, 16, 0), (8, 1, 64, 64, 0), (3, 3, 128, 7, 0), (16, 2, 64, 16, 70),
                                                   (9, 1, 128, 32, 0), (64, 1, 64, 16, 100)])
 def test_attention_f32_decode_and_prompts(n_q, n_kv, d, bs, window):
