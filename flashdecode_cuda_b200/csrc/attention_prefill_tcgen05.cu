@@ -651,7 +651,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 }
 
 // Adds up the parts of every (token, head), a warp each, four dimensions a lane: m = max m_s, out = sum acc_s e^(m_s - m) / sum
-// l_s e^(m_s - m).  A part without visible keys (l_s = 0) is left out; tokens of padding rows are left alone, as above.
+// l_s e^(m_s - m).  A part without visible keys (l_s = 0) is left out, one whose sum is no number is not: it makes the output NaN, as it
+// would be without parts.  Tokens of padding rows are left alone, as above.
 constexpr int TA_MAX_PARTS = 8;
 
 __global__ void __launch_bounds__(256)
@@ -671,17 +672,17 @@ attn_prompt_merge_kernel(const AttnParams p, const int* __restrict__ tok_row, in
     }
     float m = p.sink != nullptr ? p.sink[h] : -INFINITY;
 #pragma unroll
-    for (int s = 0; s < TA_MAX_PARTS; ++s) if (l_s[s] > 0.f) m = fmaxf(m, m_s[s]);
+    for (int s = 0; s < TA_MAX_PARTS; ++s) if (l_s[s] != 0.f) m = fmaxf(m, m_s[s]);
     float l = p.sink != nullptr ? expf(p.sink[h] - m) : 0.f;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int s = 0; s < TA_MAX_PARTS; ++s) {
-        if (!(l_s[s] > 0.f)) continue;
+        if (l_s[s] == 0.f) continue;
         const float w = expf(m_s[s] - m);
         l = fmaf(l_s[s], w, l);
         o.x = fmaf(a[s].x, w, o.x); o.y = fmaf(a[s].y, w, o.y); o.z = fmaf(a[s].z, w, o.z); o.w = fmaf(a[s].w, w, o.w);
     }
-    const float inv = l > 0.f ? p.out_scale / l : 0.f;
+    const float inv = l == 0.f ? 0.f : p.out_scale / l;
     const __nv_bfloat162 lo2 = __floats2bfloat162_rn(o.x * inv, o.y * inv), hi2 = __floats2bfloat162_rn(o.z * inv, o.w * inv);
     *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.out) + (size_t)tok * p.out_ld + h * TA_D + lane * 4) =
         make_uint2(*reinterpret_cast<const uint32_t*>(&lo2), *reinterpret_cast<const uint32_t*>(&hi2));

@@ -353,7 +353,8 @@ attn_tile_kernel(const AttnParams p) {
 
 // Merge the per-split triples of every (token, query head): m = max m_s,
 // l = sum l_s e^(m_s - m), out = sum acc_s e^(m_s - m) / l.  Splits that saw
-// no key (l_s == 0) are skipped; a padding row gives zeros.  The weights
+// no key (l_s == 0) are skipped (one whose sum is no number is not: the output
+// is NaN then, as it is unsplit); a padding row gives zeros.  The weights
 // e^(m_s - m) / l are computed once per (token, head) into shared memory; then
 // the block's four warps sum over a quarter of the splits each (d a multiple of 4).
 constexpr int COMBINE_MAX_SPLITS = 512;
@@ -384,7 +385,7 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_m, const floa
     // block-wide max of m over the splits that saw a key
     float m = -INFINITY;
     for (int s = threadIdx.x; s < n_splits; s += blockDim.x)
-        if (pl[s] > 0.f) m = fmaxf(m, pm[s]);
+        if (pl[s] != 0.f) m = fmaxf(m, pm[s]);
     m = warp_max(m);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     if (lane == 0) red[warp] = m;
@@ -398,13 +399,13 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_m, const floa
     float lsum = 0.f;
     for (int s = threadIdx.x; s < n_splits; s += blockDim.x) {
         const float ls = pl[s];
-        const float w = ls > 0.f ? expf(pm[s] - m) : 0.f;
+        const float w = ls != 0.f ? expf(pm[s] - m) : 0.f;
         w_s[s] = w;
         lsum += ls * w;
     }
     float l = block_sum(lsum, red);
     if (sink != nullptr) l += expf(sk - m);
-    const float inv = l > 0.f ? out_scale / l : 0.f;
+    const float inv = l == 0.f ? 0.f : out_scale / l;
     const float* pa = part_acc + row * n_splits * d;
     // four dims a lane, every fourth split a warp, eight splits' loads in flight; the four warps' sums are added in order.  (With
     // the first warp taking all splits and the others none it took 7.0 us for 96 heads with 19 splits of 32.)  Which warp adds a

@@ -886,6 +886,32 @@ def test_attention_prompts_in_parts(n_q, n_kv, bs, window):
     assert max(used) >= 4 and min(used) == 0 and any(1 < u < 4 for u in used)
 
 
+@pytest.mark.parametrize("dtype,ctx,new,at", [("bfloat16", 2000, 40, 100), ("bfloat16", 2000, 40, 1990), ("float32", 150, 1, 10),
+                                              ("float32", 150, 1, 149), ("float32", 40, 1, 3)])
+def test_attention_in_parts_or_splits_hides_no_nan(dtype, ctx, new, at):
+    """A key that is no number makes every query that sees it NaN, whichever part or split of the keys it lies in and however many
+    of its splits' scores are no numbers; the other key/value head's results stay what they are."""
+    def fn(q, kp, vp, out, table, tok_row, slots, starts, lens, c, rows, m, nq, nkv, d, scale, win, splits, split_len, scr, st):
+        args = (table, tok_row, slots, starts, lens, c, rows, m, nq, nkv, d, scale, win, splits, split_len, scr, st)
+        kw = {}
+        if dtype == "bfloat16":
+            n = K.attention_prompt_scratch_floats(q.shape[0], nq, d, rows, m, ctx + new)
+            assert n > 0
+            kw = dict(prompt_scratch=torch.full((n,), float("nan"), device=DEV), kv_len=ctx + new)
+        clean = torch.empty_like(out)
+        K.attention(q, kp, vp, clean, *args, **kw)
+        blk = int(table[int(slots[0]), at // 16])
+        kp[blk, 0, at % 16, 5] = float("nan")
+        K.attention(q, kp, vp, out, *args, **kw)
+        half = nq * d // 2
+        assert torch.isnan(out[:, :half]).all() and torch.equal(out[:, half:], clean[:, half:])
+        if dtype == "float32":              # every score of the first split
+            kp[:, 0] = float("nan")
+            K.attention(q, kp, vp, out, *args, **kw)
+            assert torch.isnan(out[:, :half]).all()
+    run_attention(dtype, 6, 2, 128, 16, ctx=[ctx], new=[new], n_splits=1 if new > 1 else -(-(ctx + 1) // 64), split_len=64, fn=fn)
+
+
 @pytest.mark.parametrize("window,most", [(1, 1), (64, 1), (128, 1), (300, 1), (600, 3), (1100, 5), (5000, 8)])
 def test_attention_prompts_in_parts_by_what_a_window_shows(window, most):
     """The keys are cut by how many of them a CTA's queries see, not by the sequence: no parts (and no merge) for short windows,
