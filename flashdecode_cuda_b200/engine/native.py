@@ -13,11 +13,12 @@ does not take, goes through the parts' ``forward``.
 A part whose ``forward`` was wrapped or replaced, on the object or on its class,
 is called: such a model's steps go through the parts.
 
-Kept from step to step: the weights, and their addresses.  Every step looks
-whether a part has changed since (``Part.changes``) and whether the weights lie
-where they lay, and derives everything anew if not (some 10 us at 28 layers).
-The cache's, the step's and the workspace's addresses are taken anew for every
-step.
+Kept from step to step: the weights (their memory, too), and their addresses.
+A step first looks whether a part has changed since (``Part.changes``) and
+derives everything anew if so.  Whether the weights' tensors have been given
+other memory takes 10 us to see at 28 layers, so that is asked behind the
+launches (``moved``), and such a step runs again through the parts.  The
+cache's, the step's and the workspace's addresses are taken anew for every step.
 """
 
 from __future__ import annotations
@@ -76,7 +77,7 @@ class DensePrompts:
         """The launches' constants from the model's parts as they are now; ``layers`` None: not a model of this kind."""
         self.derived_at = Part.changes                              # before anything is read
         self.blocks = list(self.model.blocks)
-        self.tensors, self.where = [], []
+        self.tensors, self.where, self.memory = [], [], []
         self.layers = self._layers()
 
     def _layers(self):
@@ -111,7 +112,7 @@ class DensePrompts:
             if any(w.dtype != torch.bfloat16 or w.shape != shape for w, shape in shapes) or \
                     any(v.dtype not in (torch.bfloat16, torch.float32) or v.shape != (n,) for v, n in vectors):
                 return None
-        self.tensors, self.where = tensors, list(map(_address, tensors))
+        self.tensors, self.where, self.memory = tensors, list(map(_address, tensors)), [t.detach() for t in tensors]
         self.positions, self.n = positions, len(blocks)
         self.hidden = H
         m, f = blocks[0].mixer, blocks[0].feed_forward
@@ -139,7 +140,7 @@ class DensePrompts:
         T = ctx.T
         if linear.PROMPT_GEMM != "auto" or ctx.max_q_len < 2 or T <= linear.GEMV_MAX_ROWS:
             return False
-        if self.derived_at != Part.changes or self.blocks != self.model.blocks or list(map(_address, self.tensors)) != self.where:
+        if self.derived_at != Part.changes or self.blocks != self.model.blocks:
             self._derive()
         if self.layers is None or [kind.forward for kind in KINDS] != FORWARDS:
             return False
@@ -147,6 +148,13 @@ class DensePrompts:
         if T <= linear.STREAM_MAX_ROWS:
             return all(linear.stream_gemm(T, n, k) for n, k in ((self.qkv, H), (H, self.n_q * self.d), (2 * self.inter, H), (H, self.inter)))
         return linear.fused_prompt_gemm(T, self.qkv, H) and linear.fused_prompt_gemm(T, 2 * self.inter, H)
+
+    def moved(self) -> bool:
+        """Whether a weight's tensor has other memory than the step that was just launched used; then everything is derived anew."""
+        if list(map(_address, self.tensors)) == self.where:
+            return False
+        self._derive()
+        return True
 
     def run(self, ctx, resid: torch.Tensor) -> torch.Tensor:
         """Every schedule entry of the step; returns the last one's output, still to be added to ``resid``."""
