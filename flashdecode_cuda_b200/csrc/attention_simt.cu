@@ -356,7 +356,7 @@ attn_tile_kernel(const AttnParams p) {
 // no key (l_s == 0) are skipped (one whose sum is no number is not: the output
 // is NaN then, as it is unsplit); a padding row gives zeros.  The weights
 // e^(m_s - m) / l are computed once per (token, head) into shared memory; then
-// the block's four warps sum over a quarter of the splits each (d a multiple of 4).
+// the block's four warps share the splits, or the dims of wide heads (d a multiple of 4).
 constexpr int COMBINE_MAX_SPLITS = 512;
 
 template <typename T>
@@ -407,25 +407,48 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_m, const floa
     if (sink != nullptr) l += expf(sk - m);
     const float inv = l == 0.f ? 0.f : out_scale / l;
     const float* pa = part_acc + row * n_splits * d;
-    // four dims a lane, every fourth split a warp, eight splits' loads in flight; the four warps' sums are added in order.  (With
-    // the first warp taking all splits and the others none it took 7.0 us for 96 heads with 19 splits of 32.)  Which warp adds a
-    // split depends on the split alone, not on how many there are.
-    __shared__ __align__(16) float sums[4][DV_MAX];
-    for (int j = lane * 4; j < d; j += 128) {
+    // Four dims a thread, eight splits' loads in flight.  (A split that saw no key has weight 0 and may have left its accumulators unwritten.)
+    auto part = [&](int s, int j) {
+        return w_s[s] != 0.f ? *reinterpret_cast<const float4*>(pa + (size_t)s * d + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if (d > 256) {
+        // as many dims as the block's threads take: all splits a thread (every fourth split a warp, below, and all dims in turn made
+        // it 10.3 us instead of 5.9 for 16 heads of 512 with 24 splits)
+        const int j = threadIdx.x * 4;
+        if (j >= d) return;
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
-        for (int s = warp; s < n_splits; s += 4) {
+        for (int s = 0; s < n_splits; ++s) {
             const float w = w_s[s];
-            // (a split that saw no key has weight 0 and may have left its accumulators unwritten)
-            const float4 v = w != 0.f ? *reinterpret_cast<const float4*>(pa + (size_t)s * d + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 v = part(s, j);
             a.x = fmaf(v.x, w, a.x); a.y = fmaf(v.y, w, a.y); a.z = fmaf(v.z, w, a.z); a.w = fmaf(v.w, w, a.w);
         }
-        *reinterpret_cast<float4*>(&sums[warp][j]) = a;
+        const float r[4] = {a.x * inv, a.y * inv, a.z * inv, a.w * inv};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { if (out_f32) of[j + e] = r[e]; else o[j + e] = from_float<T>(r[e]); }
+        return;
+    }
+    // 128 dims a warp; the other warps share the splits, every fourth one each (heads of 129 to 256: every second), and their sums are added
+    // in order.  (With the first warp taking all splits and the others none it took 7.9 us for 12 heads of 128 with 24 splits, and takes
+    // 5.0; 16 heads of 256 7.1 and 5.1.)  Which warp adds a split depends on the split and the head size alone, not on how many there are.
+    __shared__ __align__(16) float sums[4][256];
+    const int shares = d <= 128 ? 4 : 2, share = warp & (shares - 1), j = warp / shares * 128 + lane * 4;
+    if (j < d) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int s = share; s < n_splits; s += shares) {
+            const float w = w_s[s];
+            const float4 v = part(s, j);
+            a.x = fmaf(v.x, w, a.x); a.y = fmaf(v.y, w, a.y); a.z = fmaf(v.z, w, a.z); a.w = fmaf(v.w, w, a.w);
+        }
+        *reinterpret_cast<float4*>(&sums[share][j]) = a;
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < d; j += blockDim.x) {
-        const float r = (((sums[0][j] + sums[1][j]) + sums[2][j]) + sums[3][j]) * inv;
-        if (out_f32) of[j] = r; else o[j] = from_float<T>(r);
+    for (int i = threadIdx.x; i < d; i += blockDim.x) {
+        float r = sums[0][i] + sums[1][i];
+        if (shares == 4) r = (r + sums[2][i]) + sums[3][i];
+        r *= inv;
+        if (out_f32) of[i] = r; else o[i] = from_float<T>(r);
     }
 }
 

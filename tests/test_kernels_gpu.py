@@ -757,6 +757,16 @@ def test_attention_decode_splits_odd_counts(dtype):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("d", [8, 120, 128, 136, 256, 264, 384, 392, 512])
+def test_attention_merges_splits_of_wide_heads(dtype, d):
+    """The merge's shares of splits and dims at the edges of its 128 dims per warp, with fewer splits than shares and with more."""
+    for n_splits, split_len in ((2, 160), (3, 128), (10, 32), (21, 32)):
+        got, want, pad = run_attention(dtype, 4, 2, d, 16, ctx=[0, 37, 299], new=[1] * 3, n_splits=n_splits, split_len=split_len, pad_rows=1)
+        assert rel(got, want) < TOL[dtype], n_splits
+        assert float(pad.float().abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_attention_far_key_stands_out(dtype):
     """Among 700 keys one early key carries nearly all the weight of the last
     query; it lies in the first split and in a block far from the others."""
