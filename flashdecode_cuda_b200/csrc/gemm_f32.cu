@@ -1,5 +1,5 @@
 // C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]) in float32 on the CUDA cores: the matrix product of the true 32-bit path
-// (more than 16 rows of A that are not 16-byte aligned go to gemm_simt.cu's general kernel).
+// (rows that are not 16-byte aligned go to gemm_simt.cu, but for up to 16 rows of A and W of few rows).
 //
 // Every output element is one fmaf chain over k = 0 .. K-1 in that order, in every kernel and tiling of this file and in
 // the general kernel, so a token gives the same bits alone, in a prompt and in any batch; nothing is split over K.  What is
@@ -330,15 +330,18 @@ int launch_gemm_f32(const float* A, const float* W, const float* bias, float* C,
                     cudaStream_t stream) {
     if (M <= 16) {
         const bool wide = N >= 64 * 148;         // 64 rows of W per CTA still give every SM one
-        if (!aligned) return wide ? launch_rows<64, 64, 5, 16, 4, 2, 1, false>(A, W, bias, C, M, N, K, stream)
-                                  : launch_rows<16, 256, 3, 16, 2, 1, 4, false>(A, W, bias, C, M, N, K, stream);
+        // rows that are not 16-byte aligned come four bytes a copy: short steps and many CTAs (8 x 333 x 1,537 15 us, 8 x 64 x 65 2.8; with steps
+        // of 256 k and 16 rows 39 and 8.0), and the caller's kernel where W has many rows
+        if (!aligned) return wide ? 1 : launch_rows<8, 32, 6, 16, 1, 1, 1, false>(A, W, bias, C, M, N, K, stream);
         if (wide) {
             if (M <= 1) return launch_rows<64, 128, 3, 1, 1, 1, 4>(A, W, bias, C, M, N, K, stream);
             if (M <= 2) return launch_rows<64, 128, 3, 2, 1, 1, 4>(A, W, bias, C, M, N, K, stream);
             if (M <= 4) return launch_rows<64, 128, 3, 4, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
-            if (M <= 8) return launch_rows<64, 128, 3, 8, 2, 2, 1>(A, W, bias, C, M, N, K, stream);
+            if (M <= 8 && K > 64) return launch_rows<64, 128, 3, 8, 2, 2, 1>(A, W, bias, C, M, N, K, stream);
             return launch_rows<64, 64, 5, 16, 4, 2, 1>(A, W, bias, C, M, N, K, stream);
         }
+        // a short chain is not worth a ring of long steps, most of which may lie beyond K (16 x 8 x 64 4.6 us in those, 2.2 here; 16 x 1,536 x 384 6.4 and 4.3)
+        if (K <= 384) return launch_rows<16, 64, 4, 16, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
         if (M <= 1) return launch_rows<16, 256, 5, 1, 1, 1, 8>(A, W, bias, C, M, N, K, stream);
         if (M <= 2) return launch_rows<16, 256, 5, 2, 1, 1, 4>(A, W, bias, C, M, N, K, stream);
         if (M <= 4) return launch_rows<16, 256, 5, 4, 1, 1, 4>(A, W, bias, C, M, N, K, stream);

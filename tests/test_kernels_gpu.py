@@ -355,6 +355,26 @@ def test_gemm_f32_forms_give_the_same_bits(M, N, K_):
         K.gemm_f32_set_form(0)
 
 
+@pytest.mark.parametrize("N,K_", [(8, 64), (333, 1), (100, 384), (100, 388), (9472, 64), (9472, 68), (9471, 37), (9472, 37), (9500, 133)])
+@pytest.mark.parametrize("M", [1, 5, 8, 9, 16])
+def test_gemm_f32_few_rows_at_the_edges_of_the_rule(M, N, K_):
+    """Up to 16 rows, aligned and not: short chains and just longer ones, matrices just narrow and just wide, one value of k.  The
+    bits are those of the general kernel (which takes 17 rows off the 16-byte boundary)."""
+    g = torch.Generator().manual_seed(9)
+    rows = torch.randn(17, K_, generator=g)
+    w, b = torch.randn(N, K_, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
+    off = torch.empty(17 * K_ + 1, device=DEV)[1:].view(17, K_)
+    off.copy_(rows)
+    want = torch.full((17, N), float("nan"), device=DEV)
+    K.gemm_simt(off, w, b, want)
+    # as above: a rounding of 2^-24 per product and sum of size one
+    assert rel(want, P.linear(rows.double(), w.double().cpu(), b.double().cpu())) < 2e-6
+    for x in (rows[:M].to(DEV), off[:M]):
+        out = torch.full((M + 1, N), float("nan"), device=DEV)
+        K.gemm_simt(x, w, b, out[:M])
+        assert torch.equal(out[:M], want[:M]) and bool(torch.isnan(out[M]).all())
+
+
 # ---------------------------------------------------------------------------
 # paged cache helpers for the rope and attention kernels
 # ---------------------------------------------------------------------------
