@@ -762,11 +762,11 @@ static int ta_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
     const bool split = p.n_splits > 1 || g_ta_form == 2 || (g_ta_form == 0 && shared_ctas < ta_sm_count());
     if (split) {
         dim3 grid(p.n_q, (max_q_len + TA_BM - 1) / TA_BM, n_rows * (DENSE ? 1 : p.n_splits));
-        return launch_with(prompt_pdl(stream), "attention_prefill_tcgen05", attn_prefill_tcgen05_kernel<KS, VS, true, DENSE>, grid, dim3(TA_THREADS),
+        return launch_with(true, "attention_prefill_tcgen05", attn_prefill_tcgen05_kernel<KS, VS, true, DENSE>, grid, dim3(TA_THREADS),
                            smem_split, stream, dim3(1, 1, 1), mq, mk, mv, mr, p, g_tc_wait_ns, g_tc_skip_last);
     } else {
         dim3 grid(p.n_q, (max_q_len + TA_ROWS - 1) / TA_ROWS, n_rows);
-        return launch_with(prompt_pdl(stream), "attention_prefill_tcgen05", attn_prefill_tcgen05_kernel<KS, VS, false, DENSE>, grid, dim3(TA_THREADS),
+        return launch_with(true, "attention_prefill_tcgen05", attn_prefill_tcgen05_kernel<KS, VS, false, DENSE>, grid, dim3(TA_THREADS),
                            smem_two, stream, dim3(1, 1, 1), mq, mk, mv, mr, p, g_tc_wait_ns, g_tc_skip_last);
     }
 }
@@ -815,7 +815,7 @@ int launch_attn_prefill_tcgen05(const AttnParams& p0, int n_rows, int T, int max
     }
     const int rc = ta_launch<2, 2, false>(mq, mk, mv, mk, p, n_rows, max_q_len, stream);
     if (rc != 0 || p.n_splits == 1) return rc;
-    return launch_with(prompt_pdl(stream), "attention_prompt_merge", attn_prompt_merge_kernel, dim3((T * p.n_q + 7) / 8), dim3(256),
+    return launch_with(true, "attention_prompt_merge", attn_prompt_merge_kernel, dim3((T * p.n_q + 7) / 8), dim3(256),
                        0, stream, dim3(1, 1, 1), p, tok_row, T * p.n_q);
 }
 

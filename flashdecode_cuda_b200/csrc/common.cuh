@@ -169,20 +169,10 @@ inline int launch(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 bl
     return launch_with(g_pdl != 0, what, kernel, grid, block, smem, stream, cluster, args...);
 }
 
-// Prompt steps launch their norms, products and attention programmatically: a kernel is set up while the one before it drains, a
-// product's barriers and tensor memory included (the attention kernel waits first: it reads its row's lengths before anything else).
-// Launched into a graph none of them is: there every programmatic edge cost more than it gave (a norm of 400 rows of 1,536, back to back:
-// 2.6 us without, 3.1 with; a product of 129 x 4,608 x 3,584 21.9 and 23.6).  A norm or product that does not know its step's kind goes by
-// the number of rows.
+// Prompt steps launch their norms, products and attention programmatically: a kernel is set up, and its barriers and tensor
+// memory are ready, while the one before it drains.  Decode steps are replayed from graphs, where every programmatic edge
+// cost more than it gave: a norm or product that does not know its step's kind goes by the number of rows.
 constexpr int PDL_MIN_ROWS = 129;
-
-// Whether a prompt step's kernel is launched programmatically on this stream now: not into a graph.
-inline bool prompt_pdl(cudaStream_t stream) {
-    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &s) == cudaSuccess) return s == cudaStreamCaptureStatusNone;
-    cudaGetLastError();              // (the legacy stream while another one is captured: the launch itself reports that)
-    return false;
-}
 
 // fd_add_rmsnorm with the choice of a programmatic launch (elementwise.cu)
 int add_rmsnorm(const void* delta, int delta_dtype, int n_parts, long long part_stride, float* resid, int write_resid,

@@ -61,7 +61,7 @@ extern "C" int fd_dense_mixer(const FdDenseStep* s, const FdDenseLayer* L, const
     char* kp = s->k_base[g] + L->index * s->k_stride[g];
     char* vp = s->v_base[g] + L->index * s->v_stride[g];
     int rc = fd::add_rmsnorm(delta, 1, 1, 0, s->resid, 1, L->norm1, L->norm1_f32 ? 0 : 1, (float)L->eps1, s->normed, 1, nullptr, T, H,
-                             1.f, fd::prompt_pdl(s->stream), s->stream);
+                             1.f, true, s->stream);
     if (rc != 0) return rc;
     if (s->streams)
         rc = fd_gemm_stream_qkv_rope(s->normed, L->w_qkv, L->b_qkv, (int)L->bias_f32, s->q, T, H, 0, s->cos_t[r], s->sin_t[r],
@@ -85,7 +85,7 @@ extern "C" int fd_dense_mixer(const FdDenseStep* s, const FdDenseLayer* L, const
 extern "C" int fd_dense_gate_up(const FdDenseStep* s, const FdDenseLayer* L) {
     const int T = (int)s->T, H = (int)L->hidden, I = (int)L->inter;
     const int rc = fd::add_rmsnorm(s->mixer_out, 1, 1, 0, s->resid, 1, L->norm2, L->norm2_f32 ? 0 : 1, (float)L->eps2, s->normed, 1,
-                                  nullptr, T, H, 1.f, fd::prompt_pdl(s->stream), s->stream);
+                                  nullptr, T, H, 1.f, true, s->stream);
     if (rc != 0) return rc;
     if (s->streams) return fd_gemm_stream(s->normed, L->w_gate_up, nullptr, 0, s->act, 3, T, 2 * I, H, 0, s->status, nullptr, 0, 0, s->stream);
     return fd_gemm_tc(s->normed, L->w_gate_up, nullptr, 0, s->act, 3, T, 2 * I, H, s->status, s->stream);

@@ -429,7 +429,7 @@ extern "C" int fd_add_rmsnorm(const void* delta, int delta_dtype, int n_parts, l
                               void* out, int out_dtype, const int* rows, int n_out, int H, float dscale,
                               cudaStream_t stream) {
     return fd::add_rmsnorm(delta, delta_dtype, n_parts, part_stride, resid, write_resid, weight, w_dtype, eps, out, out_dtype,
-                           rows, n_out, H, dscale, n_out >= PDL_MIN_ROWS && prompt_pdl(stream), stream);
+                           rows, n_out, H, dscale, n_out >= PDL_MIN_ROWS, stream);
 }
 
 // tiled == 0: gu = [gate (I columns) | up (I columns)]; tiled != 0: tiles of 8 gate + 8 up columns.

@@ -723,7 +723,7 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
     const bool narrow = wide && g_tc_wide == 1 && (long long)tiles_m * ((p.N + TN_BN - 1) / TN_BN) <= sms;
     const int tiling = wide && !narrow && g_tc_wide == 1 && p.tile_expert == nullptr ? choose_tiling(p, sms) : 0;
     const bool pair = wide && (g_tc_wide == 2 || tiling == 2), mid = wide && (g_tc_wide == 4 || tiling == 1);
-    const bool pdl = g_pdl != 0 || (p.M >= PDL_MIN_ROWS && prompt_pdl(stream));
+    const bool pdl = g_pdl != 0 || p.M >= PDL_MIN_ROWS;
     CUtensorMap mx, mw;
     if (pair) {
         const int tiles_m2 = (p.M + 2 * TC_BM - 1) / (2 * TC_BM), tiles_n = (p.N + TW_BN - 1) / TW_BN;

@@ -1153,43 +1153,6 @@ def _rotary_case(M, n_q, n_kv, d, bs, Kd, n_pos, seed):
                 q=torch.zeros(M, n_q * d, dtype=bf, device=DEV))
 
 
-def _programmatic_edges(graph):
-    """(edges, programmatic ones) of a captured graph."""
-    import ctypes
-    cu = ctypes.CDLL("libcuda.so.1")
-    n = ctypes.c_size_t(0)
-    h = ctypes.c_void_p(graph.raw_cuda_graph())
-    assert cu.cuGraphGetEdges_v2(h, None, None, None, ctypes.byref(n)) == 0
-    a, b, data = (ctypes.c_void_p * n.value)(), (ctypes.c_void_p * n.value)(), (ctypes.c_uint8 * (8 * n.value))()
-    assert cu.cuGraphGetEdges_v2(h, a, b, data, ctypes.byref(n)) == 0
-    return n.value, sum(data[8 * i + 2] == 1 for i in range(n.value))       # byte 2: the edge's type, 1 = programmatic
-
-
-@pytest.mark.parametrize("rows", [64, 129, 192, 256])
-def test_decode_kernels_of_many_rows_leave_no_programmatic_edges_in_graphs(rows):
-    """Norms and products of a decode step's batch sizes, launched into a graph: ordered one after the other in full (a prompt
-    step of as many rows, launched directly, lets the next kernel set up early)."""
-    x, w, resid = torch.randn(rows, 512, device=DEV).bfloat16(), torch.randn(768, 512, device=DEV).bfloat16(), torch.randn(rows, 512, device=DEV)
-    gain, out, y, st = torch.ones(512, device=DEV), torch.empty(rows, 512, device=DEV).bfloat16(), torch.empty(rows, 768, device=DEV).bfloat16(), status()
-
-    def step():
-        K.add_rmsnorm(x, resid, gain, 1e-6, out, write_resid=False)
-        K.gemm_tc(out, w, None, y, status=st)
-        K.add_rmsnorm(x, resid, gain, 1e-6, out, write_resid=False)
-    step()
-    want = y.clone()
-    torch.cuda.synchronize()
-    g = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(g):
-        step()
-    edges, programmatic = _programmatic_edges(g)
-    assert edges >= 2 and programmatic == 0
-    y.zero_()
-    g.replay()
-    torch.cuda.synchronize()
-    assert torch.equal(y, want) and int(st.item()) == 0
-
-
 ROTARY_KERNELS = {
     "gemv": lambda c, dims, st: K.gemv_qkv_rope(c["x"], c["w"], None, c["q"], c["cos"], c["sin"], c["tok_row"], c["tok_pos"],
                                                 c["row_slot"], c["kp"], c["vp"], c["table"], *dims, True, st, 1),
