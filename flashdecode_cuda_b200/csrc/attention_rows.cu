@@ -259,15 +259,19 @@ attn_rows_decode_kernel(const AttnParams p) {
     }
 }
 
-constexpr int PR = 64;             // rows (query, head) per CTA of the prompt kernel
+// Rows (query, head) per CTA of the prompt kernel: 64, eight per thread, or 8 in steps whose rows of a group are no more (a few
+// queries of heads without groups: 2 queries of 8 heads of 128 12.0 us in the general kernel, 13.9 in tiles of 64 rows, 7.0 in tiles of 8).
+// A row's sums are the same in either.
+constexpr int PR_MAX = 64;
 
-template <int HD>
-constexpr int prompt_smem_floats() { return 2 * FT * (HD + 4) + FT * HD; }
+template <int HD, int TM>
+constexpr int prompt_smem_floats() { return 8 * TM * (HD + 4) + FT * (HD + 4) + FT * HD; }
 
-template <int HD>
+template <int HD, int TM>
 __global__ void __launch_bounds__(FTHREADS, 2)
 attn_f32_prompt_kernel(const AttnParams p) {
-    constexpr int LD = HD + 4, PLD = FT + 4, TM = 8, TN = 4, TV = HD / 16;     // a thread: 8 rows, 4 keys, TV dims
+    constexpr int PR = 8 * TM;
+    constexpr int LD = HD + 4, PLD = FT + 4, TN = 4, TV = HD / 16;             // a thread: TM rows, 4 keys, TV dims
     static_assert(PR * PLD <= FT * LD, "the weights take the keys' place");
     extern __shared__ __align__(16) float sm[];
     float* q_s = sm;                                         // [PR][LD]
@@ -423,24 +427,29 @@ int launch_decode(const AttnParams& p, int n_rows, cudaStream_t stream) {
     return check_launch("attention_rows_decode");
 }
 
+template <int HD, int TM>
+int launch_prompt(AttnParams p, int n_rows, int max_q_len, cudaStream_t stream) {
+    constexpr int smem = prompt_smem_floats<HD, TM>() * (int)sizeof(float);
+    static bool done = false;
+    const int rc = configure(attn_f32_prompt_kernel<HD, TM>, smem, done);
+    if (rc != 0) return rc;
+    p.QT = 8 * TM / p.G < max_q_len ? 8 * TM / p.G : max_q_len;
+    attn_f32_prompt_kernel<HD, TM><<<dim3((max_q_len + p.QT - 1) / p.QT, p.n_kv, n_rows), FTHREADS, smem, stream>>>(p);
+    return check_launch("attention_f32_prompt");
+}
+
 template <int HD>
 int launch_f32(const AttnParams& p0, int n_rows, int max_q_len, cudaStream_t stream) {
     AttnParams p = p0;
     // Which kernel takes a row depends on its group and on how many tokens it brings, never on the splits: those follow from the
     // batch's longest sequence, and a row's bits must not.
-    if (p.G > PR) return 1;
+    if (p.G > PR_MAX) return 1;
     if (max_q_len == 1) {
         p.kv_div = (p.G + GDEC - 1) / GDEC;
         return p.n_kv * p.kv_div <= 65535 ? launch_decode<float, HD, 1, GDEC>(p, n_rows, stream) : 1;
     }
     if (p.n_splits > 1) return 1;
-    p.QT = PR / p.G < max_q_len ? PR / p.G : max_q_len;
-    constexpr int smem = prompt_smem_floats<HD>() * (int)sizeof(float);
-    static bool done = false;
-    const int rc = configure(attn_f32_prompt_kernel<HD>, smem, done);
-    if (rc != 0) return rc;
-    attn_f32_prompt_kernel<HD><<<dim3((max_q_len + p.QT - 1) / p.QT, p.n_kv, n_rows), FTHREADS, smem, stream>>>(p);
-    return check_launch("attention_f32_prompt");
+    return (long long)max_q_len * p.G <= 8 ? launch_prompt<HD, 1>(p, n_rows, max_q_len, stream) : launch_prompt<HD, 8>(p, n_rows, max_q_len, stream);
 }
 
 }  // namespace

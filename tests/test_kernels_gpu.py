@@ -987,6 +987,29 @@ def test_attention_f32_decode_bits_do_not_depend_on_the_batch(n_q, n_kv, d):
         assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]), ctx
 
 
+@pytest.mark.parametrize("n_q,n_kv,d,most", [(4, 4, 128, 8), (4, 2, 64, 4), (8, 2, 128, 2), (9, 1, 128, 7)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_attention_f32_short_prompts_in_small_tiles(n_q, n_kv, d, most, window):
+    """Steps whose rows of a group fit a tile of 8 (just, and one more token; a group of 9 never does), after cached keys: right, and the
+    same bits beside a longer prompt, which brings tiles of 64."""
+    for n in (2, most, most + 1):
+        outs = []
+        for other in (0, 70):
+            new = [n, 2] + ([other] if other else [])
+            got, want, _ = run_attention("float32", n_q, n_kv, d, 16, ctx=[130, 0, 10][:len(new)], new=new, window=window, fn=K.attention)
+            assert rel(got, want) < TOL["float32"], (n, other)
+
+        def fn(q, kp, vp, out, table, tok_row, slots, starts, lens, ctx, rows, m, nq, nkv, d_, scale, win, splits, split_len, scr, st):
+            rest = (nq, nkv, d_, scale, win, splits, split_len, scr, st)
+            K.attention(q, kp, vp, out, table, tok_row, slots, starts, lens, ctx, rows, m, *rest)
+            alone = torch.empty_like(out[:n + 2])
+            K.attention(q[:n + 2].contiguous(), kp, vp, alone, table, tok_row[:n + 2].contiguous(), slots[:2].contiguous(),
+                        starts[:2].contiguous(), lens[:2].contiguous(), ctx[:2].contiguous(), 2, n, *rest)
+            outs.append(torch.equal(out[:n + 2], alone))
+        run_attention("float32", n_q, n_kv, d, 16, ctx=[130, 0, 10], new=[n, 2, 70], window=window, fn=fn)
+        assert outs == [True], n
+
+
 @pytest.mark.parametrize("n_q,n_kv,d,window", [(12, 2, 128, 0), (9, 1, 64, 0), (5, 5, 128, 100), (12, 2, 96, 0), (66, 1, 128, 0)])
 @pytest.mark.parametrize("split_len", [64, 256])
 def test_attention_f32_single_tokens_beside_prompts(n_q, n_kv, d, window, split_len):
