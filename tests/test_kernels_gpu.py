@@ -1176,6 +1176,36 @@ def _rotary_case(M, n_q, n_kv, d, bs, Kd, n_pos, seed):
                 q=torch.zeros(M, n_q * d, dtype=bf, device=DEV))
 
 
+@pytest.mark.parametrize("rows", [128, 129, 192, 256])
+def test_many_rows_replay_from_graphs_as_they_run(rows):
+    """Norms and products of a decode step's larger batches, replayed from a graph, whose edges are programmatic from 129 rows on:
+    each kernel sees what the one before it wrote, and the next replay overwrites nothing that is still read."""
+    x, resid = torch.randn(rows, 512, device=DEV).bfloat16(), torch.randn(rows, 512, device=DEV)
+    w1, w2 = (torch.randn(n, k, device=DEV).bfloat16() / 20 for n, k in ((768, 512), (512, 768)))
+    gain, a, b, c, st = torch.ones(512, device=DEV), torch.empty_like(x), torch.empty(rows, 768, device=DEV).bfloat16(), torch.empty_like(x), status()
+
+    def step():
+        for _ in range(4):
+            K.add_rmsnorm(x, resid, gain, 1e-6, a)
+            K.gemm_tc(a, w1, None, b, status=st)
+            K.gemm_tc(b, w2, None, c, status=st)
+            x.copy_(c)
+    start = x.clone(), resid.clone()
+    step()
+    step()
+    want = resid.clone(), x.clone()
+    x.copy_(start[0])
+    resid.copy_(start[1])
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        step()
+    g.replay()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(resid, want[0]) and torch.equal(x, want[1]) and int(st.item()) == 0
+
+
 ROTARY_KERNELS = {
     "gemv": lambda c, dims, st: K.gemv_qkv_rope(c["x"], c["w"], None, c["q"], c["cos"], c["sin"], c["tok_row"], c["tok_pos"],
                                                 c["row_slot"], c["kp"], c["vp"], c["table"], *dims, True, st, 1),
