@@ -346,7 +346,8 @@ def test_norm_per_head_with_gate_into_a_shared_buffer(dtype, H, dv, weighted, ga
     assert bool((out[:, :col] == 9.0).all()) and bool((out[:, col + H * dv:] == 9.0).all())
 
 
-def _mixed_attention_case(dtype, d, dv, G, n_kv, window, keep, softcap, bs, S, portions, seed, far=False, tensor_cores=True):
+def _mixed_attention_case(dtype, d, dv, G, n_kv, window, keep, softcap, bs, S, portions, seed, far=False, tensor_cores=True,
+                          split_len=64):
     """Keys that stand out: every seventh position (each is the oldest key inside the window of one query and the
     newest outside it for the next), the last kept position and the first that is not kept, and - with ``far`` - one
     key hundreds of positions back that only the kept range or a long window still shows.  A visibility that is one
@@ -387,9 +388,8 @@ def _mixed_attention_case(dtype, d, dv, G, n_kv, window, keep, softcap, bs, S, p
         if n <= 0:
             break
         tok_row, _, row_slot, q_start, q_len, ctx_len = step_arrays([at], [n], [1])
-        n_splits, split_len, scratch = 1, 0, None
-        if n == 1 and at + 1 > 64:
-            split_len = 64
+        n_splits, scratch = 1, None
+        if n == 1 and at + 1 > split_len:
             n_splits = -(-(at + 1) // split_len)
             scratch = torch.zeros(K.attention_scratch_floats(1, n_q * n_kv, dv, n_splits), device=DEV)
         per_head = torch.full((n, n_q * n_kv * dv), float("nan"), device=DEV)
@@ -439,6 +439,22 @@ def test_capped_windowed_attention_in_portions_and_token_by_token(dtype, case):
     _mixed_attention_case(dtype, d, dv, G, n_kv, window, keep, cap, bs, S, [w * 2 - 1, 2, w, 3, 129, 2] + [1] * S, seed=2,
                           far=True)
     _mixed_attention_case(dtype, d, dv, G, n_kv, window, keep, cap, bs, min(S, 3 * w + keep + 2), [1] * S, seed=3)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("split_len", [64, 96, 160, 1024])
+@pytest.mark.parametrize("case", [  # d, dv, G, n_kv, window, kept, soft cap, block size, length
+    (128, 128, 4, 4, 200, 70, 15.0, 16, 450),     # four value heads, kept positions over two tiles
+    (64, 64, 4, 4, 70, 130, None, 64, 400),       # more kept positions than the window is long
+    (128, 128, 1, 4, None, 0, 30.0, 16, 200),     # one query head per key head, no window
+    (64, 64, 3, 3, 100, 70, 10.0, 16, 300),       # three value heads, and groups of eight on two: the general kernel's
+    (64, 64, 8, 2, 100, 5, 10.0, 16, 250),
+])
+def test_mixed_heads_decode_on_more_value_heads_and_splits_off_the_tiles(dtype, case, split_len):
+    """Decode steps whose weights go to every value head: each number of value heads and group of the kernel for heads of 64 and 128
+    and the first that it leaves to the general one; splits of its 64-key tiles, off them, and none."""
+    d, dv, G, n_kv, window, keep, cap, bs, S = case
+    _mixed_attention_case(dtype, d, dv, G, n_kv, window, keep, cap, bs, S, [S - 100] + [1] * 100, seed=4, far=True, split_len=split_len)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
