@@ -677,8 +677,10 @@ int g_tc_wide = 1;      // where N >= 256: 1: the persistent one-SM kernel (128 
                         // than the SMs), 128 x 192 or the two-SM kernel by choose_tiling; 2: the two-SM kernel; 3, 4: one SM and
                         // 128 x 256 or 128 x 192 tiles always; 0: 128 x 128 tiles, one per CTA
 
-// The tiling of a product of several rounds over the SMs: 0 one SM per 128 x 256 tile, 1 one SM per 128 x 192, 2 two SMs per 256 x 256.  A
-// round's time goes with the bytes it brings in (rows of x + rows of W), and a pair's takes 0.87 of the wide tile's where the
+enum { TILING_WIDE = 0, TILING_MID = 1, TILING_PAIR = 2, TILING_NARROW = 3, TILING_SINGLE = 4 };
+
+// The tiling of a product of several rounds over the SMs: TILING_WIDE one SM per 128 x 256 tile, _MID one SM per 128 x 192, _PAIR two SMs
+// per 256 x 256.  A round's time goes with the bytes it brings in (rows of x + rows of W), and a pair's takes 0.87 of the wide tile's where the
 // products of a tile are long: gate/up of 5,120 columns at 1,200 and 2,048 rows 250 / 280 and 378 / 442 us (pair / one SM), of 3,584
 // columns at 2,048 rows 376 / 444, q/k/v of the same 142 / 162 and 67 / 78; 0.94 at 1,536 columns (gate/up at 2,048 and 9,208
 // rows 83 / 89 and 336 / 365), where the q/k/v epilogue is the longer part and the pair slower (78 / 68).  Coarser rounds can lose
@@ -688,14 +690,24 @@ static int choose_tiling(const TcParams& p, int sms) {
     const long long tm = (p.M + TC_BM - 1) / TC_BM, tn = (p.N + TW_BN - 1) / TW_BN;
     auto rounds = [](long long tiles, long long at_once) { return (tiles + at_once - 1) / at_once; };
     const long long wide = rounds(tm * tn, sms);
-    if (wide < 2) return 0;
+    if (wide < 2) return TILING_WIDE;
     double best = (double)wide * (TC_BM + TW_BN);
-    int form = 0;
+    int form = TILING_WIDE;
     const double mid = (double)rounds(tm * ((p.N + TM_BN - 1) / TM_BN), sms) * (TC_BM + TM_BN);
-    if (mid < best) { best = mid; form = 1; }
+    if (mid < best) { best = mid; form = TILING_MID; }
     const double pair = (double)rounds((long long)((p.M + 2 * TC_BM - 1) / (2 * TC_BM)) * tn, sms / 2) * (TC_BM + TW_BN) * (p.K < 2048 ? 0.95 : 0.9);
-    if (pair < best && (p.K >= 2048 || (p.mode != 4 && p.M >= 1024))) form = 2;
+    if (pair < best && (p.K >= 2048 || (p.mode != 4 && p.M >= 1024))) form = TILING_PAIR;
     return form;
+}
+
+// Of any product: TILING_SINGLE (128 x 128, a CTA each) below 256 columns; TILING_NARROW (persistent, 128 x 128) where even those give no
+// CTA a second tile: twice the CTAs at work.  (Where CTAs would take two of them in a row, the wider tile is faster: q/k/v
+// of 2,048 tokens 22.5 against 25.3 us.)
+static int tiling_of(const TcParams& p, int sms) {
+    if (!g_tc_wide || p.N < TW_BN) return TILING_SINGLE;
+    if (g_tc_wide != 1) return g_tc_wide == 2 ? TILING_PAIR : (g_tc_wide == 4 ? TILING_MID : TILING_WIDE);
+    if ((long long)((p.M + TC_BM - 1) / TC_BM) * ((p.N + TN_BN - 1) / TN_BN) <= sms) return TILING_NARROW;
+    return p.tile_expert == nullptr ? choose_tiling(p, sms) : TILING_WIDE;
 }
 
 // w_stack: matrices in the stack w [w_stack][N, K] (the grouped form; 1: the plain product).
@@ -717,12 +729,8 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
         configured = true;
     }
     const int tiles_m = (p.M + TC_BM - 1) / TC_BM;
-    const bool wide = g_tc_wide && p.N >= TW_BN;
-    // 128 x 128 tiles where even those give no CTA a second tile: twice the CTAs at work.  (Where CTAs would take two
-    // of them in a row, the wider tile is faster: q/k/v of 2,048 tokens 22.5 against 25.3 us.)
-    const bool narrow = wide && g_tc_wide == 1 && (long long)tiles_m * ((p.N + TN_BN - 1) / TN_BN) <= sms;
-    const int tiling = wide && !narrow && g_tc_wide == 1 && p.tile_expert == nullptr ? choose_tiling(p, sms) : 0;
-    const bool pair = wide && (g_tc_wide == 2 || tiling == 2), mid = wide && (g_tc_wide == 4 || tiling == 1);
+    const int tiling = tiling_of(p, sms);
+    const bool wide = tiling != TILING_SINGLE, narrow = tiling == TILING_NARROW, pair = tiling == TILING_PAIR, mid = tiling == TILING_MID;
     const bool pdl = g_pdl != 0 || p.M >= PDL_MIN_ROWS;
     CUtensorMap mx, mw;
     if (pair) {
@@ -777,6 +785,15 @@ using namespace fd;
 extern "C" int fd_gemm_tc_set_wide(int on) {
     g_tc_wide = on < 0 ? 0 : (on > 4 ? 4 : on);
     return 0;
+}
+
+extern "C" int fd_sm_count();
+
+// The tiling that fd_gemm_tc takes for these sizes (TILING_WIDE ..), for tests.
+extern "C" int fd_gemm_tc_tiling(int M, int N, int K, int mode) {
+    TcParams p = {};
+    p.M = M; p.N = N; p.K = K; p.mode = mode;
+    return tiling_of(p, fd_sm_count());
 }
 
 // 1 if the tensor-core product takes these sizes (K a multiple of 8, enough rows to be worth a

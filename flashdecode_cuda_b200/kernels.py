@@ -91,6 +91,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "fd_gemv_splits": [I, I, I, I, I],
         "fd_gemv": [P, P, P, I, P, I, I, I, I, I, P, c_ulonglong, P, I, I, P],
         "fd_gemm_f32_set_form": [I],
+        "fd_gemm_tc_tiling": [I, I, I, I],
         "fd_gemm_simt": [P, P, P, P, I, I, I, I, I, I, P],
         "fd_attn_simt_qt": [I],
         "fd_attn_decode_group": [I, I, I],
@@ -742,6 +743,12 @@ def gemm_f32_set_form(form: int) -> None:
     """The tiling of float32 products of more than 16 rows: 0 by the kernel's rule, 1..6 one of the six (tests and
     measurements; all give the same bits)."""
     _check(lib().fd_gemm_f32_set_form(int(form)))
+
+
+def gemm_tc_tiling(M: int, N: int, K: int, qkv: bool = False) -> str:
+    """The tiling that ``gemm_tc`` (``qkv``: ``gemm_tc_qkv_rope``) takes for these sizes: "wide", "mid", "pair", "narrow" or "single"
+    (tests)."""
+    return ("wide", "mid", "pair", "narrow", "single")[lib().fd_gemm_tc_tiling(M, N, K, 4 if qkv else 1)]
 
 
 def attention_decode_heads(n_q: int, n_kv: int, head_dim: int, v_dim: int) -> int:

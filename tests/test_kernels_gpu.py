@@ -279,6 +279,25 @@ def tc_tiling(request):
     K.gemm_tc_set_wide(TC_DEFAULT_TILING)
 
 
+def test_gemm_tcgen05_rule_reaches_every_tiling():
+    """The default rule at the layer sizes of the presets, and the results of the tilings that it chooses there by rounds."""
+    reached = {}
+    for M, N, K_, qkv, want in ((2048, 17920, 1536, False, "pair"), (384, 17920, 1536, False, "mid"), (2048, 2048, 1536, True, "wide"),
+                                (300, 2048, 1536, True, "narrow"), (2048, 4608, 3584, True, "pair"), (384, 37888, 3584, False, "wide"),
+                                (1200, 27648, 5120, False, "pair"), (300, 200, 64, False, "single")):
+        assert K.gemm_tc_tiling(M, N, K_, qkv) == want, (M, N, K_)
+        reached[want] = (M, N, K_)
+    assert len(reached) == 5
+    for M, N, K_ in ((384, 17920, 264), (1030, 9000, 264), (700, 20000, 2056)):
+        assert K.gemm_tc_tiling(M, N, K_) in ("mid", "pair")
+        g = torch.Generator(device=DEV).manual_seed(M)
+        x, w = (torch.randn(n, K_, device=DEV, generator=g).bfloat16() for n in (M, N))
+        out, st = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV), status()
+        K.gemm_tc(x, w, None, out, status=st)
+        # a bfloat16 rounding of the result, 2^-9 of itself
+        assert rel(out, x.double() @ w.double().T) < 5e-3 and int(st.item()) == 0
+
+
 @pytest.mark.parametrize("M,N,K_", [(128, 128, 64), (128, 256, 256), (130, 200, 72), (70, 333, 1536), (2048, 2048, 1536),
                                     (300, 1536, 8960), (17, 16, 8), (1000, 384, 136), (4096, 4864, 256), (129, 257, 64)])
 def test_gemm_tcgen05(M, N, K_, tc_tiling):
