@@ -35,7 +35,9 @@ struct AttnParams {
     int QT, n_splits, split_len, window;
     int chunk;                 // > 0: a query at position i sees key j <= i only if i / chunk == j / chunk
     float scale;
-    // The CUDA-core kernel and the extended prompt kernel only (the launchers of the others are not called when any of these is set):
+    // Options that not every kernel has; a launcher is not called with one that its kernel lacks.  The CUDA-core kernel and the extended
+    // mma.sync prompt kernel have all of them; the tcgen05 prompt kernel and the tensor-core decode kernel softcap and sink; the decode
+    // kernel of attention_rows.cu all of them in bfloat16, none in float32:
     float softcap;             // > 0: score <- softcap * tanh(score / softcap) after scaling
     int keep_first;            // with a window: keys at positions below this stay visible however far back they lie
     const float* sink;         // [n_q] or null: exp(sink[h]) is one more term of head h's softmax denominator

@@ -466,7 +466,9 @@ int launch_attn_f32(const AttnParams& p, int n_rows, int max_q_len, cudaStream_t
 }
 
 // bfloat16 decode steps with the options that the tensor-core kernel has not: kept first keys, and weights applied to every value
-// head (2 or 4 of them) for the caller to mix.  Returns 1 if it does not take the sizes.
+// head for the caller to mix.  The number of value heads and the most query heads of a group are the kernel's register tile (value heads x
+// query heads x 4 sums a thread, 64 at most), so it is built for 2 and 4 value heads under groups of up to 4, which
+// the sizes at hand have (33 us in the general kernel, 13 here), and returns 1 for others: three or eight value heads, larger groups.
 int launch_attn_rows_ext(const AttnParams& p, int n_rows, cudaStream_t stream) {
     if (p.d != p.dv || p.v_ld != p.dv || p.kv_div != 1 || (uintptr_t)p.out % 16 != 0 || p.out_ld % 4 != 0) return 1;
     if (p.v_rep > 1 && p.v_rep != p.n_kv_pool) return 1;

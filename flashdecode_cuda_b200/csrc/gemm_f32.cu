@@ -184,8 +184,10 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
 // did); a thread of the others runs the chains of TN rows of W with TM rows of A.  Three bounds: HBM for the wide
 // matrices; for those with few rows the chain itself, K dependent fmaf of four cycles each; and what shared memory delivers,
 // 128 bytes a cycle to all lanes together whether they read the same value or not, which larger TM x TN need less of - but
-// then fewer warps are there to hide its latency.  The sizes below are the fastest of those tried.  Measured (M rows; us, and
-// before with the loads of one step ahead in registers): M 8: 1,536 x 8,960 43 (81), 17,920 x 1,536 31 (73), the head of 151,936
+// then fewer warps are there to hide its latency.  The sizes below are the fastest of those tried at the widths of
+// Qwen2.5-1.5B (the tiles of 12 rows: 128 CTAs for its 1,536 columns); at 8 to 37,888 columns and 64 to 8,960 k none was slower than the
+// register-fed kernels before them.  Measured (M rows; us, and before with the loads of
+// one step ahead in registers): M 8: 1,536 x 8,960 43 (81), 17,920 x 1,536 31 (73), the head of 151,936
 // rows 0.24 ms; M 1: 33 and 23; M 16: 60 and 39.  V16: rows are 16-byte aligned.  G: float4s of k read ahead of the multiplications.
 template <int NT, int KT, int S, int MP, int TM, int TN, int G, bool V16>
 __global__ void __launch_bounds__(256)
