@@ -24,6 +24,7 @@ cache's, the step's and the workspace's addresses are taken anew for every step.
 from __future__ import annotations
 
 import ctypes
+import weakref
 from ctypes import c_double, c_longlong, c_void_p
 from typing import List, Optional
 
@@ -70,18 +71,18 @@ class DensePrompts:
         return native if native.layers is not None else None
 
     def __init__(self, model):
-        self.model = model
+        self._model = weakref.ref(model)        # (the model holds this object: a dropped model's weights go at once)
         self._derive()
 
     def _derive(self) -> None:
         """The launches' constants from the model's parts as they are now; ``layers`` None: not a model of this kind."""
         self.derived_at = Part.changes                              # before anything is read
-        self.blocks = list(self.model.blocks)
+        self.blocks = list(self._model().blocks)
         self.tensors, self.where, self.memory = [], [], []
         self.layers = self._layers()
 
     def _layers(self):
-        model = self.model
+        model = self._model()
         if model.dtype != torch.bfloat16 or model.blueprint.lanes != 1 or model.stream_ops:
             return None
         blocks = [self.blocks[run.layer] for run in model.schedule]
@@ -140,7 +141,7 @@ class DensePrompts:
         T = ctx.T
         if linear.PROMPT_GEMM != "auto" or ctx.max_q_len < 2 or T <= linear.GEMV_MAX_ROWS:
             return False
-        if self.derived_at != Part.changes or self.blocks != self.model.blocks:
+        if self.derived_at != Part.changes or self.blocks != self._model().blocks:
             self._derive()
         if self.layers is None or [kind.forward for kind in KINDS] != FORWARDS:
             return False

@@ -213,6 +213,34 @@ def test_native_prompt_steps_see_what_became_of_the_parts(engines, monkeypatch):
     m.check_status()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_a_dropped_model_goes_at_once(dtype):
+    """A model that was bound and stepped holds no reference to itself: its weights' memory is free when the last name goes,
+    without the garbage collector."""
+    import gc
+    import weakref
+    from flashdecode_cuda_b200.config import config_from_dict
+    from flashdecode_cuda_b200.engine import Model, random_weights
+    from flashdecode_cuda_b200.measure import PartTimer
+    dt = {"float32": torch.float32, "bfloat16": torch.bfloat16}[dtype]
+    gc.collect()
+    gc.disable()
+    try:
+        m = Model.from_config(config_from_dict(dict(TINY["D"])), dt, "cuda")
+        m.bind(random_weights(m, 3, dt, device="cuda"))
+        cache = m.new_cache(max_tokens=512, block_size=16)
+        slot = cache.admit()
+        m.step(cache, [slot], [list(range(1, 40))], "last")
+        with PartTimer(m):
+            m.step(cache, [slot], [list(range(1, 40))], "last")
+        m.step(cache, [slot], [list(range(1, 30))], "last")
+        seen, weight = weakref.ref(m), weakref.ref(m.blocks[0].mixer.w_qkv)
+        del m, cache
+        assert seen() is None and weight() is None
+    finally:
+        gc.enable()
+
+
 @pytest.mark.parametrize("name", ["D", "E"])
 def test_asking_l2_for_what_comes_next_changes_no_bit(engines, folders, name, monkeypatch):
     """Decode steps hand ``ctx.upcoming`` (the weights the step streams next) to their kernels, which ask L2
