@@ -408,9 +408,9 @@ class Model:
             embedded.copy_(resid)
         delta = None
         entries = self.schedule
-        if self.native is not None and self.trace is None and self.native.takes(ctx):
+        if self.native is not None and self.trace is None and self.native.takes(self, ctx):
             delta, entries = self.native.run(ctx, resid), []
-            if self.native.moved():                  # a step's launches may be repeated: they start from the embedding and append
+            if self.native.moved(self):                  # a step's launches may be repeated: they start from the embedding and append
                 self.embedding.forward(ctx, resid)   # the same keys and values
                 delta, entries = None, self.schedule
         caches = self._layer_caches(ctx.cache) if entries else []

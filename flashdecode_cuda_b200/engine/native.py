@@ -24,7 +24,6 @@ cache's, the step's and the workspace's addresses are taken anew for every step.
 from __future__ import annotations
 
 import ctypes
-import weakref
 from ctypes import c_double, c_longlong, c_void_p
 from typing import List, Optional
 
@@ -67,22 +66,27 @@ class DensePrompts:
 
     @staticmethod
     def of(model) -> Optional["DensePrompts"]:
-        native = DensePrompts(model)
+        native = DensePrompts()
+        native._derive(model)
         return native if native.layers is not None else None
 
-    def __init__(self, model):
-        self._model = weakref.ref(model)        # (the model holds this object: a dropped model's weights go at once)
-        self._derive()
+    def __init__(self):
+        # (no reference to the model, which holds this object: a dropped model's weights go at once)
+        self.derived_at, self.blocks, self.schedule, self.layers = -1, [], None, None
+        self.tensors, self.where, self.memory = [], [], []
 
-    def _derive(self) -> None:
+    def __reduce__(self):
+        """A copied model's is derived from its own parts, at its first step."""
+        return DensePrompts, ()
+
+    def _derive(self, model) -> None:
         """The launches' constants from the model's parts as they are now; ``layers`` None: not a model of this kind."""
         self.derived_at = Part.changes                              # before anything is read
-        self.blocks = list(self._model().blocks)
+        self.blocks, self.schedule = list(model.blocks), model.schedule
         self.tensors, self.where, self.memory = [], [], []
-        self.layers = self._layers()
+        self.layers = self._layers(model)
 
-    def _layers(self):
-        model = self._model()
+    def _layers(self, model):
         if model.dtype != torch.bfloat16 or model.blueprint.lanes != 1 or model.stream_ops:
             return None
         blocks = [self.blocks[run.layer] for run in model.schedule]
@@ -136,13 +140,13 @@ class DensePrompts:
         self.addresses = [ctypes.addressof(layers[i]) for i in range(self.n)]
         return layers
 
-    def takes(self, ctx) -> bool:
+    def takes(self, model, ctx) -> bool:
         """Whether the parts would run this step on the kernels that the native calls launch."""
         T = ctx.T
         if linear.PROMPT_GEMM != "auto" or ctx.max_q_len < 2 or T <= linear.GEMV_MAX_ROWS:
             return False
-        if self.derived_at != Part.changes or self.blocks != self._model().blocks:
-            self._derive()
+        if self.derived_at != Part.changes or self.blocks != model.blocks or self.schedule is not model.schedule:
+            self._derive(model)
         if self.layers is None or [kind.forward for kind in KINDS] != FORWARDS:
             return False
         H = self.hidden
@@ -150,11 +154,11 @@ class DensePrompts:
             return all(linear.stream_gemm(T, n, k) for n, k in ((self.qkv, H), (H, self.n_q * self.d), (2 * self.inter, H), (H, self.inter)))
         return linear.fused_prompt_gemm(T, self.qkv, H) and linear.fused_prompt_gemm(T, 2 * self.inter, H)
 
-    def moved(self) -> bool:
+    def moved(self, model) -> bool:
         """Whether a weight's tensor has other memory than the step that was just launched used; then everything is derived anew."""
         if list(map(_address, self.tensors)) == self.where:
             return False
-        self._derive()
+        self._derive(model)
         return True
 
     def run(self, ctx, resid: torch.Tensor) -> torch.Tensor:

@@ -180,7 +180,7 @@ def test_native_prompt_steps_see_what_became_of_the_parts(engines, monkeypatch):
             m.native = native
     first = logits()
     derived = []
-    monkeypatch.setattr(native, "_derive", lambda f=native._derive: (derived.append(1), f())[1])
+    monkeypatch.setattr(native, "_derive", lambda model, f=native._derive: (derived.append(1), f(model))[1])
     assert all(torch.equal(a, b) for a, b in zip(logits(), first)) and not derived
     called = []
     for part in (block, block.norm1, block.norm2, block.mixer, block.feed_forward):
@@ -211,6 +211,35 @@ def test_native_prompt_steps_see_what_became_of_the_parts(engines, monkeypatch):
     before = len(derived)
     assert all(torch.equal(a, b) for a, b in zip(logits(), first)) and len(derived) <= before + 1
     m.check_status()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_copied_models_run_on_their_own_parts(dtype):
+    """copy.deepcopy gives a model whose prompt steps use its own weights; copy.copy one that sees what is put in its place, whichever
+    of the two steps, and outlives the original."""
+    import copy
+    from flashdecode_cuda_b200.config import config_from_dict
+    from flashdecode_cuda_b200.engine import Model, random_weights
+    dt = {"float32": torch.float32, "bfloat16": torch.bfloat16}[dtype]
+    m = Model.from_config(config_from_dict(dict(TINY["D"])), dt, "cuda")
+    m.bind(random_weights(m, 3, dt, device="cuda"))
+
+    def logits(model, n):
+        cache = model.new_cache(max_tokens=256, block_size=16)
+        return model.step(cache, [cache.admit()], [list(range(1, n))], "last").clone()
+    copies = [copy.deepcopy(m) for _ in range(2)]                   # (before a first step: events are not copied)
+    for n, deep in zip((30, 150), copies):
+        first = logits(m, n)
+        flat = copy.copy(m)
+        assert torch.equal(logits(deep, n), first) and torch.equal(logits(flat, n), first)
+        deep.blocks[0].mixer.w_o = torch.zeros_like(deep.blocks[0].mixer.w_o)
+        flat.blocks = list(deep.blocks)
+        other = logits(deep, n)
+        assert not torch.equal(other, first)
+        assert torch.equal(logits(m, n), first) and torch.equal(logits(flat, n), other) and torch.equal(logits(m, n), first)
+    kept = copy.copy(m)
+    del m
+    assert torch.equal(logits(kept, n), first)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
