@@ -96,8 +96,9 @@ attn_rows_decode_kernel(const AttnParams p) {
     float* a_s = l_s + GDEC;
     __shared__ int row_s[FT], vrow_s[FT];
     // pieces of a group of more than GDEC heads are as equal as whole heads allow: the last one may have fewer
-    const int split = blockIdx.x, kvh = blockIdx.y / p.kv_div, per = (p.G + p.kv_div - 1) / p.kv_div, b = blockIdx.z;
-    const int g0 = (blockIdx.y - kvh * p.kv_div) * per, G = min(per, p.G - g0), head = kvh * p.G + g0;
+    // (heads whose weights are mixed are not cut)
+    const int split = blockIdx.x, kvh = VR > 1 ? blockIdx.y : blockIdx.y / p.kv_div, per = VR > 1 ? p.G : (p.G + p.kv_div - 1) / p.kv_div, b = blockIdx.z;
+    const int g0 = VR > 1 ? 0 : (blockIdx.y - kvh * p.kv_div) * per, G = VR > 1 ? p.G : min(per, p.G - g0), head = kvh * p.G + g0;
     const int slot = p.row_slot[b];
     if (slot < 0 || p.row_q_len[b] != 1) return;
     const int tok = p.row_q_start[b], pos = p.row_ctx_len[b];

@@ -359,7 +359,8 @@ attn_tile_kernel(const AttnParams p) {
 // the block's four warps share the splits, or the dims of wide heads (d a multiple of 4).
 constexpr int COMBINE_MAX_SPLITS = 512;
 
-template <typename T>
+// ROWS: the partial sums of rows that bring one token beside longer ones (ROWS_SINGLE), by row; else by token.
+template <typename T, bool ROWS = false>
 __global__ void attn_combine_kernel(const float* __restrict__ part_m, const float* __restrict__ part_l,
                                     const float* __restrict__ part_acc, T* __restrict__ out,
                                     const int* __restrict__ tok_row, const int* __restrict__ row_slot,
@@ -370,10 +371,9 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_m, const floa
     __shared__ float red[33];
     pdl_launch_dependents();
     pdl_wait();
-    // row_q_len given: the partial sums of rows (ROWS_SINGLE), of which those that bring one token have any
-    const int h = blockIdx.x, tok = row_q_len != nullptr ? row_q_start[blockIdx.y] : blockIdx.y;
+    const int h = blockIdx.x, tok = ROWS ? row_q_start[blockIdx.y] : blockIdx.y;
     const size_t row = (size_t)blockIdx.y * n_q + h;
-    if (row_q_len != nullptr && (row_slot[blockIdx.y] < 0 || row_q_len[blockIdx.y] != 1)) return;
+    if (ROWS && (row_slot[blockIdx.y] < 0 || row_q_len[blockIdx.y] != 1)) return;
     T* o = out + (size_t)tok * out_ld + (size_t)h * d;
     float* of = reinterpret_cast<float*>(out) + (size_t)tok * out_ld + (size_t)h * d;       // the same row when the output is float whatever T is
     if (row_slot[tok_row[tok]] < 0) {
@@ -606,7 +606,7 @@ static int attention_impl(const void* q, const void* k_pool, const void* v_pool,
         if (use_mma != 0) rc = launch_attn_f32(one, n_rows, 1, stream);
         if (rc == 1) rc = launch_attn<float>(one, n_rows, 1, stream);
         if (rc == 0 && one.n_splits > 1)
-            rc = launch("attention_combine", attn_combine_kernel<float>, dim3(n_q, n_rows), dim3(128), 0, stream, dim3(1, 1, 1),
+            rc = launch("attention_combine", attn_combine_kernel<float, true>, dim3(n_q, n_rows), dim3(128), 0, stream, dim3(1, 1, 1),
                         (const float*)one.part_m, (const float*)one.part_l, (const float*)one.part_acc, (float*)out, tok_row,
                         row_slot, n_q, dv, one.n_splits, (const float*)nullptr, 1, 0, p.out_ld, out_scale, row_q_start, row_q_len);
         if (rc != 0) return rc;
