@@ -5,6 +5,7 @@
 // the GPU needs for prompts of up to some hundred tokens (19 tokens: 1.7 ms).  The kernels and their order are those of the
 // parts (parts/attention.py, mlp.py, norm.py); which step may come this way is decided in engine/native.py.
 #include "common.cuh"
+#include "dense_step.cuh"
 
 extern "C" {
 int fd_gemm_stream(const void* x, const void* w, const void* bias, int bias_f32, void* out, int mode, int M, int N, int K,
@@ -27,15 +28,6 @@ int fd_attention(const void* q, const void* k_pool, const void* v_pool, void* ou
                  float* scratch, int* counters, int* status, const void* prefetch, unsigned long long prefetch_bytes,
                  int out_ld, float out_scale, float* prompt_scratch, int kv_len, cudaStream_t stream);
 }
-
-// One schedule entry; weights and sizes, fixed when the model is bound (engine/native.py has the same order).
-struct FdDenseLayer {
-    const void *norm1, *norm2, *w_qkv, *b_qkv, *w_o, *w_gate_up, *w_down;
-    long long norm1_f32, norm2_f32, bias_f32;      // whether these vectors are float32
-    long long hidden, inter, n_q, n_kv, d, window, chunk, write_kv;
-    long long group, index, position;              // cache group, layer in it, rotation tables
-    double eps1, eps2, scale;
-};
 
 // A step: its buffers and index arrays; the cache's pools by group (a layer's pool is `stride` bytes after the one before) and
 // the rotation tables by position.

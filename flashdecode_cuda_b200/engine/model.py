@@ -408,10 +408,14 @@ class Model:
             embedded.copy_(resid)
         delta = None
         entries = self.schedule
-        if self.native is not None and self.trace is None and self.native.takes(self, ctx):
-            delta, entries = self.native.run(ctx, resid), []
-            if self.native.moved(self):                  # a step's launches may be repeated: they start from the embedding and append
-                self.embedding.forward(ctx, resid)   # the same keys and values
+        if self.native is not None and self.trace is None:
+            if self.native.takes(self, ctx):
+                delta, entries = self.native.run(ctx, resid), []
+            elif self.native.decodes(self, ctx):
+                self.native.decode(ctx, resid, self.head.first_weights() if ctx.n_want else None)
+                entries = []
+            if not entries and self.native.moved(self):      # a step's launches may be repeated: they start from the embedding and
+                self.embedding.forward(ctx, resid)           # append the same keys and values
                 delta, entries = None, self.schedule
         caches = self._layer_caches(ctx.cache) if entries else []
         for i, run in enumerate(entries):

@@ -1,4 +1,4 @@
-"""Prompt steps of dense models, launched from native code (``csrc/dense_step.cu``).
+"""Prompt steps and small decode steps of dense models, launched from native code (``csrc/dense_step.cu``, ``csrc/dense_decode.cu``).
 
 A prompt step runs some seven kernels per layer; launched one by one through
 the parts they cost the host about 12 us each (2.4 ms per step at 28 layers,
@@ -7,7 +7,8 @@ pre-norm block, RMS norms, grouped-query attention, SiLU-gated feed-forward,
 nothing between the layers - the same launches are made by ``fd_dense_layers``
 (up to 128 tokens: the whole step in one call) or, layer by layer, by
 ``fd_dense_mixer`` and ``fd_dense_gate_up`` around the library products of the
-output and down projections.  Everything else, and every step that this module
+output and down projections.  A decode step of up to 16 sequences is one kernel
+for all layers (``fd_dense_decode``) where it takes the sizes.  Everything else, and every step that this module
 does not take, goes through the parts' ``forward``.
 
 A part whose ``forward`` was wrapped or replaced, on the object or on its class,
@@ -60,9 +61,18 @@ class _Step(ctypes.Structure):
                 + [(n, c_void_p * MAX_POSITIONS) for n in ("cos", "sin")] + [("table_len", c_longlong * MAX_POSITIONS)])
 
 
+class _Decode(ctypes.Structure):
+    _fields_ = ([(n, c_void_p) for n in ("resid", "tok_pos", "row_slot", "row_ctx_len", "status", "stream", "exchange")]
+                + [(n, c_longlong) for n in ("M", "num_blocks", "block_size")]
+                + [(n, c_void_p * MAX_GROUPS) for n in ("k_base", "v_base", "table")]
+                + [(n, c_longlong * MAX_GROUPS) for n in ("k_stride", "v_stride", "max_blocks")]
+                + [(n, c_void_p * MAX_POSITIONS) for n in ("cos", "sin")] + [("table_len", c_longlong * MAX_POSITIONS)]
+                + [("next", c_void_p), ("next_bytes", c_longlong)])
+
+
 class DensePrompts:
-    """The native form of a bound model's prompt steps; ``DensePrompts.of(model)`` is None for a model that is not of
-    that kind."""
+    """The native form of a bound model's prompt steps and small decode steps; ``DensePrompts.of(model)`` is None for a
+    model that is not of that kind."""
 
     @staticmethod
     def of(model) -> Optional["DensePrompts"]:
@@ -138,21 +148,64 @@ class DensePrompts:
             L.eps1, L.eps2, L.scale = b.norm1.eps, b.norm2.eps, m.scale
             self.products.append((m.w_o.t(), f.w_down.t()))
         self.addresses = [ctypes.addressof(layers[i]) for i in range(self.n)]
+        self.exchange_words = {}                                    # of a decode step, by its rows; 0: not taken
+        self.all_write = all(writes for _, _, writes, _ in model._layout[2])
         return layers
+
+    def _current(self, model) -> bool:
+        """Whether the model is of the kind, as its parts are now."""
+        if self.derived_at != Part.changes or self.blocks != model.blocks or self.schedule is not model.schedule:
+            self._derive(model)
+        return self.layers is not None and [kind.forward for kind in KINDS] == FORWARDS
 
     def takes(self, model, ctx) -> bool:
         """Whether the parts would run this step on the kernels that the native calls launch."""
         T = ctx.T
         if linear.PROMPT_GEMM != "auto" or ctx.max_q_len < 2 or T <= linear.GEMV_MAX_ROWS:
             return False
-        if self.derived_at != Part.changes or self.blocks != model.blocks or self.schedule is not model.schedule:
-            self._derive(model)
-        if self.layers is None or [kind.forward for kind in KINDS] != FORWARDS:
+        if not self._current(model):
             return False
         H = self.hidden
         if T <= linear.STREAM_MAX_ROWS:
             return all(linear.stream_gemm(T, n, k) for n, k in ((self.qkv, H), (H, self.n_q * self.d), (2 * self.inter, H), (H, self.inter)))
         return linear.fused_prompt_gemm(T, self.qkv, H) and linear.fused_prompt_gemm(T, 2 * self.inter, H)
+
+    def decodes(self, model, ctx) -> bool:
+        """Whether the step is one token each of so few sequences that one kernel runs all of its layers
+        (``csrc/dense_decode.cu``); every layer has to write the keys that it reads."""
+        T = ctx.T
+        if ctx.max_q_len != 1 or T > linear.GEMV_MAX_ROWS or T != ctx.n_rows or not self._current(model) or not self.all_write:
+            return False
+        if any(g.table.shape[1] * ctx.cache.block_size ** 2 >= 1 << 32 for g in ctx.cache.groups):
+            return False                                            # (the kernel divides positions by the block size in 32 bits)
+        words = self.exchange_words.get(T)
+        if words is None:
+            words = self.exchange_words[T] = K.dense_decode_words(T, self.hidden, self.inter, self.n_q, self.n_kv, self.d)
+        return words > 0
+
+    def decode(self, ctx, resid: torch.Tensor, upcoming: Optional[torch.Tensor]) -> None:
+        """Every schedule entry of the step; ``resid`` is the finished stream then.  ``upcoming``: what the step streams next."""
+        s, cache = _Decode(), ctx.cache
+        s.resid, s.tok_pos, s.row_slot = resid.data_ptr(), ctx.tok_pos.data_ptr(), ctx.row_slot.data_ptr()
+        s.row_ctx_len, s.status, s.stream = ctx.row_ctx_len.data_ptr(), ctx.rt.status.data_ptr(), K._stream()
+        # zeroed when it is made; for these rows only, so that every word is written in every step
+        s.exchange = ctx.ws.get(f"dense_decode.{ctx.T}", (self.exchange_words[ctx.T],), torch.int64).data_ptr()
+        s.M = ctx.T
+        if upcoming is not None:
+            s.next = upcoming.data_ptr()
+            s.next_bytes = min(upcoming.numel() * upcoming.element_size(), linear.UPCOMING_BYTES)
+        self._cache_args(s, cache)
+        K._check(K.lib().fd_dense_decode(ctypes.addressof(s), self.addresses[0], self.n))
+
+    def _cache_args(self, s, cache) -> None:
+        """The pools, tables and rotation tables of a step."""
+        s.num_blocks, s.block_size = cache.num_blocks, cache.block_size
+        for i, g in enumerate(cache.groups):
+            s.k_base[i], s.v_base[i], s.table[i] = g.keys.data_ptr(), g.values.data_ptr(), g.table.data_ptr()
+            s.k_stride[i], s.v_stride[i] = 2 * g.keys.stride(0), 2 * g.values.stride(0)
+            s.max_blocks[i] = g.table.shape[1]
+        for i, p in enumerate(self.positions):
+            s.cos[i], s.sin[i], s.table_len[i] = p.cos.data_ptr(), p.sin.data_ptr(), p.cos.shape[0]
 
     def moved(self, model) -> bool:
         """Whether a weight's tensor has other memory than the step that was just launched used; then everything is derived anew."""
@@ -177,13 +230,8 @@ class DensePrompts:
         s.T, s.n_rows, s.max_q_len, s.kv_len = T, ctx.n_rows, ctx.max_q_len, ctx.kv_len_bound
         scratch = prompt_scratch(ctx, self.n_q, self.d)
         s.attn_scratch = None if scratch is None else scratch.data_ptr()
-        s.num_blocks, s.block_size, s.streams = cache.num_blocks, cache.block_size, T <= linear.STREAM_MAX_ROWS
-        for i, g in enumerate(cache.groups):
-            s.k_base[i], s.v_base[i], s.table[i] = g.keys.data_ptr(), g.values.data_ptr(), g.table.data_ptr()
-            s.k_stride[i], s.v_stride[i] = 2 * g.keys.stride(0), 2 * g.values.stride(0)
-            s.max_blocks[i] = g.table.shape[1]
-        for i, p in enumerate(self.positions):
-            s.cos[i], s.sin[i], s.table_len[i] = p.cos.data_ptr(), p.sin.data_ptr(), p.cos.shape[0]
+        s.streams = T <= linear.STREAM_MAX_ROWS
+        self._cache_args(s, cache)
         L, step = K.lib(), ctypes.addressof(s)
         if s.streams:
             K._check(L.fd_dense_layers(step, self.addresses[0], self.n))

@@ -151,6 +151,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "fd_dense_mixer": [P, P, P],
         "fd_dense_gate_up": [P, P],
         "fd_dense_layers": [P, P, I],
+        "fd_dense_decode": [P, P, I],
         "fd_sample": [P, I, I, P, P, P, c_ulonglong, P, P, P, P],
         "fd_copy_h2d_async": [P, P, LL, P],
         "fd_copy_d2h_sync": [P, P, LL, P],
@@ -162,6 +163,8 @@ def _declare(L: ctypes.CDLL) -> None:
     L.fd_attn_scratch_floats.argtypes = [I, I, I, I]
     L.fd_attn_prompt_scratch_floats.argtypes = [I] * 8
     L.fd_attn_prompt_scratch_floats.restype = LL
+    L.fd_dense_decode_plan.argtypes = [I] * 8 + [P]
+    L.fd_dense_decode_plan.restype = LL
     L.fd_launch_count.restype = c_ulonglong
     L.fd_launch_count.argtypes = []
     L.fd_attn_scratch_floats.restype = LL
@@ -767,6 +770,19 @@ def attention_prompt_scratch_floats(n_tokens: int, n_q: int, head_dim: int, n_ro
     """Floats of scratch with which ``attention`` may cut a bfloat16 prompt step's keys into parts; 0: it would not.  Without
     ``window`` and ``chunk``: enough for any."""
     return int(lib().fd_attn_prompt_scratch_floats(n_tokens, n_q, head_dim, n_rows, max_q_len, kv_len, window, chunk))
+
+
+def dense_decode_words(n_rows: int, hidden: int, inter: int, n_q: int, n_kv: int, head_dim: int, sm_count: int = 0,
+                       smem: int = 0, info: Optional[list] = None) -> int:
+    """64-bit words of exchange memory (zeroed once) that the one-kernel decode step of a dense model takes for ``n_rows`` sequences;
+    0: it does not take these sizes.  ``sm_count`` and ``smem``: another device than the current one.  ``info``, a list, is
+    given [slices of the down projection's k, row tiles per group, ring stages, bytes of shared memory, most gate/up
+    tiles of a CTA]."""
+    out = (c_longlong * 5)()
+    n = int(lib().fd_dense_decode_plan(n_rows, hidden, inter, n_q, n_kv, head_dim, sm_count, smem, ctypes.addressof(out)))
+    if info is not None:
+        info[:] = list(out)
+    return n
 
 
 _attn_counters = {}      # per device: zeroed ints the decode kernel counts arriving splits in (kept alive for good)

@@ -134,3 +134,28 @@ def test_a_layer_is_a_block_name_and_named_parts():
         LayerSpec("prenorm", norm1="not a spec")
     with pytest.raises(AttributeError):
         by_name.norm3
+
+
+@pytest.mark.parametrize("sizes", [(1536, 8960, 12, 2, 128), (3584, 18944, 28, 4, 128), (5120, 13824, 40, 8, 128), (64, 64, 1, 1, 64),
+                                   (192, 320, 3, 1, 128), (4096, 4160, 32, 32, 128)])
+def test_decode_steps_of_one_kernel_are_dealt_out(sizes):
+    """The one-kernel decode step's plan (host code): within the grid and the shared memory, or not taken; sizes that the kernel cannot
+    tile are refused."""
+    from flashdecode_cuda_b200 import kernels as K
+    H, inter, n_q, n_kv, d = sizes
+    smem = 232448
+    for sms in (148, 132):
+        for M in range(1, 17):
+            info = []
+            words = K.dense_decode_words(M, H, inter, n_q, n_kv, d, sms, smem, info)
+            if words == 0:
+                assert M > 8 and H > 3000       # the rows of x leave no room for a ring
+                continue
+            slices, rows, ring, used, most = info
+            stages, blocks = divmod(ring, 100)
+            assert used <= smem and stages >= 4 and blocks in (12, 16)
+            assert -(-(H // 16) // rows) * slices <= sms and slices <= -(-(inter // 64) // blocks)
+            assert most * sms >= inter // 8 and most <= -(-(inter // 8) // sms)
+    for bad in ((H + 16, inter, n_q, n_kv, d), (H, inter + 32, n_q, n_kv, d), (H, inter, n_q, n_kv, 96), (H, inter, 9 * n_kv, n_kv, d)):
+        assert K.dense_decode_words(1, *bad, 148, smem) == 0
+    assert K.dense_decode_words(17, *sizes, 148, smem) == 0

@@ -157,6 +157,101 @@ def test_native_prompt_steps_change_no_bit(engines, name, block_size):
     assert len(taken) >= 6 and len(a) == len(b) and all(torch.equal(x, y) for x, y in zip(a, b))
 
 
+@pytest.mark.parametrize("n_seqs", [1, 2, 8, 9, 16])
+@pytest.mark.parametrize("name,block_size", [("D", 5), ("D", 64), ("E", 16), ("E", 24)])
+def test_decode_steps_in_one_kernel(engines, folders, name, block_size, n_seqs):
+    """Decode steps of up to 16 sequences, all layers in one kernel: contexts around the kernel's tiles of 16 keys and splits of 128
+    (and a window, and more than one split), rows of one and of two column tiles, blocks that do and do not hold whole
+    tiles, padding rows, against the plain implementation; the same bits when a step is made again; keys and values of the
+    new tokens as the parts leave them, to rounding."""
+    eng = engines[(name, "bfloat16")]
+    m = eng.model
+    lengths = [600, 1, 16, 128, 15, 127, 129, 17, 255, 256, 3, 383, 64, 31, 500, 2][:n_seqs]
+    reqs = prompts_for(m.vocab_size, [n + 2 for n in lengths], seed=90)
+    native, taken = m.native, []
+
+    def steps(on, pad=0):
+        cache = m.new_cache(batch_size=n_seqs, max_len=640, block_size=block_size)
+        slots = [cache.admit() for _ in reqs]
+        m.step(cache, slots, [r[:n] for r, n in zip(reqs, lengths)], None)
+        out = []
+        native.decode = lambda *a, f=type(native).decode: (taken.append(1), f(native, *a))[1]
+        m.native = native if on else None
+        try:
+            for j in range(2):
+                tokens = [[r[n + j]] for r, n in zip(reqs, lengths)]
+                cache.reserve([(s, 1) for s in slots])
+                cache.sync()
+                ctx = m.make_context(cache, slots, tokens, "all", pad_rows=pad)
+                out.append(m.forward(ctx)[:n_seqs].clone())
+                for s in slots:
+                    cache.advance(s, 1)
+        finally:
+            m.native = native
+            del native.decode
+        return out, [cache.gather(s, 0, layer_group) for s in slots for layer_group in range(1)]
+    (got, kv), (again, _), (parts, kv_parts) = steps(True), steps(True), steps(False)
+    assert len(taken) == 4
+    assert all(torch.equal(a, b) for a, b in zip(got, again))
+    if n_seqs < 16:
+        for pad in (1, 16 - n_seqs):
+            padded, _ = steps(True, pad=pad)
+            assert all(rel_err(a, b) < TOL["bfloat16"] for a, b in zip(padded, got))
+        assert len(taken) == 8
+    for i, (r, n) in enumerate(zip(reqs, lengths)):
+        want = oracle_logits(folders[name], r)
+        for j in range(2):
+            assert rel_err(got[j][i], want[n + j]) < TOL["bfloat16"], (n, j)
+    for a, b in zip(kv, kv_parts):
+        assert all(rel_err(x, y) < TOL["bfloat16"] for x, y in zip(a, b))
+    m.check_status()
+
+
+def test_decode_in_one_kernel_reports(engines):
+    """A wait that runs out (one CTA keeps its last words to itself), a missing block and a position beyond the rotation table set
+    their status bits and nothing else: the kernel returns, and the next step is right."""
+    from flashdecode_cuda_b200 import kernels as K
+    m = engines[("E", "bfloat16")].model
+    req = prompts_for(m.vocab_size, [41], seed=5)[0]
+    cache = m.new_cache(batch_size=1, max_len=64, block_size=16)
+    slot = cache.admit()
+    m.step(cache, [slot], [req[:40]], None)
+    cache.reserve([(slot, 1)])
+    cache.sync()
+
+    def step():
+        return m.forward(m.make_context(cache, [slot], [[req[40]]], "all")).clone()
+    first = step()
+    m.check_status()
+    try:
+        K.tc_test_hook(wait_ns=1_000_000, skip_last=True)
+        step()
+        with pytest.raises(RuntimeError, match="wait"):
+            m.check_status()
+    finally:
+        K.tc_test_hook()
+    assert torch.equal(step(), first)
+    for group, entry in ((0, -1), (1, cache.num_blocks)):
+        table = cache.groups[group].table
+        kept = table.clone()
+        table[slot, 1] = entry                   # of a block in the middle
+        step()
+        table.copy_(kept)
+        with pytest.raises(RuntimeError, match="block"):
+            m.check_status()
+    rope = m.blocks[0].mixer.position
+    kept = rope.cos
+    rope.cos = kept[:40]                         # position 40 is the first without an angle
+    try:
+        step()
+        with pytest.raises(RuntimeError, match="position"):
+            m.check_status()
+    finally:
+        rope.cos = kept
+    assert torch.equal(step(), first)
+    m.check_status()
+
+
 def test_native_prompt_steps_see_what_became_of_the_parts(engines, monkeypatch):
     """A forward wrapped on a part or on its class is called, and replaced weights are used, by prompt steps of every length (18
     tokens: one native call; 140: two per layer) as by the parts; steps that change nothing derive nothing anew."""
