@@ -185,10 +185,11 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
 // matrices; for those with few rows the chain itself, K dependent fmaf of four cycles each; and what shared memory delivers,
 // 128 bytes a cycle to all lanes together whether they read the same value or not, which larger TM x TN need less of - but
 // then fewer warps are there to hide its latency.  The sizes below are the fastest of those tried at the widths of
-// Qwen2.5-1.5B (the tiles of 12 rows: 128 CTAs for its 1,536 columns); at 8 to 37,888 columns and 64 to 8,960 k none was slower than the
+// Qwen2.5-1.5B (the tiles of 12 rows: 128 CTAs for its 1,536 columns, of 14: 147 for 2,048); at 8 to 37,888 columns and 64 to 8,960 k none was slower than the
 // register-fed kernels before them.  Measured (M rows; us, and before with the loads of
-// one step ahead in registers): M 8: 1,536 x 8,960 43 (81), 17,920 x 1,536 31 (73), the head of 151,936
-// rows 0.24 ms; M 1: 33 and 23; M 16: 60 and 39.  V16: rows are 16-byte aligned.  G: float4s of k read ahead of the multiplications.
+// one step ahead in registers): M 8: 1,536 x 8,960 39 (81), 17,920 x 1,536 31 (73), the head of 151,936
+// rows 0.24 ms; M 1: 31 and 23; M 16: 51 and 39.  Two rows of A to a thread instead of one took the first from 43 to 39 (and M 16 with 12
+// instead of 16 rows of W from 60 to 51); four, or two rows of W, 52 and more: too few threads.  V16: rows are 16-byte aligned.  G: float4s of k read ahead of the multiplications.
 template <int NT, int KT, int S, int MP, int TM, int TN, int G, bool V16>
 __global__ void __launch_bounds__(256)
 gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
@@ -344,10 +345,22 @@ int launch_gemm_f32(const float* A, const float* W, const float* bias, float* C,
         }
         // a short chain is not worth a ring of long steps, most of which may lie beyond K (16 x 8 x 64 4.6 us in those, 2.2 here; 16 x 1,536 x 384 6.4 and 4.3)
         if (K <= 384) return launch_rows<16, 64, 4, 16, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
-        if (M <= 1) return launch_rows<16, 256, 5, 1, 1, 1, 8>(A, W, bias, C, M, N, K, stream);
+        // The rings take most of an SM's shared memory, one CTA each: 12, 14 or 16 rows of W per CTA, the fewest that leave no second
+        // round (M 8: 2,048 x 1,536 16.5 us with 12 rows, 171 CTAs, and 12.0 with 14, 147 CTAs).
+        const int rows = N <= 12 * 148 ? 12 : N <= 14 * 148 ? 14 : 16;
+        if (M <= 1) {
+            if (rows == 12) return launch_rows<12, 256, 5, 1, 1, 1, 8>(A, W, bias, C, M, N, K, stream);
+            return launch_rows<16, 256, 5, 1, 1, 1, 8>(A, W, bias, C, M, N, K, stream);
+        }
         if (M <= 2) return launch_rows<16, 256, 5, 2, 1, 1, 4>(A, W, bias, C, M, N, K, stream);
         if (M <= 4) return launch_rows<16, 256, 5, 4, 1, 1, 4>(A, W, bias, C, M, N, K, stream);
-        if (M <= 8) return launch_rows<12, 256, 5, 8, 1, 1, 4>(A, W, bias, C, M, N, K, stream);
+        if (M <= 8) {
+            if (rows == 14) return launch_rows<14, 256, 5, 8, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
+            if (N > 14 * 148 && N <= 16 * 148) return launch_rows<16, 256, 5, 8, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
+            return launch_rows<12, 256, 5, 8, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
+        }
+        if (rows == 12) return launch_rows<12, 256, 4, 16, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
+        if (rows == 14) return launch_rows<14, 256, 3, 16, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
         return launch_rows<16, 256, 3, 16, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
     }
     if (!aligned) return 1;

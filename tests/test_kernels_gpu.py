@@ -394,6 +394,21 @@ def test_gemm_f32_few_rows_at_the_edges_of_the_rule(M, N, K_):
         assert torch.equal(out[:M], want[:M]) and bool(torch.isnan(out[M]).all())
 
 
+@pytest.mark.parametrize("N", [1776, 1777, 2072, 2073, 2368, 2369])
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
+def test_gemm_f32_rows_per_cta(M, N):
+    """The widths at which a CTA's rows of W change from 12 to 14 to 16: the bits of the general kernel."""
+    g = torch.Generator().manual_seed(10)
+    rows = torch.randn(17, 520, generator=g)
+    w = torch.randn(N, 520, generator=g).to(DEV)
+    off = torch.empty(17 * 520 + 1, device=DEV)[1:].view(17, 520)
+    off.copy_(rows)
+    want, out = torch.empty(17, N, device=DEV), torch.full((M + 1, N), float("nan"), device=DEV)
+    K.gemm_simt(off, w, None, want)
+    K.gemm_simt(rows[:M].to(DEV), w, None, out[:M])
+    assert torch.equal(out[:M], want[:M]) and bool(torch.isnan(out[M]).all())
+
+
 # ---------------------------------------------------------------------------
 # paged cache helpers for the rope and attention kernels
 # ---------------------------------------------------------------------------
