@@ -218,7 +218,8 @@ __device__ __forceinline__ void load_batch(const u64* src, int row_ld, int units
         for (int k = 0; k < B; ++k) at = fresh(v[k], num) ? at : from[k];
         const uint32_t who = __ballot_sync(0xffffffffu, at != 0xffffffffu);
         if (who == 0 || !w.more(spins, since)) break;
-        w.first(src + at, num, lane - (__ffs(who) - 1));                         // one lane waits for it
+        // many words: one lane waits for that one; few (by a per cent or two): all look again
+        if (B > 6) w.first(src + at, num, lane - (__ffs(who) - 1));
     }
 #pragma unroll
     for (int k = 0; k < B; ++k) *reinterpret_cast<uint2*>(dst + to[k]) = make_uint2((uint32_t)v[k].a, (uint32_t)v[k].b);
@@ -1169,7 +1170,7 @@ static bool dd_plan(int M, int H, int I, int n_q, int n_kv, int D, int sms, int 
     const int merge = DD_WARPS * 8 * (D + 1) * 4;
     // The stage (24 or 32 KB: an SM keeps about five bulk copies in flight, whatever their size, and with 16 KB copies that was 32
     // GB/s of the 44 that are an SM's share of HBM) and down's tp row tiles x S slices of k per group of S CTAs: the fewest blocks
-    // on a CTA (an exchange of partial sums counts four per other slice), with room for at least four stages beside the rows of x.
+    // on a CTA (an exchange of partial sums counts twelve per other slice), with room for at least four stages beside the rows of x.
     long best = -1;
     for (int kbs = 16; kbs >= 12; kbs -= 4)
         for (int tp = 1; tp <= DD_OWN; ++tp) {
@@ -1186,7 +1187,7 @@ static bool dd_plan(int M, int H, int I, int n_q, int n_kv, int D, int sms, int 
                 long stages = (smem_max - rest) / (kbs * DD_BLOCK);
                 if (stages < 4) continue;
                 if (stages > DD_MAX_STAGES) stages = DD_MAX_STAGES;
-                const long cost = (long)kbs * (tp * ((KI + S - 1) / S) + own * KQ + (long)(Tg + n - 1) / n * KH) + 4l * (S - 1);
+                const long cost = (long)kbs * (tp * ((KI + S - 1) / S) + own * KQ + (long)(Tg + n - 1) / n * KH) + 12l * (S - 1);
                 if (best >= 0 && cost >= best) continue;
                 best = cost;
                 out->n = n; out->S = S; out->tp = tp; out->n_groups = groups; out->n_stages = (int)stages; out->kbs = kbs;
