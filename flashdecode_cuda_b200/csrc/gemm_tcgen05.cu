@@ -353,18 +353,21 @@ constexpr int TW_SMEM = TW_STAGES * TW_STAGE_BYTES + 1024 /* alignment slack */ 
 // chain of copies and MMAs (q/k/v with its epilogue at 512 and 1,024 tokens: 16 against 22 us).
 constexpr int TN_BN = 128, TN_STAGES = 6;
 constexpr int TN_SMEM = TN_STAGES * (TC_A_BYTES + TN_BN * TC_BK * 2) + 1024 + 256;
+// With 128 x 64 tiles and four stages of two k-blocks, 48 KB, where those number no more than the SMs either.
+constexpr int TH_BN = 64, TH_STAGES = 4;
+static_assert(TH_STAGES * 2 * (TC_A_BYTES + TH_BN * TC_BK * 2) <= TN_STAGES * (TC_A_BYTES + TN_BN * TC_BK * 2), "the same shared memory");
 // And with 128 x 192 tiles and five stages of 40 KB (choose_tiling).
 constexpr int TM_BN = 192, TM_STAGES = 5;
 constexpr int TM_SMEM = TM_STAGES * (TC_A_BYTES + TM_BN * TC_BK * 2) + 1024 + 256;
 constexpr int TW_EPI_WARPS = 8;               // two per quarter of the tensor-memory lanes, half of the columns each
 constexpr int TW_THREADS = (2 + TW_EPI_WARPS) * 32;
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, int KB = 1>
 __global__ void __launch_bounds__(TW_THREADS, 1)
 gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                          const TcParams p, const TcRope ra, const int tiles_m, const int tiles_n) {
     constexpr int TMEM_COLS = BN <= 128 ? 256 : 512;             // two accumulators, in a power of two of columns
-    constexpr int STAGE_BYTES = TC_A_BYTES + BN * TC_BK * 2;
+    constexpr int STAGE_BYTES = KB * (TC_A_BYTES + BN * TC_BK * 2);      // x: KB tiles of a k-block, then W: KB tiles
     extern __shared__ unsigned char tc_smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + STAGES * STAGE_BYTES);
@@ -376,7 +379,7 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k_iters = (p.K + TC_BK - 1) / TC_BK;
+    const int k_iters = (p.K + KB * TC_BK - 1) / (KB * TC_BK);
 
     if (threadIdx.x == 0) {
         abort_flag[0] = 0;
@@ -420,9 +423,11 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                 const uint32_t fb = s_addr(&full[s]);
                 mbar_expect_tx(fb, STAGE_BYTES);
                 unsigned char* a = tiles + s * STAGE_BYTES;
-                tma_load_2d(s_addr(a), &map_x, fb, k * TC_BK, m0);
+                if (KB == 1) tma_load_2d(s_addr(a), &map_x, fb, k * TC_BK, m0);
+                else tma_load_3d(s_addr(a), &map_x, fb, 0, m0, k * KB);
                 if (p.skip_last && k == k_iters - 1 && tile + (int)gridDim.x >= n_tiles) continue;       // tests: this CTA's very last copy
-                tma_load_2d(s_addr(a + TC_A_BYTES), &map_w, fb, k * TC_BK, n0);     // BN rows of W in one box
+                if (KB == 1) tma_load_2d(s_addr(a + TC_A_BYTES), &map_w, fb, k * TC_BK, n0);     // BN rows of W in one box
+                else tma_load_3d(s_addr(a + KB * TC_A_BYTES), &map_w, fb, 0, n0, k * KB);
             }
         }
         if (*abort_flag) {
@@ -444,10 +449,13 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                 if (!mbar_wait(s_addr(&full[s]), (it / STAGES) & 1, abort_flag, p.status, p.wait_ns)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t a = s_addr(tiles + s * STAGE_BYTES);
-                const uint64_t adesc = smem_desc_sw128(a), bdesc = smem_desc_sw128(a + TC_A_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < TC_BK / 16; ++kk)
-                    tc_mma(acc, adesc + 2 * kk, bdesc + 2 * kk, idesc, (k | kk) != 0);
+                for (int kb = 0; kb < KB; ++kb) {
+                    const uint64_t adesc = smem_desc_sw128(a + kb * TC_A_BYTES), bdesc = smem_desc_sw128(a + KB * TC_A_BYTES + kb * BN * TC_BK * 2);
+#pragma unroll
+                    for (int kk = 0; kk < TC_BK / 16; ++kk)
+                        tc_mma(acc, adesc + 2 * kk, bdesc + 2 * kk, idesc, (k | kb | kk) != 0);
+                }
                 tc_commit(s_addr(&empty[s]));
             }
             if (ok) tc_commit(s_addr(&acc_full[buf]));
@@ -719,6 +727,8 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
         cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_wide_kernel<TW_BN, TW_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, TW_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_wide_kernel<TN_BN, TN_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, TN_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_wide_kernel<TH_BN, TH_STAGES, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TN_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_wide_kernel<TN_BN, TN_STAGES / 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TN_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_wide_kernel<TM_BN, TM_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, TM_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM);
@@ -732,7 +742,7 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
     const int tiling = tiling_of(p, sms);
     const bool wide = tiling != TILING_SINGLE, narrow = tiling == TILING_NARROW, pair = tiling == TILING_PAIR, mid = tiling == TILING_MID;
     const bool pdl = g_pdl != 0 || p.M >= PDL_MIN_ROWS;
-    CUtensorMap mx, mw;
+    CUtensorMap mx, mw, mx2, mw2;
     if (pair) {
         const int tiles_m2 = (p.M + 2 * TC_BM - 1) / (2 * TC_BM), tiles_n = (p.N + TW_BN - 1) / TW_BN;
         const long long n_tiles = (long long)tiles_m2 * tiles_n;
@@ -759,6 +769,18 @@ static int launch_tc(const void* x, const void* w, const TcParams& p, const TcRo
         const long long n_tiles = (long long)tiles_m * tiles_n;
         FD_REQUIRE(n_tiles < (1ll << 30), -2, "gemm_tcgen05: %lld tiles", n_tiles);
         const int grid = (int)(n_tiles < sms ? n_tiles : sms);
+        // Two k-blocks per copy where the three-dimensional view of the operands exists (an SM keeps few copies in flight whatever their
+        // size), and tiles of half the columns while they number no more than the SMs: a CTA that takes one tile is as long as that
+        // tile's copies.  384 rows of q/k/v (2,048 x 1,536) 16.2 us with one k-block per copy, 15.7 with two, 12.3 with 64 columns.
+        if (narrow && w_stack == 1 && p.K % 64 == 0 && p.K >= 128 && tensor_map_blocks(x, p.M, p.K, &mx2, TC_BM, 2) == 0) {
+            const int tiles_h = (p.N + TH_BN - 1) / TH_BN;
+            if ((long long)tiles_m * tiles_h <= sms && tensor_map_blocks(w, p.N, p.K, &mw2, TH_BN, 2) == 0)
+                return launch_with(pdl, what, gemm_tcgen05_wide_kernel<TH_BN, TH_STAGES, 2>, dim3(tiles_m * tiles_h), dim3(TW_THREADS), TN_SMEM,
+                                   stream, dim3(1, 1, 1), mx2, mw2, p, ra, tiles_m, tiles_h);
+            if (tensor_map_blocks(w, p.N, p.K, &mw2, TN_BN, 2) == 0)
+                return launch_with(pdl, what, gemm_tcgen05_wide_kernel<TN_BN, TN_STAGES / 2, 2>, dim3(grid), dim3(TW_THREADS), TN_SMEM, stream,
+                                   dim3(1, 1, 1), mx2, mw2, p, ra, tiles_m, tiles_n);
+        }
         if (narrow)
             return launch_with(pdl, what, gemm_tcgen05_wide_kernel<TN_BN, TN_STAGES>, dim3(grid), dim3(TW_THREADS), TN_SMEM, stream,
                                dim3(1, 1, 1), mx, mw, p, ra, tiles_m, tiles_n);

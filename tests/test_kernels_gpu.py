@@ -329,6 +329,19 @@ def test_gemm_tcgen05(M, N, K_, tc_tiling):
         assert rel(act, P.swiglu(P.linear(x.double(), gate.double()), P.linear(x.double(), up.double()))) < 6e-3
 
 
+@pytest.mark.parametrize("K_", [64, 128, 192, 200, 1536])
+@pytest.mark.parametrize("M,N", [(300, 3136), (300, 3137), (129, 4736), (129, 4752), (513, 272), (1024, 2048)])
+def test_gemm_tcgen05_few_tiles(M, N, K_):
+    """The tilings of products of few tiles: 128 x 64 while those number no more than the SMs (148 and 150 of them, ragged columns), then
+    128 x 128; two k-blocks per copy, an odd number of them, and one where the three-dimensional view does not exist."""
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x, w = torch.randn(M, K_, device=DEV, generator=g).bfloat16(), torch.randn(N, K_, device=DEV, generator=g).bfloat16()
+    out, st = torch.full((M + 1, N), float("nan"), dtype=torch.bfloat16, device=DEV), status()
+    K.gemm_tc(x, w, None, out[:M], status=st)
+    # a bfloat16 rounding of the result, 2^-9 of itself
+    assert rel(out[:M], x.double() @ w.double().T) < 5e-3 and int(st.item()) == 0 and bool(torch.isnan(out[M]).all())
+
+
 @pytest.mark.parametrize("N,K_", [(77, 300), (200, 1537), (10000, 520)])
 def test_gemm_simt_rows_do_not_depend_on_the_batch(N, K_):
     """The same row gives the same bits alone, among 8 and among 100 others: the kernels for up to 16 rows (a
