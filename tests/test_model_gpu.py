@@ -207,6 +207,34 @@ def test_decode_steps_in_one_kernel(engines, folders, name, block_size, n_seqs):
     m.check_status()
 
 
+def test_decode_in_one_kernel_of_many_layers():
+    """More layers than one launch takes (48): the stream is handed on from launch to launch.  Each of the 50 layers adds little, so
+    that the two paths' roundings stay those of a few layers."""
+    from flashdecode_cuda_b200 import kernels as K
+    from flashdecode_cuda_b200.config import config_from_dict
+    m = fd.Model.from_config(config_from_dict(dict(TINY["D"], num_hidden_layers=50)), torch.bfloat16, "cuda")
+    weights = fd.random_weights(m, 3, torch.bfloat16, device="cuda")
+    for name, w in weights.items():
+        if name.endswith(("down_proj.weight", "o_proj.weight")):
+            w.mul_(0.05)
+    m.bind(weights)
+    req = prompts_for(m.vocab_size, [50], seed=8)[0]
+    native, out = m.native, []
+    for on in (True, False):
+        m.native = native
+        cache = m.new_cache(batch_size=1, max_len=64, block_size=16)
+        slot = cache.admit()
+        m.step(cache, [slot], [req[:48]], None)
+        m.native = native if on else None
+        before = K.launch_count()
+        m.step(cache, [slot], [req[48:49]], None)
+        assert (K.launch_count() - before == 3) == on            # the embedding and two for the layers
+        out.append(m.step(cache, [slot], [req[49:]], "last").clone())
+    m.native = native
+    m.check_status()
+    assert rel_err(out[0], out[1]) < TOL["bfloat16"]
+
+
 def test_decode_in_one_kernel_reports(engines):
     """A wait that runs out (one CTA keeps its last words to itself), a missing block and a position beyond the rotation table set
     their status bits and nothing else: the kernel returns, and the next step is right."""
