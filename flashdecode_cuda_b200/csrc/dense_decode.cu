@@ -1,4 +1,4 @@
-// A decode step of a dense model (one new token of up to 16 sequences, bfloat16) in ONE kernel: every layer's norms, q/k/v projection
+// A decode step of a dense model (one new token of up to 24 sequences, bfloat16) in ONE kernel: every layer's norms, q/k/v projection
 // with rotation and cache append, attention over the paged cache, output projection and gated feed-forward.
 //
 // What bounds it.  The step reads every weight once, so HBM does: 14.3 us per layer at the 1.5B sizes.  As seven kernels per layer it took
@@ -7,7 +7,7 @@
 // of shared-memory stages: weights depend on nothing, so the ring runs ahead through every exchange of activations.  With
 // everything but the ring left out a layer takes 14.0 us; what remains on top is the chain of exchanges below.  Measured, us per layer
 // of a replayed step, parts / one kernel: 1.5B sizes, 1 sequence of 1,300 tokens 42.2 / 29.4, 2 of 1,500 41.6 / 32.4, 8 of 2,200 46.2 /
-// 39.1, 16 of 600 49.6 / 44.2; 7B 1 of 1,800 103.8 / 88.7, 8 of 1,800 120.7 / 110.9; 14B 1 of 1,000 127.4 / 103.6, 8 of 1,000 141.8 / 136.4.
+// 39.1, 16 of 600 49.6 / 42.2, 24 of 1,200 63.8 / 56.7; 7B 1 of 1,800 103.8 / 88.7, 8 of 1,800 120.7 / 110.9; 14B 1 of 1,000 127.4 / 103.6, 8 of 1,000 141.8 / 136.4.
 //
 // What is exchanged, and how.  A layer is a chain of exchanges through L2: normed stream -> q, k, v -> partial attention -> attention
 // -> normed stream -> gated activations -> partial sums -> stream.  Each 32-bit word (two bfloat16, or a float) travels in an 8-byte
@@ -20,7 +20,7 @@
 // step and hands out bfloat16(r w) and the sum of r^2; the product's epilogue multiplies by 1 / rms.  One rounding to bfloat16, as
 // with the norm before the product.
 //
-// Split.  Weight rows in tiles of 16 (the M side of mma.sync.m16n8k16: at most 16 rows of x cannot feed a 128-row tcgen05 tile
+// Split.  Weight rows in tiles of 16 (the M side of mma.sync.m16n8k16: at most 24 rows of x cannot feed a 128-row tcgen05 tile
 // from a matrix that is read once), in stages of 16 rows x 768 or 1,024 k, one copy each (3-D tensor map, 128-byte swizzle); the eight
 // consumer warps take 32 k of a stage in turn, the warps' sums meet in shared memory, where one of three finishing warps takes them:
 // what becomes of a tile's sums passes beside the next tiles.  The down projection has few rows and a long k: its k is cut into S
@@ -67,7 +67,7 @@ namespace fd {
 constexpr int DD_WARPS = 8, DD_CONS = DD_WARPS * 32, DD_FIN = 3;                     // consumer warps, finishing warps; and one producer
 constexpr int DD_THREADS = DD_CONS + 32 + DD_FIN * 32;
 constexpr int DD_LAYERS = 48;                                                       // per launch: the kernel's parameters are at most 32 KB
-constexpr int DD_SPLITS = 32, DD_ROWS = 16, DD_OWN = 16, DD_CTAS = 160, DD_MAX_STAGES = 13;
+constexpr int DD_SPLITS = 32, DD_ROWS = 24, DD_OWN = 16, DD_CTAS = 160, DD_MAX_STAGES = 13;
 constexpr int DD_FLYING = 4;                                                        // copies of a CTA under way at a time
 constexpr int DD_BLOCK = 2048;                                                      // 16 rows x 64 k; a stage is kbs of them, one copy
 constexpr unsigned long long DD_WAIT_NS = 2000ull * 1000 * 1000;
@@ -1164,13 +1164,14 @@ struct DdPlan {
 static bool dd_plan(int M, int H, int I, int n_q, int n_kv, int D, int sms, int smem_max, DdPlan* out) {
     if (M < 1 || M > DD_ROWS || (D != 64 && D != 128) || n_kv < 1 || n_q % n_kv != 0 || n_q / n_kv > 8) return false;
     if (H % 64 != 0 || I % 64 != 0 || H < 64 || I < 64 || sms < 1) return false;
-    const int n = sms < DD_CTAS ? sms : DD_CTAS, NT = M > 8 ? 2 : 1;
+    const int n = sms < DD_CTAS ? sms : DD_CTAS, NT = (M + 7) / 8;
     const int Q = n_q * D, Tq = (n_q + 2 * n_kv) * D / 16, Th = H / 16, Tg = I / 8;
     const int wide = H > Q ? H : Q;
     const int merge = DD_WARPS * 8 * (D + 1) * 4;
     // The stage (24 or 32 KB: an SM keeps about five bulk copies in flight, whatever their size, and with 16 KB copies that was 32
     // GB/s of the 44 that are an SM's share of HBM) and down's tp row tiles x S slices of k per group of S CTAs: the fewest blocks
-    // on a CTA (an exchange of partial sums counts twelve per other slice), with room for at least four stages beside the rows of x.
+    // on a CTA (an exchange of partial sums counts twelve per other slice), with room for at least four stages beside the rows of x (three from
+    // 17 rows on: 24 rows of 300 tokens 51.0 us per layer against 59.3 in the kernels of their own; 32 rows, 66.4 against 60.4).
     long best = -1;
     for (int kbs = 16; kbs >= 12; kbs -= 4)
         for (int tp = 1; tp <= DD_OWN; ++tp) {
@@ -1185,7 +1186,7 @@ static bool dd_plan(int M, int H, int I, int n_q, int n_kv, int D, int sms, int 
                 x = (x + 127) / 128 * 128;
                 const long rest = (long)x + dd_red_bytes(NT) + dd_own_bytes(NT, own);
                 long stages = (smem_max - rest) / (kbs * DD_BLOCK);
-                if (stages < 4) continue;
+                if (stages < (NT == 3 ? 3 : 4)) continue;
                 if (stages > DD_MAX_STAGES) stages = DD_MAX_STAGES;
                 const long cost = (long)kbs * (tp * ((KI + S - 1) / S) + own * KQ + (long)(Tg + n - 1) / n * KH) + 12l * (S - 1);
                 if (best >= 0 && cost >= best) continue;
@@ -1337,8 +1338,14 @@ extern "C" int fd_dense_decode(const FdDenseDecode* s, const FdDenseLayer* layer
             o.window = (int)L.window; o.chunk = (int)L.chunk;
             o.f32 = (L.norm1_f32 ? 1 : 0) | (L.norm2_f32 ? 2 : 0) | (L.bias_f32 ? 4 : 0);
         }
-        if (D == 128) rc = plan.NT == 1 ? dd_launch<128, 1>(p, plan, s->stream) : dd_launch<128, 2>(p, plan, s->stream);
-        else rc = plan.NT == 1 ? dd_launch<64, 1>(p, plan, s->stream) : dd_launch<64, 2>(p, plan, s->stream);
+        switch (plan.NT * 1000 + D) {
+            case 1128: rc = dd_launch<128, 1>(p, plan, s->stream); break;
+            case 2128: rc = dd_launch<128, 2>(p, plan, s->stream); break;
+            case 3128: rc = dd_launch<128, 3>(p, plan, s->stream); break;
+            case 1064: rc = dd_launch<64, 1>(p, plan, s->stream); break;
+            case 2064: rc = dd_launch<64, 2>(p, plan, s->stream); break;
+            default: rc = dd_launch<64, 3>(p, plan, s->stream); break;
+        }
         if (rc != 0) return rc;
     }
     return 0;

@@ -7,7 +7,7 @@ pre-norm block, RMS norms, grouped-query attention, SiLU-gated feed-forward,
 nothing between the layers - the same launches are made by ``fd_dense_layers``
 (up to 128 tokens: the whole step in one call) or, layer by layer, by
 ``fd_dense_mixer`` and ``fd_dense_gate_up`` around the library products of the
-output and down projections.  A decode step of up to 16 sequences is one kernel
+output and down projections.  A decode step of up to 24 sequences is one kernel
 for all layers (``fd_dense_decode``) where it takes the sizes.  Everything else, and every step that this module
 does not take, goes through the parts' ``forward``.
 
@@ -39,6 +39,7 @@ from ..parts.mlp import SwiGLU
 from ..parts.norm import RMSNorm
 
 MAX_GROUPS, MAX_POSITIONS = 8, 4
+DECODE_MAX_ROWS = 24         # sequences of a decode step that one kernel takes
 KINDS = (PreNormBlock, RMSNorm, GQAAttention, SwiGLU)
 FORWARDS = [kind.forward for kind in KINDS]                         # what the native calls stand for
 _address = torch.Tensor.data_ptr
@@ -174,7 +175,7 @@ class DensePrompts:
         """Whether the step is one token each of so few sequences that one kernel runs all of its layers
         (``csrc/dense_decode.cu``); every layer has to write the keys that it reads."""
         T = ctx.T
-        if ctx.max_q_len != 1 or T > linear.GEMV_MAX_ROWS or T != ctx.n_rows or not self._current(model) or not self.all_write:
+        if ctx.max_q_len != 1 or T > DECODE_MAX_ROWS or T != ctx.n_rows or not self._current(model) or not self.all_write:
             return False
         if any(g.table.shape[1] * ctx.cache.block_size ** 2 >= 1 << 32 for g in ctx.cache.groups):
             return False                                            # (the kernel divides positions by the block size in 32 bits)

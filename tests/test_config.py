@@ -145,7 +145,7 @@ def test_decode_steps_of_one_kernel_are_dealt_out(sizes):
     H, inter, n_q, n_kv, d = sizes
     smem = 232448
     for sms in (148, 132):
-        for M in range(1, 17):
+        for M in range(1, 25):
             info = []
             words = K.dense_decode_words(M, H, inter, n_q, n_kv, d, sms, smem, info)
             if words == 0:
@@ -153,9 +153,9 @@ def test_decode_steps_of_one_kernel_are_dealt_out(sizes):
                 continue
             slices, rows, ring, used, most = info
             stages, blocks = divmod(ring, 100)
-            assert used <= smem and stages >= 4 and blocks in (12, 16)
+            assert used <= smem and stages >= (4 if M <= 16 else 3) and blocks in (12, 16)
             assert -(-(H // 16) // rows) * slices <= sms and slices <= -(-(inter // 64) // blocks)
             assert most * sms >= inter // 8 and most <= -(-(inter // 8) // sms)
     for bad in ((H + 16, inter, n_q, n_kv, d), (H, inter + 32, n_q, n_kv, d), (H, inter, n_q, n_kv, 96), (H, inter, 9 * n_kv, n_kv, d)):
         assert K.dense_decode_words(1, *bad, 148, smem) == 0
-    assert K.dense_decode_words(17, *sizes, 148, smem) == 0
+    assert K.dense_decode_words(25, *sizes, 148, smem) == 0

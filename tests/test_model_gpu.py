@@ -157,16 +157,16 @@ def test_native_prompt_steps_change_no_bit(engines, name, block_size):
     assert len(taken) >= 6 and len(a) == len(b) and all(torch.equal(x, y) for x, y in zip(a, b))
 
 
-@pytest.mark.parametrize("n_seqs", [1, 2, 8, 9, 16])
+@pytest.mark.parametrize("n_seqs", [1, 2, 8, 9, 16, 17, 24])
 @pytest.mark.parametrize("name,block_size", [("D", 5), ("D", 64), ("E", 16), ("E", 24)])
 def test_decode_steps_in_one_kernel(engines, folders, name, block_size, n_seqs):
-    """Decode steps of up to 16 sequences, all layers in one kernel: contexts around the kernel's tiles of 16 keys and splits of 128
-    (and a window, and more than one split), rows of one and of two column tiles, blocks that do and do not hold whole
+    """Decode steps of up to 24 sequences, all layers in one kernel: contexts around the kernel's tiles of 16 keys and splits of 128
+    (and a window, and more than one split), rows of one to three column tiles, blocks that do and do not hold whole
     tiles, padding rows, against the plain implementation; the same bits when a step is made again; keys and values of the
     new tokens as the parts leave them, to rounding."""
     eng = engines[(name, "bfloat16")]
     m = eng.model
-    lengths = [600, 1, 16, 128, 15, 127, 129, 17, 255, 256, 3, 383, 64, 31, 500, 2][:n_seqs]
+    lengths = [600, 1, 16, 128, 15, 127, 129, 17, 255, 256, 3, 383, 64, 31, 500, 2, 9, 33, 100, 260, 1, 32, 47, 400][:n_seqs]
     reqs = prompts_for(m.vocab_size, [n + 2 for n in lengths], seed=90)
     native, taken = m.native, []
 
@@ -193,8 +193,8 @@ def test_decode_steps_in_one_kernel(engines, folders, name, block_size, n_seqs):
     (got, kv), (again, _), (parts, kv_parts) = steps(True), steps(True), steps(False)
     assert len(taken) == 4
     assert all(torch.equal(a, b) for a, b in zip(got, again))
-    if n_seqs < 16:
-        for pad in (1, 16 - n_seqs):
+    if n_seqs < 24:
+        for pad in (1, 24 - n_seqs):
             padded, _ = steps(True, pad=pad)
             assert all(rel_err(a, b) < TOL["bfloat16"] for a, b in zip(padded, got))
         assert len(taken) == 8
