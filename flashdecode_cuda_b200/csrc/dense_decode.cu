@@ -1300,6 +1300,7 @@ extern "C" int fd_dense_decode(const FdDenseDecode* s, const FdDenseLayer* layer
     if (rc != 0) return rc;
     DdPlan plan;
     FD_REQUIRE(dd_plan(M, H, I, n_q, n_kv, D, sms, smem, &plan), -2, "dense_decode: sizes not taken");
+    FD_REQUIRE((uintptr_t)s->next % 16 == 0, -2, "dense_decode: the memory to prefetch must be 16-byte aligned");
     const DdBuffers buf = dd_buffers(M, H, I, n_q, n_kv, D, plan.S);
     static thread_local DdParams p;               // (26 KB: not on the caller's stack)
     u64* at = static_cast<u64*>(s->exchange);

@@ -192,9 +192,7 @@ class DensePrompts:
         # zeroed when it is made; for these rows only, so that every word is written in every step
         s.exchange = ctx.ws.get(f"dense_decode.{ctx.T}", (self.exchange_words[ctx.T],), torch.int64).data_ptr()
         s.M = ctx.T
-        if upcoming is not None:
-            s.next = upcoming.data_ptr()
-            s.next_bytes = min(upcoming.numel() * upcoming.element_size(), linear.UPCOMING_BYTES)
+        s.next, s.next_bytes = K._prefetch_args(upcoming, linear.UPCOMING_BYTES)       # (a hint: the head may be any part)
         self._cache_args(s, cache)
         K._check(K.lib().fd_dense_decode(ctypes.addressof(s), self.addresses[0], self.n))
 
