@@ -34,8 +34,8 @@
 // code, and batches of loads have a fixed number (beyond the end: an earlier one once more).
 //
 // Waits: on mbarriers and on packets, all bounded (fd_tc_test_hook's limit does for both): a wait that runs out sets the abort flag
-// of its CTA and STATUS_WAIT_TIMEOUT, and everything after it goes on without waiting.  The launch is cooperative, so that all CTAs
-// are on the GPU together or the launch is refused.
+// of its CTA and STATUS_WAIT_TIMEOUT, and everything after it goes on without waiting.  Where a warp votes on what its lanes saw, the lanes
+// give up together.  The launch is cooperative, so that all CTAs are on the GPU together or the launch is refused.
 #include <string.h>
 
 #include <type_traits>
@@ -93,7 +93,8 @@ struct DdParams {
     const unsigned char* pf_ptr;         // what the step streams next: the last CTAs ask L2 for its beginning
     unsigned long long pf_bytes, wait_ns;
     int n_layers, M, H, I, n_q, n_kv, num_blocks, block_size;
-    int S, tp, n_groups, n_stages, skip;
+    int S, tp, n_groups, n_stages;
+    int skip;                            // tests: what one CTA keeps to itself in the last layer: 1 normed stream, 2 queries, 3 attention, 4 partial sums
     int flying;                          // copies of a CTA under way at a time
     int kbs;                             // blocks of 64 k in a stage
     int x_bytes;                         // shared memory for the rows of x
@@ -129,17 +130,19 @@ struct Waiter {
     volatile int* abort;                          // in shared memory
     int* status;
     u64 limit;
+    // Having said no it goes on saying so: where a warp looks at its words together, a lane that has given up drops out of the vote on
+    // who still waits, and the lanes leave together when nobody does.
     __device__ __forceinline__ bool more(uint32_t& spins, u64& since) const {
         if ((++spins & 63) != 0) return true;
-        if (*abort) return false;
-        const u64 now = global_ns();
-        if (since == 0) since = now;
-        else if (now - since > limit) {
+        if (!*abort) {
+            const u64 now = global_ns();
+            if (since == 0) since = now;
+            if (now - since <= limit) return true;
             *abort = 1;
             set_status(status, STATUS_WAIT_TIMEOUT);
-            return false;
         }
-        return true;
+        --spins;
+        return false;
     }
     __device__ __forceinline__ bool bar(uint32_t bar, uint32_t parity) const {
         uint32_t spins = 0;
@@ -216,8 +219,8 @@ __device__ __forceinline__ void load_batch(const u64* src, int row_ld, int units
         uint32_t at = 0xffffffffu;                // the last one that is not there
 #pragma unroll
         for (int k = 0; k < B; ++k) at = fresh(v[k], num) ? at : from[k];
-        const uint32_t who = __ballot_sync(0xffffffffu, at != 0xffffffffu);
-        if (who == 0 || !w.more(spins, since)) break;
+        const uint32_t who = __ballot_sync(0xffffffffu, at != 0xffffffffu && w.more(spins, since));
+        if (who == 0) break;
         // many words: one lane waits for that one; few (by a per cent or two): all look again
         if (B > 6) w.first(src + at, num, lane - (__ffs(who) - 1));
     }
@@ -263,6 +266,7 @@ __device__ __forceinline__ void tile_sums(const DdParams& p, const Waiter& w, Dd
 #pragma unroll 1
     for (int st = 0; st < nst; ++st) {
         w.bar(s_addr(&sh->full[at.slot]), at.phase);
+        __syncwarp();
         const uint32_t a_s = a_row + at.slot * p.kbs * DD_BLOCK;
         const int u1 = min(units, left - st * units);
         auto load = [&](int u, uint32_t (&a)[2][4], uint32_t (&b)[NT][4]) {
@@ -305,6 +309,7 @@ __device__ __forceinline__ void tile_sums(const DdParams& p, const Waiter& w, Dd
     }
     // to finishing warp f (bit f of `turns`: the parity of its turn), when it has taken its tile before
     w.bar(s_addr(&sh->taken[f]), (turns >> f & 1) ^ 1);
+    __syncwarp();
     turns ^= 1u << f;
     float* red = red_all + f * (DD_WARPS * NT * 128);
 #pragma unroll
@@ -321,6 +326,7 @@ __device__ __forceinline__ void tile_sums(const DdParams& p, const Waiter& w, Dd
 template <int NT>
 __device__ __forceinline__ void take_sums(const Waiter& w, DdShared* sh, const float* red_all, int f, uint32_t& turn, int lane, float2 (&v)[NT][2]) {
     w.bar(s_addr(&sh->sums[f]), turn);
+    __syncwarp();
     turn ^= 1;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
@@ -363,8 +369,8 @@ __device__ __forceinline__ void row_norms(const u64* ss, float* out, int M, int 
                 for (int k = 0; k < R; ++k)
 #pragma unroll
                     for (int i = 0; i < B; ++i) done = done && fresh(v[k][i], num);
-                const uint32_t who = __ballot_sync(0xffffffffu, !done);
-                if (who == 0 || !w.more(spins, since)) break;
+                const uint32_t who = __ballot_sync(0xffffffffu, !done && w.more(spins, since));
+                if (who == 0) break;
                 const u64* at = word(0, 0);
 #pragma unroll
                 for (int k = 0; k < R; ++k)
@@ -463,8 +469,8 @@ __device__ __forceinline__ void wait_words(const u64* p, uint32_t num, const Wai
         done = true;
 #pragma unroll
         for (int j = 0; j < C; ++j) done = done && fresh(v[j][0], num) && fresh(v[j][1], num);
-        const uint32_t who = __ballot_sync(0xffffffffu, !done);
-        if (who == 0 || !w.more(spins, since)) break;
+        const uint32_t who = __ballot_sync(0xffffffffu, !done && w.more(spins, since));
+        if (who == 0) break;
         const u64* at = p;
 #pragma unroll
         for (int j = 0; j < C; ++j) at = fresh(v[j][0], num) && fresh(v[j][1], num) ? at : p + j * 16 + (fresh(v[j][0], num) ? 2 : 0);
@@ -483,7 +489,7 @@ __device__ __forceinline__ void attend(const DdParams& p, const DdLayer& L, DdSh
                                        const Waiter& w, int tid) {
     constexpr int C = D / 32, OS = D + 1;
     const int warp = tid >> 5, lane = tid & 31, r = lane >> 2, q = lane & 3;
-    const int G = p.n_q / p.n_kv, ctx = sh->ctx[b], slot = sh->slot[b], ns = sh->ns[b];
+    const int G = p.n_q / p.n_kv, ctx = sh->ctx[b], slot = sh->slot[b];
     const int k0 = sh->lo[b] + split * sh->cut, k1 = min(k0 + sh->cut, ctx + 1);
     const int bs = p.block_size;
     auto column = [&](int key) -> int { return (int)((u64)key * p.bs_inv >> 32); };           // key / bs
@@ -631,7 +637,8 @@ __device__ __forceinline__ void attend(const DdParams& p, const DdLayer& L, DdSh
         for (int k = 0; k < C; ++k) a[k] = fmaf(from[k * 32], fi, a[k]);
     }
     const size_t row = (size_t)b * p.n_q + kvh * G + h;
-    if (ns > 1) {
+    if (p.skip == 3 && &L == &p.layer[p.n_layers - 1] && blockIdx.x == gridDim.x - 1) return;
+    if (sh->ns[b] > 1) {
         u64* out = p.part + (row * DD_SPLITS + split) * (D + 2);
 #pragma unroll
         for (int k = 0; k < C; ++k) put(out + 2 + k * 32 + lane, __float_as_uint(a[k]), num);
@@ -688,8 +695,7 @@ __device__ __forceinline__ void merge_splits(const DdParams& p, DdShared* sh, ui
 #pragma unroll
                     for (int k = 0; k < W / 2; ++k) all = all && fresh(v[i][k], num);
                 }
-                all = __all_sync(0xffffffffu, all);
-                if (all || !w.more(spins, t0)) break;
+                if (!__any_sync(0xffffffffu, !all && w.more(spins, t0))) break;
                 int late = 0;                     // the last split that is not there
 #pragma unroll
                 for (int i = 1; i < B; ++i) late = fresh(ml[i], num) ? late : i;
@@ -946,6 +952,7 @@ __global__ void __launch_bounds__(DD_THREADS, 1) dense_decode_kernel(const __gri
                             const uint32_t word = pair_words(x, r);
                             if (m >= M) continue;
                             if (head < p.n_q) {
+                                if (p.skip == 2 && l == p.n_layers - 1 && c == 0) continue;
                                 put(p.q + ((size_t)m * p.n_q + head) * (D / 2) + dim / 2, word, num);
                                 continue;
                             }
@@ -974,7 +981,7 @@ __global__ void __launch_bounds__(DD_THREADS, 1) dense_decode_kernel(const __gri
                     v[nt][1] = make_float2(o.y + v[nt][1].x, o.w + v[nt][1].y);
                     *own = make_float4(v[nt][0].x, v[nt][1].x, v[nt][0].y, v[nt][1].y);
                 }
-                if (p.skip && l == p.n_layers - 1 && c == 0) continue;
+                if (p.skip == 1 && l == p.n_layers - 1 && c == 0) continue;
                 hand_out(1, w0, w1, row0, v, num);
             }
             // ---- gate and up: norm, activation
@@ -1015,7 +1022,7 @@ __global__ void __launch_bounds__(DD_THREADS, 1) dense_decode_kernel(const __gri
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const int m = nt * 8 + cq + e;
-                        if (m < M)
+                        if (m < M && !(p.skip == 4 && l == p.n_layers - 1 && c == 0))
                             put2(p.dpart + ((((size_t)(g0 + j) * p.S + member) * M + m) * 8 + r) * 2, __float_as_uint(v[nt][e].x), __float_as_uint(v[nt][e].y), num);
                     }
                 }

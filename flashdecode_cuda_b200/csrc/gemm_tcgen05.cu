@@ -905,9 +905,9 @@ extern "C" int fd_gemm_tc_qkv_rope(const void* x, const void* w, const void* bia
 
 // Tests only: the limit of every bounded wait in the TMA + tcgen05 kernels (nanoseconds; 0 restores the
 // default of 0.2 s), and whether their TMA producers leave out their very last copy, so that a wait runs
-// out, the kernel reports STATUS_WAIT_TIMEOUT and returns.  Nothing faults or hangs.
+// out, the kernel reports STATUS_WAIT_TIMEOUT and returns (dense_decode.cu: 1 to 4 say which words a CTA keeps).  Nothing faults or hangs.
 extern "C" int fd_tc_test_hook(long long wait_ns, int skip_last) {
     g_tc_wait_ns = wait_ns > 0 ? (unsigned long long)wait_ns : TC_WAIT_NS;
-    g_tc_skip_last = skip_last ? 1 : 0;
+    g_tc_skip_last = skip_last;
     return 0;
 }

@@ -682,10 +682,11 @@ def gemm_stream_last_map3d() -> bool:
     return bool(lib().fd_gemm_stream_last_map3d())
 
 
-def tc_test_hook(wait_ns: int = 0, skip_last: bool = False) -> None:
+def tc_test_hook(wait_ns: int = 0, skip_last: int = 0) -> None:
     """Tests only.  The limit of every bounded wait of the TMA + tcgen05 kernels (0: the default of
     0.2 s) and whether their producers leave out their very last copy, so that a wait runs out and the
-    kernel reports ``STATUS_WAIT_TIMEOUT`` and returns."""
+    kernel reports ``STATUS_WAIT_TIMEOUT`` and returns.  In a one-kernel decode step one CTA keeps words of the last layer
+    to itself: 1 its normed stream, 2 its queries, 3 its attention, 4 its partial sums of the down projection."""
     lib().fd_tc_test_hook(int(wait_ns), int(skip_last))
 
 

@@ -235,6 +235,91 @@ def test_decode_in_one_kernel_of_many_layers():
     assert rel_err(out[0], out[1]) < TOL["bfloat16"]
 
 
+# Decode steps at real widths, two layers: hidden, feed-forward, query heads, KV heads, head size, the numbers of sequences
+DECODE_WIDTHS = {
+    "1.5B": (1536, 8960, 12, 2, 128, [8, 9, 16, 17, 24]),
+    "7B": (3584, 18944, 28, 4, 128, [8, 9, 14]),
+    "14B": (5120, 13824, 40, 8, 128, [8, 9]),
+    "groups of 8": (2048, 8192, 32, 4, 64, [5, 16, 24]),
+}
+
+
+def _decode_model(sizes, seed=3):
+    """Two layers of such widths, a small vocabulary."""
+    from flashdecode_cuda_b200.config import config_from_dict
+    hidden, inter, n_q, n_kv, d, _ = DECODE_WIDTHS[sizes]
+    raw = dict(TINY["D"], hidden_size=hidden, intermediate_size=inter, num_attention_heads=n_q, num_key_value_heads=n_kv, head_dim=d,
+               vocab_size=512, max_position_embeddings=2048)
+    m = fd.Model.from_config(config_from_dict(raw), torch.bfloat16, "cuda")
+    return m.bind(fd.random_weights(m, seed, torch.bfloat16, device="cuda"))
+
+
+@pytest.fixture(scope="module")
+def decode_models():
+    made = {}
+
+    def get(sizes):
+        if sizes not in made:
+            made.clear()
+            made[sizes] = _decode_model(sizes)
+        return made[sizes]
+    return get
+
+
+def _decode_steps(m, reqs, lengths, native, steps=2, pad=0, bound=None, block_size=16):
+    """The sequences' prompts, then ``steps`` decode steps with or without the one-kernel path: the logits of every step, and the
+    cache with its slots."""
+    cache = m.new_cache(batch_size=len(reqs), max_len=1280, block_size=block_size)
+    slots = [cache.admit() for _ in reqs]
+    for s, r, n in zip(slots, reqs, lengths):
+        m.step(cache, [s], [r[:n]], None)                # each alone: their keys are the same bits beside any other sequences
+    kept, out = m.native, []
+    m.native = kept if native else None
+    try:
+        for j in range(steps):
+            cache.reserve([(s, 1) for s in slots])
+            cache.sync()
+            ctx = m.make_context(cache, slots, [[r[n + j]] for r, n in zip(reqs, lengths)], "all", pad_rows=pad, kv_len_bound=bound)
+            assert not native or kept.decodes(m, ctx)
+            out.append(m.forward(ctx)[:len(reqs)].clone())
+            for s in slots:
+                cache.advance(s, 1)
+    finally:
+        m.native = kept
+    m.check_status()
+    return out, cache, slots
+
+
+@pytest.mark.parametrize("kept", [1, 2, 3, 4])
+def test_decode_in_one_kernel_every_wait_ends(decode_models, kept):
+    """Words that one CTA keeps to itself - its normed stream, its queries, its attention, its partial sums - let the waits for them run
+    out: the kernel reports that and returns, and the next step is right."""
+    from flashdecode_cuda_b200 import kernels as K
+    m = decode_models("1.5B")
+    lengths = [900, 40]
+    reqs = prompts_for(m.vocab_size, [n + 1 for n in lengths], seed=6)
+    first, cache, slots = _decode_steps(m, reqs, lengths, True, steps=1)
+    for s in slots:
+        cache.release(s)
+    slots = [cache.admit() for _ in reqs]
+    for s, r, n in zip(slots, reqs, lengths):
+        m.step(cache, [s], [r[:n]], None)
+    cache.reserve([(s, 1) for s in slots])
+    cache.sync()
+
+    def step():
+        return m.forward(m.make_context(cache, slots, [[r[n]] for r, n in zip(reqs, lengths)], "all")).clone()
+    try:
+        K.tc_test_hook(wait_ns=1_000_000, skip_last=kept)
+        step()
+        with pytest.raises(RuntimeError, match="wait"):
+            m.check_status()
+    finally:
+        K.tc_test_hook()
+    assert torch.equal(step(), first[0])
+    m.check_status()
+
+
 def test_decode_in_one_kernel_reports(engines):
     """A wait that runs out (one CTA keeps its last words to itself), a missing block and a position beyond the rotation table set
     their status bits and nothing else: the kernel returns, and the next step is right."""
