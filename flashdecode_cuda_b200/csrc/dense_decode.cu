@@ -26,7 +26,7 @@
 // what becomes of a tile's sums passes beside the next tiles.  The down projection has few rows and a long k: its k is cut into S
 // slices and `tp` row tiles share a CTA so that tiles x slices fill the grid (dd_plan), the partial sums go to the tile's owner in
 // packets.  Keys and values go from global memory straight to registers as MMA fragments, the first tile before the queries arrive;
-// splits of at least 128 keys, as many as the grid takes.
+// a row's keys in as many splits of at least 128 as are its share of the grid.
 //
 // No local memory.  Beside 227 KB of shared memory an SM has some 20 KB of L1, and every word of a stack that 384 threads share goes
 // to L2: with 100 to 600 bytes of stack a thread (arguments by reference to functions that were not inlined, arrays that were filled
@@ -97,6 +97,7 @@ struct DdParams {
     int skip;                            // tests: what one CTA keeps to itself in the last layer: 1 normed stream, 2 queries, 3 attention, 4 partial sums
     int flying;                          // copies of a CTA under way at a time
     int kbs;                             // blocks of 64 k in a stage
+    int splits;                          // of a row's keys, at the most
     int x_bytes;                         // shared memory for the rows of x
     short gu[DD_CTAS + 1];               // gate/up tiles of CTA c: gu[c] .. gu[c + 1]
 };
@@ -180,8 +181,8 @@ struct DdShared {
     int abort;
     uint32_t base;
     int slot[DD_ROWS], pos[DD_ROWS], ctx[DD_ROWS];
-    // attention: keys that row b sees from lo[b] on, cut into ns[b] splits of `cut` keys; items of one KV head before row b
-    int lo[DD_ROWS], ns[DD_ROWS], before[DD_ROWS + 1], cut;
+    // attention: keys that row b sees from lo[b] on, cut into ns[b] splits of cut[b] keys; items of one KV head before row b
+    int lo[DD_ROWS], ns[DD_ROWS], cut[DD_ROWS], before[DD_ROWS + 1];
     float inv[2][DD_ROWS];
     float m[DD_WARPS][8], l[DD_WARPS][8];
     float merge[DD_WARPS][132];
@@ -401,7 +402,9 @@ __device__ __forceinline__ uint32_t pair_words(float2 v, int r) {
     return (r & 1) ? pack_bf16(got, v.y) : pack_bf16(v.x, got);
 }
 
-// Which keys each row sees in a layer, and how they are cut; by one warp.
+// Which keys each row sees in a layer, and how they are cut: into at the most p.splits splits of 128 keys and more, in steps of 64.  That
+// follows from the row's own length and the number of rows, not from the other rows' lengths, and so does every bit of its result.
+// By one warp.
 __device__ __forceinline__ void cut_keys(const DdParams& p, DdShared* sh, int window, int chunk, int lane) {
     const bool live = lane < p.M && sh->slot[lane] >= 0;
     int lo = 0, len = 0;
@@ -411,24 +414,7 @@ __device__ __forceinline__ void cut_keys(const DdParams& p, DdShared* sh, int wi
         if (chunk > 0) lo = max(lo, ctx / chunk * chunk);
         len = ctx + 1 - lo;
     }
-    int total = len, longest = len;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        total += __shfl_xor_sync(0xffffffffu, total, o);
-        longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
-    }
-    const int places = max((int)gridDim.x / p.n_kv, p.M);
-    int cut = max((total + places - 1) / places, (longest + DD_SPLITS - 1) / DD_SPLITS);
-    cut = max(128, (cut + 127) / 128 * 128);
-    int ns, sum;
-#pragma unroll 1
-    for (;; cut += 128) {                         // ends at the latest when every row is one split
-        ns = (len + cut - 1) / cut;
-        sum = ns;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (sum <= places) break;
-    }
+    const int cut = max(128, ((len + p.splits - 1) / p.splits + 63) / 64 * 64), ns = (len + cut - 1) / cut;
     int inc = ns;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -438,8 +424,9 @@ __device__ __forceinline__ void cut_keys(const DdParams& p, DdShared* sh, int wi
     if (lane < DD_ROWS) {
         sh->lo[lane] = lo;
         sh->ns[lane] = ns;
+        sh->cut[lane] = cut;
         sh->before[lane + 1] = inc;
-        if (lane == 0) { sh->before[0] = 0; sh->cut = cut; }
+        if (lane == 0) sh->before[0] = 0;
     }
 }
 
@@ -490,7 +477,7 @@ __device__ __forceinline__ void attend(const DdParams& p, const DdLayer& L, DdSh
     constexpr int C = D / 32, OS = D + 1;
     const int warp = tid >> 5, lane = tid & 31, r = lane >> 2, q = lane & 3;
     const int G = p.n_q / p.n_kv, ctx = sh->ctx[b], slot = sh->slot[b];
-    const int k0 = sh->lo[b] + split * sh->cut, k1 = min(k0 + sh->cut, ctx + 1);
+    const int k0 = sh->lo[b] + split * sh->cut[b], k1 = min(k0 + sh->cut[b], ctx + 1);
     const int bs = p.block_size;
     auto column = [&](int key) -> int { return (int)((u64)key * p.bs_inv >> 32); };           // key / bs
     const int* table = L.table + (size_t)slot * L.max_blocks;
@@ -1109,7 +1096,7 @@ __global__ void __launch_bounds__(DD_THREADS, 1) dense_decode_kernel(const __gri
             int b = 0;
 #pragma unroll 1
             while (sh->before[b + 1] <= place) ++b;
-            const int k0 = sh->lo[b] + (place - sh->before[b]) * sh->cut, k1 = min(k0 + sh->cut, sh->ctx[b]);
+            const int k0 = sh->lo[b] + (place - sh->before[b]) * sh->cut[b], k1 = min(k0 + sh->cut[b], sh->ctx[b]);
 #pragma unroll 1
             for (int key = k0 + (tid >> 1); key < k1; key += DD_CONS / 2) {
                 const int col = (int)((u64)key * p.bs_inv >> 32), blk = L.table[(size_t)sh->slot[b] * L.max_blocks + col];
@@ -1227,6 +1214,17 @@ static bool dd_plan(int M, int H, int I, int n_q, int n_kv, int D, int sms, int 
     return Tg <= 32767;
 }
 
+// The splits of a row's keys at the most: its share of a grid in which every CTA takes one (row, KV head, split).  A CTA that takes two is
+// some 2.7 us later than one with a single one of the same keys, so shares are rounded down.  What it costs that rows of unequal lengths get equal
+// shares, us per layer, keys cut by the batch's mean length / by the row's own: 1.5B sizes, 8 rows of 2,200 tokens 41.0 / 40.4, of 1,500 to 3,000
+// 42.4 / 42.4, 12 of 500 to 900 45.8 / 46.8, 16 of 600 47.1 / 46.9, 24 of 400 to 1,800 58.1 / 58.9; 7B 8 of 1,800 105.8 / 106.3, of 1,100 to
+// 2,600 105.7 / 109.5.  In steps of 128 keys the last is 110.5, in steps of 16 108.8 (and the second 42.6).  Cut by the step's length bound, 0.6
+// of which a row has on average, 8 of 1,800 take 108.7 at 7B and 8 of 1,000 126.7 at 14B sizes (124.3): two splits for most CTAs.
+static int dd_splits(int M, int n_kv, int n) {
+    const int share = n / (M * n_kv);
+    return share < 1 ? 1 : share > DD_SPLITS ? DD_SPLITS : share;
+}
+
 // The exchange memory, in packets: where each buffer starts, and the whole
 struct DdBuffers {
     size_t x[2], ss[2], q, kv, part, attn, act, dpart, all;
@@ -1323,6 +1321,7 @@ extern "C" int fd_dense_decode(const FdDenseDecode* s, const FdDenseLayer* layer
     p.num_blocks = (int)s->num_blocks; p.block_size = (int)s->block_size;
     p.bs_inv = (0x100000000ull + p.block_size - 1) / p.block_size;
     p.S = plan.S; p.tp = plan.tp; p.n_groups = plan.n_groups; p.n_stages = plan.n_stages; p.kbs = plan.kbs; p.flying = plan.n_stages - 1 < DD_FLYING ? plan.n_stages - 1 : DD_FLYING; p.x_bytes = plan.x_bytes;
+    p.splits = dd_splits(M, n_kv, plan.n);
     memcpy(p.gu, plan.gu, sizeof(p.gu));
     for (int l0 = 0; l0 < count; l0 += DD_LAYERS) {
         p.pf_ptr = static_cast<const unsigned char*>(s->next);

@@ -266,7 +266,7 @@ def decode_models():
     return get
 
 
-def _decode_steps(m, reqs, lengths, native, steps=2, pad=0, bound=None, block_size=16):
+def _decode_steps(m, reqs, lengths, native, steps=2, pad=0, block_size=16):
     """The sequences' prompts, then ``steps`` decode steps with or without the one-kernel path: the logits of every step, and the
     cache with its slots."""
     cache = m.new_cache(batch_size=len(reqs), max_len=1280, block_size=block_size)
@@ -279,7 +279,7 @@ def _decode_steps(m, reqs, lengths, native, steps=2, pad=0, bound=None, block_si
         for j in range(steps):
             cache.reserve([(s, 1) for s in slots])
             cache.sync()
-            ctx = m.make_context(cache, slots, [[r[n + j]] for r, n in zip(reqs, lengths)], "all", pad_rows=pad, kv_len_bound=bound)
+            ctx = m.make_context(cache, slots, [[r[n + j]] for r, n in zip(reqs, lengths)], "all", pad_rows=pad)
             assert not native or kept.decodes(m, ctx)
             out.append(m.forward(ctx)[:len(reqs)].clone())
             for s in slots:
@@ -288,6 +288,22 @@ def _decode_steps(m, reqs, lengths, native, steps=2, pad=0, bound=None, block_si
         m.native = kept
     m.check_status()
     return out, cache, slots
+
+
+@pytest.mark.parametrize("sizes,n_seqs", [("1.5B", 2), ("1.5B", 8), ("1.5B", 24), ("groups of 8", 16)])
+def test_decode_bits_do_not_depend_on_the_neighbours(decode_models, sizes, n_seqs):
+    """At one batch size a sequence's logits have the same bits whatever the other sequences' lengths, and beside padding rows: where its
+    keys are cut follows from its own length."""
+    m = decode_models(sizes)
+    first = prompts_for(m.vocab_size, [902], seed=4)[0]
+    out = []
+    for lengths, pad in (([900] + [1000 - 31 * i for i in range(n_seqs - 1)], 0), ([900] + [3 + i for i in range(n_seqs - 1)], 0),
+                         ([900], n_seqs - 1)):
+        reqs = [first] + prompts_for(m.vocab_size, [n + 2 for n in lengths[1:]], seed=5)
+        got, _, _ = _decode_steps(m, reqs, lengths, True, pad=pad)
+        out.append([x[0] for x in got])
+    for other in out[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(out[0], other))
 
 
 @pytest.mark.parametrize("kept", [1, 2, 3, 4])
