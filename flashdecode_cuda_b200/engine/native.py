@@ -175,7 +175,9 @@ class DensePrompts:
         """Whether the step is one token each of so few sequences that one kernel runs all of its layers
         (``csrc/dense_decode.cu``); every layer has to write the keys that it reads."""
         T = ctx.T
-        if ctx.max_q_len != 1 or T > DECODE_MAX_ROWS or T != ctx.n_rows or not self._current(model) or not self.all_write:
+        if ctx.max_q_len != 1 or T > (DECODE_MAX_ROWS if linear.PROMPT_GEMM == "auto" else linear.GEMV_MAX_ROWS) or T != ctx.n_rows:
+            return False
+        if not self._current(model) or not self.all_write:
             return False
         if any(g.table.shape[1] * ctx.cache.block_size ** 2 >= 1 << 32 for g in ctx.cache.groups):
             return False                                            # (the kernel divides positions by the block size in 32 bits)

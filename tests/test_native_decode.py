@@ -77,3 +77,10 @@ def test_only_memory_that_l2_can_be_asked_for(calls, upcoming, want):
     assert native.decodes(None, ctx)
     native.decode(ctx, torch.zeros(2, 1536), upcoming)
     assert [(s.next, s.next_bytes) for s in calls] == [want]
+
+
+@pytest.mark.parametrize("gemm,most", [("auto", 24), ("tcgen05", 16), ("cublas", 16)])
+def test_the_switch_for_products_rules_from_17_rows_on(calls, monkeypatch, gemm, most):
+    """``linear.PROMPT_GEMM`` names the kernels of steps of more than 16 rows; a step that is to run on others is not one kernel."""
+    monkeypatch.setattr(linear, "PROMPT_GEMM", gemm)
+    assert [rows for rows in range(1, 26) if _step(rows)[0].decodes(None, _step(rows)[1])] == list(range(1, most + 1))
