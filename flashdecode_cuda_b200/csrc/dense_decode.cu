@@ -626,7 +626,7 @@ __device__ __forceinline__ void attend(const DdParams& p, const DdLayer& L, DdSh
     const size_t row = (size_t)b * p.n_q + kvh * G + h;
     if (p.skip == 3 && &L == &p.layer[p.n_layers - 1] && blockIdx.x == gridDim.x - 1) return;
     if (sh->ns[b] > 1) {
-        u64* out = p.part + (row * DD_SPLITS + split) * (D + 2);
+        u64* out = p.part + (uint32_t)(((int)row * p.splits + split) * (D + 2));
 #pragma unroll
         for (int k = 0; k < C; ++k) put(out + 2 + k * 32 + lane, __float_as_uint(a[k]), num);
         if (lane == 0) put2(out, __float_as_uint(m * scale_log2), __float_as_uint(l), num);
@@ -657,7 +657,7 @@ __device__ __forceinline__ void merge_splits(const DdParams& p, DdShared* sh, ui
 #pragma unroll
             for (int i = 0; i < W / 2; ++i) put(out + i, 0u, num);
         }
-        const u64* src = p.part + (size_t)item * DD_SPLITS * (D + 2);
+        const u64* src = p.part + (uint32_t)(item * p.splits * (D + 2));
         float m = -INFINITY, l = 0.f, a[W];
 #pragma unroll
         for (int i = 0; i < W; ++i) a[i] = 0.f;
@@ -1225,11 +1225,13 @@ static int dd_splits(int M, int n_kv, int n) {
     return share < 1 ? 1 : share > DD_SPLITS ? DD_SPLITS : share;
 }
 
-// The exchange memory, in packets: where each buffer starts, and the whole
+// The exchange memory, in packets: where each buffer starts, and the whole.  The control words come first for all sizes: steps of
+// different ones may share the memory, as what an earlier step left anywhere has another number than any that is awaited (numbers come
+// round after 2^32: a word would have to lie unwritten for all of them).  At 24 rows of the 1.5B sizes 3.5 MB, at 8 of 7B 3.1.
 struct DdBuffers {
     size_t x[2], ss[2], q, kv, part, attn, act, dpart, all;
 };
-static DdBuffers dd_buffers(int M, int H, int I, int n_q, int n_kv, int D, int S) {
+static DdBuffers dd_buffers(int M, int H, int I, int n_q, int n_kv, int D, const DdPlan& plan) {
     DdBuffers b;
     size_t at = 16;                               // the control words
     auto take = [&](size_t packets) { const size_t o = at; at += (packets + 15) / 16 * 16; return o; };
@@ -1242,8 +1244,8 @@ static DdBuffers dd_buffers(int M, int H, int I, int n_q, int n_kv, int D, int S
     b.kv = take(m * n_kv * D);
     b.attn = take(m * n_q * D / 2);
     b.act = take(m * I / 2);
-    b.dpart = take(m * H * S);
-    b.part = take(m * n_q * DD_SPLITS * (D + 2));
+    b.dpart = take(m * H * plan.S);
+    b.part = take(m * n_q * dd_splits(M, n_kv, plan.n) * (D + 2));
     b.all = at;
     return b;
 }
@@ -1292,7 +1294,7 @@ extern "C" long long fd_dense_decode_plan(int M, int H, int I, int n_q, int n_kv
         for (int c = 0; c < plan.n; ++c)
             if (plan.gu[c + 1] - plan.gu[c] > info[4]) info[4] = plan.gu[c + 1] - plan.gu[c];
     }
-    return (long long)fd::dd_buffers(M, H, I, n_q, n_kv, D, plan.S).all;
+    return (long long)fd::dd_buffers(M, H, I, n_q, n_kv, D, plan).all;
 }
 
 // All `count` entries of a decode step; the finished stream is left in resid.
@@ -1306,7 +1308,7 @@ extern "C" int fd_dense_decode(const FdDenseDecode* s, const FdDenseLayer* layer
     DdPlan plan;
     FD_REQUIRE(dd_plan(M, H, I, n_q, n_kv, D, sms, smem, &plan), -2, "dense_decode: sizes not taken");
     FD_REQUIRE((uintptr_t)s->next % 16 == 0, -2, "dense_decode: the memory to prefetch must be 16-byte aligned");
-    const DdBuffers buf = dd_buffers(M, H, I, n_q, n_kv, D, plan.S);
+    const DdBuffers buf = dd_buffers(M, H, I, n_q, n_kv, D, plan);
     static thread_local DdParams p;               // (26 KB: not on the caller's stack)
     u64* at = static_cast<u64*>(s->exchange);
     p.resid = s->resid;

@@ -191,8 +191,8 @@ class DensePrompts:
         s, cache = _Decode(), ctx.cache
         s.resid, s.tok_pos, s.row_slot = resid.data_ptr(), ctx.tok_pos.data_ptr(), ctx.row_slot.data_ptr()
         s.row_ctx_len, s.status, s.stream = ctx.row_ctx_len.data_ptr(), ctx.rt.status.data_ptr(), K._stream()
-        # zeroed when it is made; for these rows only, so that every word is written in every step
-        s.exchange = ctx.ws.get(f"dense_decode.{ctx.T}", (self.exchange_words[ctx.T],), torch.int64).data_ptr()
+        # zeroed when it is made; steps of all row counts share it
+        s.exchange = ctx.ws.get("dense_decode", (self.exchange_words[ctx.T],), torch.int64).data_ptr()
         s.M = ctx.T
         s.next, s.next_bytes = K._prefetch_args(upcoming, linear.UPCOMING_BYTES)       # (a hint: the head may be any part)
         self._cache_args(s, cache)

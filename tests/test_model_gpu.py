@@ -306,6 +306,17 @@ def test_decode_bits_do_not_depend_on_the_neighbours(decode_models, sizes, n_seq
         assert all(torch.equal(a, b) for a, b in zip(out[0], other))
 
 
+def test_decode_steps_of_all_row_counts_in_one_memory(decode_models):
+    """Steps of 24, 2, 17 and 24 sequences in turn, whose words lie at other places of the same memory: the bits of the first time."""
+    m = decode_models("1.5B")
+    out = {}
+    for n_seqs in (24, 2, 17, 24, 2, 17):
+        lengths = [300 + 7 * i for i in range(n_seqs)]
+        reqs = prompts_for(m.vocab_size, [n + 2 for n in lengths], seed=8)
+        got, _, _ = _decode_steps(m, reqs, lengths, True)
+        assert all(torch.equal(a, b) for a, b in zip(out.setdefault(n_seqs, got), got))
+
+
 @pytest.mark.parametrize("kept", [1, 2, 3, 4])
 def test_decode_in_one_kernel_every_wait_ends(decode_models, kept):
     """Words that one CTA keeps to itself - its normed stream, its queries, its attention, its partial sums - let the waits for them run

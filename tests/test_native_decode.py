@@ -84,3 +84,18 @@ def test_the_switch_for_products_rules_from_17_rows_on(calls, monkeypatch, gemm,
     """``linear.PROMPT_GEMM`` names the kernels of steps of more than 16 rows; a step that is to run on others is not one kernel."""
     monkeypatch.setattr(linear, "PROMPT_GEMM", gemm)
     assert [rows for rows in range(1, 26) if _step(rows)[0].decodes(None, _step(rows)[1])] == list(range(1, most + 1))
+
+
+def test_steps_of_all_row_counts_share_their_exchange_memory(calls):
+    """A workspace holds the words of the largest step so far, and no more splits of the attention than a step can have."""
+    ws = Workspace(torch.device("cpu"))
+    sizes = {rows: K.dense_decode_words(rows, 1536, 8960, 12, 2, 128) for rows in (24, 3, 17, 1)}
+    for rows in sizes:
+        native, ctx = _step(rows)
+        ctx.ws = ws
+        assert native.decodes(None, ctx)
+        native.decode(ctx, torch.zeros(rows, 1536), None)
+    assert len({s.exchange for s in calls}) == 1
+    assert sum(b.numel() for (_, dtype), b in ws._bufs.items() if dtype == torch.int64) == sizes[24]
+    # packets of a row: x twice, sums of squares, q, k and v, attention, activations, at most 4 slices' partial sums, 3 splits of 12 heads
+    assert sizes[24] <= 24 * (1536 + 192 + 768 + 256 + 768 + 4480 + 4 * 1536 + 3 * 12 * 130) + 200
