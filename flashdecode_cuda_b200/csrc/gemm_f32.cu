@@ -326,13 +326,24 @@ static int launch_tile(const float* A, const float* W, const float* bias, float*
     return check_launch("gemm_f32_tile");
 }
 
+static int f32_sm_count() {
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    return sms > 0 ? sms : 1;      // (no device: the launch says so)
+}
+
 static int g_f32_form = 0;       // 0: by the rule below; 1 + i: form i (tests and measurements)
 
 // aligned: A and W 16-byte aligned and K a multiple of 4.  Returns 1 if it does not take the sizes.
 int launch_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, bool aligned,
                     cudaStream_t stream) {
+    const int sms = f32_sm_count();
     if (M <= 16) {
-        const bool wide = N >= 64 * 148;         // 64 rows of W per CTA still give every SM one
+        const bool wide = N >= 64 * sms;         // 64 rows of W per CTA still give every SM one
         // rows that are not 16-byte aligned come four bytes a copy: short steps and many CTAs (8 x 333 x 1,537 15 us, 8 x 64 x 65 2.8; with steps
         // of 256 k and 16 rows 39 and 8.0), and the caller's kernel where W has many rows
         if (!aligned) return wide ? 1 : launch_rows<8, 32, 6, 16, 1, 1, 1, false>(A, W, bias, C, M, N, K, stream);
@@ -345,9 +356,13 @@ int launch_gemm_f32(const float* A, const float* W, const float* bias, float* C,
         }
         // a short chain is not worth a ring of long steps, most of which may lie beyond K (16 x 8 x 64 4.6 us in those, 2.2 here; 16 x 1,536 x 384 6.4 and 4.3)
         if (K <= 384) return launch_rows<16, 64, 4, 16, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
-        // The rings take most of an SM's shared memory, one CTA each: 12, 14 or 16 rows of W per CTA, the fewest that leave no second
-        // round (M 8: 2,048 x 1,536 16.5 us with 12 rows, 171 CTAs, and 12.0 with 14, 147 CTAs).
-        const int rows = N <= 12 * 148 ? 12 : N <= 14 * 148 ? 14 : 16;
+        // Rows of W per CTA: where CTAs outnumber the SMs, some SM has two, which share what its shared memory delivers (rings of up to 114
+        // KB: M 8, 2,048 x 1,536 12.9 us in 171 CTAs of 12 rows, 10.0 in 147 of 14) or, where two rings do not fit, follow one another (12 rows
+        // at M 16, 117 KB: 22.2 against 12.0 us).  So the fewest of 12, 14 and 16 rows with a CTA per SM; fewer are faster where all have
+        // one (M 8, 1,536 columns 9.5, 9.9, 10.8 us).  Where none has: for M of 5 to 8 twelve rows, whose rings fit twice (2,560 columns 13.2 us,
+        // with 16 rows, 125 KB, 20.3), for more 16 (18.5, with 12 rows 22.4).  M of 2 to 4 always 16: 12 rows take as long at M 2 (8.8 us for 2,048
+        // columns) and longer at M 4 (10.7 against 8.9).  M 1 has no form of 14 (its 12 rows 7.4 us up to 1,776 columns, 16 8.6).
+        const int rows = N <= 12 * sms ? 12 : N <= 14 * sms ? 14 : 16;
         if (M <= 1) {
             if (rows == 12) return launch_rows<12, 256, 5, 1, 1, 1, 8>(A, W, bias, C, M, N, K, stream);
             return launch_rows<16, 256, 5, 1, 1, 1, 8>(A, W, bias, C, M, N, K, stream);
@@ -356,7 +371,7 @@ int launch_gemm_f32(const float* A, const float* W, const float* bias, float* C,
         if (M <= 4) return launch_rows<16, 256, 5, 4, 1, 1, 4>(A, W, bias, C, M, N, K, stream);
         if (M <= 8) {
             if (rows == 14) return launch_rows<14, 256, 5, 8, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
-            if (N > 14 * 148 && N <= 16 * 148) return launch_rows<16, 256, 5, 8, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
+            if (N > 14 * sms && N <= 16 * sms) return launch_rows<16, 256, 5, 8, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
             return launch_rows<12, 256, 5, 8, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
         }
         if (rows == 12) return launch_rows<12, 256, 4, 16, 2, 1, 4>(A, W, bias, C, M, N, K, stream);
@@ -375,7 +390,7 @@ int launch_gemm_f32(const float* A, const float* W, const float* bias, float* C,
         for (int i = 0; i < 6; ++i) {
             if ((M + bm[i] - 1) / bm[i] > 65535) continue;           // more rows of tiles than a grid has
             const long long tiles = (long long)((M + bm[i] - 1) / bm[i]) * ((N + bn[i] - 1) / bn[i]);
-            const float per_sm = (float)((tiles + 147) / 148) * shared[i], t = per_sm > alone[i] ? per_sm : alone[i];
+            const float per_sm = (float)((tiles + sms - 1) / sms) * shared[i], t = per_sm > alone[i] ? per_sm : alone[i];
             if (form < 0 || t < best) { form = i; best = t; }
         }
     }
