@@ -189,7 +189,9 @@ def test_decode_steps_in_one_kernel(engines, folders, name, block_size, n_seqs):
         finally:
             m.native = native
             del native.decode
-        return out, [cache.gather(s, 0, layer_group) for s in slots for layer_group in range(1)]
+        # keys and values of the two new tokens, in every layer of every group (the window's too)
+        return out, [[t[n:n + 2] for t in cache.gather(s, g, layer)] for s, n in zip(slots, lengths)
+                     for g, group in enumerate(cache.groups) for layer in range(group.keys.shape[0])]
     (got, kv), (again, _), (parts, kv_parts) = steps(True), steps(True), steps(False)
     assert len(taken) == 4
     assert all(torch.equal(a, b) for a, b in zip(got, again))
@@ -202,8 +204,9 @@ def test_decode_steps_in_one_kernel(engines, folders, name, block_size, n_seqs):
         want = oracle_logits(folders[name], r)
         for j in range(2):
             assert rel_err(got[j][i], want[n + j]) < TOL["bfloat16"], (n, j)
+    assert len(kv) == len(kv_parts) == 2 * n_seqs
     for a, b in zip(kv, kv_parts):
-        assert all(rel_err(x, y) < TOL["bfloat16"] for x, y in zip(a, b))
+        assert all(float(y.abs().max()) > 0 and rel_err(x, y) < TOL["bfloat16"] for x, y in zip(a, b))
     m.check_status()
 
 
