@@ -5,9 +5,10 @@
 // 42 us (one sequence): each kernel starts its loads only when the one before has drained, and its own last reductions and first
 // trips to memory leave HBM idle.  Here one persistent CTA per SM copies ITS share of all weights, layer after layer, through one ring
 // of shared-memory stages: weights depend on nothing, so the ring runs ahead through every exchange of activations.  With
-// everything but the ring left out a layer takes 14.0 us; what remains on top is the chain of exchanges below.  Measured, us per layer
-// of a replayed step, parts / one kernel: 1.5B sizes, 1 sequence of 1,300 tokens 42.2 / 29.4, 2 of 1,500 41.6 / 32.4, 8 of 2,200 46.2 /
-// 39.1, 16 of 600 49.6 / 42.2, 24 of 1,200 63.8 / 56.7; 7B 1 of 1,800 103.8 / 88.7, 8 of 1,800 120.7 / 110.9; 14B 1 of 1,000 127.4 / 103.6, 8 of 1,000 141.8 / 136.4.
+// everything but the ring left out a layer takes 14.0 us; what remains on top is the chain of exchanges below.  Measured, us of a replayed
+// step by its layers (head and sampler included), parts / one kernel: 1.5B sizes, 1 sequence of 1,300 tokens 41.3 / 30.8, 2 of 1,500 43.9 /
+// 35.5, 8 of 2,200 47.2 / 42.2, 16 of 600 52.4 / 45.2, 24 of 1,200 67.0 / 58.8; 7B 1 of 1,800 103.4 / 89.2, 8 of 1,800 108.2 / 106.0, of 1,100
+// to 2,600 113.0 / 109.1; 14B 1 of 1,000 127.5 / 99.4, 8 of 1,000 134.9 / 125.0.  Counters: HBM reads 1.008 of the matrices, keys and values.
 //
 // What is exchanged, and how.  A layer is a chain of exchanges through L2: normed stream -> q, k, v -> partial attention -> attention
 // -> normed stream -> gated activations -> partial sums -> stream.  Each 32-bit word (two bfloat16, or a float) travels in an 8-byte
